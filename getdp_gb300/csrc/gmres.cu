@@ -42,8 +42,9 @@ struct Segment {
 
 // sliced-ELL copy of one triangular part, wide levels only: slice s holds
 // 32 rows x width[s] entries at 32 * wscan[s], entry j of lane l at
-// + 32 j + l; src is the entry's position in the CSR factor (-1: padding,
-// col = the row itself with value 0)
+// + 32 j + l; src is the entry's position in the CSR factor; padding has
+// src = col = -1 and is skipped (a product of its zero with a vector entry
+// not yet written would be NaN when that memory happens to hold one)
 struct EllPart {
   std::vector<int> slice0;  // per segment: its first slice (wide segments)
   int nslices = 0;
@@ -219,14 +220,11 @@ __global__ void k_ell_fill(int r0, int w, int nsl, int slice0, const int *__rest
   int s = slice0 + (t >> 5), lane = t & 31;
   long long base = 32 * wscan[s] + lane;
   int W = width[s];
-  int i = 0, k0 = 0, cnt = 0;
-  if(t < w) {
-    i = rows[r0 + t];
-    part_range<UPPER>(i, rowptr, diag, k0, cnt);
-  }
+  int k0 = 0, cnt = 0;
+  if(t < w) part_range<UPPER>(rows[r0 + t], rowptr, diag, k0, cnt);
   for(int j = 0; j < W; j++) {
     bool in = j < cnt;
-    ecol[base + 32LL * j] = in ? col[k0 + j] : i;
+    ecol[base + 32LL * j] = in ? col[k0 + j] : -1;
     esrc[base + 32LL * j] = in ? k0 + j : -1;
   }
 }
@@ -459,7 +457,10 @@ k_level_ell(int r0, int w, int slice0, const int *__restrict__ rows,
   long long e = 32 * wscan[s] + (t & 31);
   int W = width[s];
   X acc = (MODE == 1) ? src[i] : x[i];
-  for(int j = 0; j < W; j++, e += 32) acc = acc - (X)ev[e] * x[ecol[e]];
+  for(int j = 0; j < W; j++, e += 32) {
+    const int c = ecol[e];
+    if(c >= 0) acc = acc - (X)ev[e] * x[c];
+  }
   x[i] = (MODE == 2) ? (X)inv[i] * acc : acc;
 }
 

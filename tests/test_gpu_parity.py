@@ -15,6 +15,7 @@ import numpy as np
 import pytest
 
 import oracle
+from getdp_gb300 import _lib
 from getdp_gb300 import generate as G_
 from getdp_gb300 import linalg as LA
 from getdp_gb300 import workloads as W
@@ -648,3 +649,25 @@ def test_solve_again_reuses_the_factorisation(renumbering, algorithm):
     xg = LA.LinAlg_CreateVector(None, n)
     ig = LA.LinAlg_SolveAgain(A, b, S, xg)
     assert ig["status"] == 0 and ig["ilu_factorized"] == 1
+
+
+@pytest.mark.parametrize("precision", [0, 2])
+def test_wide_sweeps_do_not_read_the_output(precision):
+    """The padding of the sliced-ELL rows must not touch the vector being
+    written: its memory may hold anything, NaN included, before the sweep."""
+    import ctypes
+
+    A = _red_black_laplacian(90)
+    n = A.shape[0]
+    G2 = LA.LinAlg_CreateMatrix(None, n)
+    G2.set_csr(A.indptr, A.indices, A.data)
+    v = LA.LinAlg_CreateVector(None, n)
+    v.set(np.random.default_rng(3).standard_normal(n))
+    out = []
+    for fill in (0.0, np.nan):
+        z = LA.LinAlg_CreateVector(None, n)
+        z.set(np.full(n, fill))
+        S = _solver({"Preconditioner": 6, "Renumbering_Technique": 0, "Precision": precision})
+        _lib.check(_lib.load().gb300_precond_apply(G2.h, ctypes.byref(S.params), v.h, z.h))
+        out.append(z.numpy())
+    assert np.array_equal(out[0], out[1])
