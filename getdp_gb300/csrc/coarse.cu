@@ -25,9 +25,9 @@
 //     no sum can overflow; each term is rounded once, by at most half a
 //     quantum, 2^(h-62) of max|a_ij| with h - 1 the bits of the largest
 //     number of entries one coarse entry receives (2^-51 for 1,000);
-//   * the dense inverse is Gauss-Jordan elimination without pivoting, one
-//     launch per pivot (Ac is symmetric positive definite when A is and no
-//     aggregate is empty; a pivot <= 0 is reported as an error);
+//   * the dense inverse is a blocked symmetric elimination without pivoting,
+//     two launches per 32 pivots (Ac is symmetric positive definite when A is
+//     and no aggregate is empty; a pivot <= 0 is reported as an error);
 //   * restriction and the coarse product are warp sums in a fixed order.
 #include <math.h>
 #include <string.h>
@@ -41,6 +41,8 @@
 #include "sparse.cuh"
 
 namespace gb {
+
+constexpr int kSwB = 32;  // block of the coarse inverse's elimination (below)
 
 void coarse_free(Coarse *c) { delete c; }
 
@@ -108,8 +110,7 @@ int coarse_set(gb300_matrix *A, const int *agg, int nc)
   GB_TRY(c->aperm.alloc(n));
   GB_TRY(c->aptr.alloc(nc + 1));
   GB_TRY(c->inv.alloc((size_t)nc * nc));
-  GB_TRY(c->rbuf.alloc(2 * (size_t)nc));
-  GB_TRY(c->cbuf.alloc(2 * (size_t)nc));
+  GB_TRY(c->panel.alloc((2 * (size_t)nc + kSwB) * kSwB));
   GB_TRY(c->rc.alloc(nc));
   GB_TRY(c->ec.alloc(nc));
   GB_TRY(c->err.alloc(1));
@@ -245,8 +246,7 @@ int coarse_follow(const gb300_matrix *A, gb300_matrix *B, const Colouring *C,
   GB_TRY(c->aperm.alloc(n));
   GB_TRY(c->aptr.alloc(nc + 1));
   GB_TRY(c->inv.alloc((size_t)nc * nc));
-  GB_TRY(c->rbuf.alloc(2 * (size_t)nc));
-  GB_TRY(c->cbuf.alloc(2 * (size_t)nc));
+  GB_TRY(c->panel.alloc((2 * (size_t)nc + kSwB) * kSwB));
   GB_TRY(c->rc.alloc(nc));
   GB_TRY(c->ec.alloc(nc));
   GB_TRY(c->err.alloc(1));
@@ -326,44 +326,196 @@ __global__ void k_coarse_to_double(long long m, int headroom,
   }
 }
 
-__global__ void k_gj_init(int nc, const double *__restrict__ a, double *rbuf, double *cbuf)
-{
-  for(int j = blockIdx.x * blockDim.x + threadIdx.x; j < nc; j += gridDim.x * blockDim.x) {
-    rbuf[j] = a[j];                 // row 0
-    cbuf[j] = a[(size_t)j * nc];    // column 0
-  }
-}
+// The inverse of the symmetric positive definite nc x nc matrix, in place, by
+// the symmetric sweep operator on blocks of kSwB columns: for the block K
+// with diagonal block D and panel P = A(:, K),
+//
+//   A(i, j) -= P(i) D^-1 P(j)^T   (i, j outside K)
+//   A(i, K)  = P(i) D^-1,  A(K, K) = -D^-1,
+//
+// after which A holds -A^-1.  The matrix stays symmetric, so only the lower
+// triangle is kept up: nc^3 / 2 FMAs.  GB300's FP64 pipe (two FMAs per SM
+// per clock) bounds the update (1.0 ms at nc = 1024); a sweep of one pivot
+// per launch read and wrote all nc^2 entries 1,024 times (8 GB each way
+// through L2 and 1,024 launches, 14.6 ms).  32 columns: narrower blocks
+// re-read the triangle more often, wider ones lengthen the serial inversion
+// of D.  No pivoting: the pivots met inside the blocks are those of the
+// unblocked elimination, and one that is not positive is reported.
+constexpr int kSwRows = 16;  // panel rows per CTA
 
-// pivot step k of the in-place Gauss-Jordan inversion; row k and column k of
-// the matrix before the step come from the buffers of parity k, and the step
-// writes row and column k + 1 of its result to the other parity
-__global__ void k_gj_step(int nc, int k, double *a, double *rbuf, double *cbuf, int *err)
+// W(i) = P(i) D^-1 for this CTA's kSwRows rows; P, W: nc x kSwB; the first
+// CTA also writes D^-1.  Every CTA inverts D itself (in shared memory, one
+// barrier per pivot): cheaper than a launch of its own.
+__global__ void __launch_bounds__(256)
+k_sweep_panel(int nc, int k0, const double *__restrict__ a, double *__restrict__ P,
+              double *__restrict__ W, double *__restrict__ dinv, int *err)
 {
   if(*err) return;
-  const double *R = rbuf + (size_t)(k & 1) * nc;
-  const double *Cc = cbuf + (size_t)(k & 1) * nc;
-  double *Rn = rbuf + (size_t)((k + 1) & 1) * nc;
-  double *Cn = cbuf + (size_t)((k + 1) & 1) * nc;
-  const double piv = R[k];
-  if(!(piv > 0.) || !(piv <= 1.7976931348623157e308)) {
-    if(blockIdx.x == 0 && threadIdx.x == 0) atomicCAS(err, 0, k + 1);
+  __shared__ double D[2][kSwB][kSwB + 1];
+  __shared__ double sp[kSwRows][kSwB + 1];
+  __shared__ double rp[2];
+  const int t = threadIdx.x;
+  const int bw = nc - k0 < kSwB ? nc - k0 : kSwB;
+  const int i = t >> 3, j0 = (t & 7) * 4;
+#pragma unroll
+  for(int u = 0; u < 4; u++) {
+    const int j = j0 + u;
+    const int hi = i > j ? i : j, lo = i > j ? j : i;
+    D[0][i][j] = hi < bw ? a[(size_t)(k0 + hi) * nc + k0 + lo] : (i == j ? 1. : 0.);
+  }
+  const int r0 = blockIdx.x * kSwRows;
+  for(int q = t; q < kSwRows * kSwB; q += 256) {
+    // the panel's rows below K by row, those above K (stored transposed) by
+    // column, so that both read runs of the lower triangle
+    int r, c;
+    if(r0 >= k0) {
+      r = q / kSwB;
+      c = q % kSwB;
+    }
+    else {
+      r = q % kSwRows;
+      c = q / kSwRows;
+    }
+    const int gi = r0 + r, gj = k0 + c;
+    double v = 0.;
+    if(gi < nc && c < bw)
+      v = gi >= gj ? a[(size_t)gi * nc + gj] : a[(size_t)gj * nc + gi];
+    sp[r][c] = v;
+  }
+  __syncthreads();
+  if(t == 0) rp[0] = 1. / D[0][0][0];
+  __syncthreads();
+  for(int k = 0; k < kSwB; k++) {
+    const int cur = k & 1, nxt = cur ^ 1;
+    const double piv = D[cur][k][k];
+    if(!(piv > 0.) || !(piv <= 1.7976931348623157e308)) {  // the same in every thread
+      if(blockIdx.x == 0 && t == 0) atomicCAS(err, 0, k0 + k + 1);
+      return;
+    }
+    // one FMA per entry (FP64 instructions, not memory, pace the pivots):
+    // row k is 0 + p R, column k is 0 + m 1, the rest D + m R
+    const double p = rp[cur], m = i == k ? p : -D[cur][i][k] * p;
+#pragma unroll
+    for(int u = 0; u < 4; u++) {
+      const int j = j0 + u;
+      const double r = j == k ? 1. : D[cur][k][j];
+      const double v = fma(m, r, (i == k || j == k) ? 0. : D[cur][i][j]);
+      D[nxt][i][j] = v;
+      if(i == k + 1 && j == k + 1) rp[nxt] = 1. / v;
+    }
+    __syncthreads();
+  }
+  static_assert(kSwB % 2 == 0, "the result is in D[0]");
+  {
+    const int r = t >> 4, c = (t & 15) * 2;
+    double w0 = 0., w1 = 0.;
+#pragma unroll 8
+    for(int k = 0; k < kSwB; k++) {
+      w0 = fma(sp[r][k], D[0][k][c], w0);
+      w1 = fma(sp[r][k], D[0][k][c + 1], w1);
+    }
+    if(r0 + r < nc) {
+      const size_t o = (size_t)(r0 + r) * kSwB + c;
+      P[o] = sp[r][c];
+      P[o + 1] = sp[r][c + 1];
+      W[o] = w0;
+      W[o + 1] = w1;
+    }
+  }
+  if(blockIdx.x == 0)
+#pragma unroll
+    for(int u = 0; u < 4; u++) dinv[i * kSwB + j0 + u] = D[0][i][j0 + u];
+}
+
+// the lower triangle's 32 x 32 tile (ti, tj) after the sweep of block K
+__global__ void __launch_bounds__(64)
+k_sweep_update(int nc, int kb, double *__restrict__ a, const double *__restrict__ P,
+               const double *__restrict__ W, const double *__restrict__ dinv, const int *err)
+{
+  if(*err) return;
+  // tile number -> (ti, tj), tj <= ti
+  int ti = (int)((sqrtf(8.f * (float)blockIdx.x + 1.f) - 1.f) * 0.5f);
+  while((long long)(ti + 1) * (ti + 2) / 2 <= (long long)blockIdx.x) ti++;
+  while((long long)ti * (ti + 1) / 2 > (long long)blockIdx.x) ti--;
+  const int tj = (int)((long long)blockIdx.x - (long long)ti * (ti + 1) / 2);
+  const int t = threadIdx.x, i0 = ti * kSwB, j0 = tj * kSwB;
+  if(ti == kb || tj == kb) {
+    for(int q = t; q < kSwB * kSwB; q += 64) {
+      const int r = q / kSwB, c = q % kSwB;
+      if(i0 + r >= nc || j0 + c >= nc) continue;
+      double v;
+      if(ti == tj)
+        v = -dinv[q];
+      else if(tj == kb)
+        v = W[(size_t)(i0 + r) * kSwB + c];
+      else
+        v = W[(size_t)(j0 + c) * kSwB + r];
+      a[(size_t)(i0 + r) * nc + j0 + c] = v;
+    }
     return;
   }
-  const double p = 1.0 / piv;
-  const long long m = (long long)nc * nc;
-  for(long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < m;
-      idx += (long long)gridDim.x * blockDim.x) {
-    const int i = (int)(idx / nc), j = (int)(idx - (long long)i * nc);
-    double v;
-    if(i == k)
-      v = (j == k) ? p : R[j] * p;
-    else if(j == k)
-      v = -Cc[i] * p;
-    else
-      v = fma(-Cc[i] * p, R[j], a[idx]);
-    a[idx] = v;
-    if(i == k + 1) Rn[j] = v;
-    if(j == k + 1) Cn[i] = v;
+  __shared__ double sw[kSwB][kSwB + 1], spt[kSwB][kSwB + 1];  // [k][row]
+  for(int q = t; q < kSwB * kSwB; q += 64) {
+    const int r = q / kSwB, c = q % kSwB;
+    sw[c][r] = i0 + r < nc ? W[(size_t)(i0 + r) * kSwB + c] : 0.;
+    spt[c][r] = j0 + r < nc ? P[(size_t)(j0 + r) * kSwB + c] : 0.;
+  }
+  // 4 x 4 entries per thread, rows and columns 8 apart (no bank conflicts,
+  // coalesced columns)
+  const int ty = t >> 3, tx = t & 7;
+  double acc[4][4];
+#pragma unroll
+  for(int u = 0; u < 4; u++)
+#pragma unroll
+    for(int v = 0; v < 4; v++) {
+      const int r = i0 + ty + 8 * u, c = j0 + tx + 8 * v;
+      acc[u][v] = (r < nc && c < nc) ? a[(size_t)r * nc + c] : 0.;
+    }
+  __syncthreads();
+#pragma unroll 4
+  for(int k = 0; k < kSwB; k++) {
+    double wr[4], pc[4];
+#pragma unroll
+    for(int u = 0; u < 4; u++) {
+      wr[u] = sw[k][ty + 8 * u];
+      pc[u] = spt[k][tx + 8 * u];
+    }
+#pragma unroll
+    for(int u = 0; u < 4; u++)
+#pragma unroll
+      for(int v = 0; v < 4; v++) acc[u][v] = fma(-wr[u], pc[v], acc[u][v]);
+  }
+#pragma unroll
+  for(int u = 0; u < 4; u++)
+#pragma unroll
+    for(int v = 0; v < 4; v++) {
+      const int r = i0 + ty + 8 * u, c = j0 + tx + 8 * v;
+      if(r < nc && c < nc) a[(size_t)r * nc + c] = acc[u][v];
+    }
+}
+
+// A^-1 = -(swept matrix), the upper triangle from the lower one
+__global__ void __launch_bounds__(256)
+k_sweep_finish(int nc, double *__restrict__ a, const int *err)
+{
+  if(*err) return;
+  __shared__ double s[32][33];
+  const int ti = blockIdx.y, tj = blockIdx.x;
+  if(tj > ti) return;
+  const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
+  for(int r = y; r < 32; r += 8) {
+    const int i = ti * 32 + r, j = tj * 32 + x;
+    double v = 0.;
+    if(i < nc && j <= i) {
+      v = -a[(size_t)i * nc + j];
+      a[(size_t)i * nc + j] = v;
+    }
+    s[r][x] = v;
+  }
+  __syncthreads();
+  for(int r = y; r < 32; r += 8) {
+    const int i = tj * 32 + r, j = ti * 32 + x;  // transposed tile
+    if(j < nc && i < j) a[(size_t)i * nc + j] = s[x][r];
   }
 }
 
@@ -385,28 +537,15 @@ int coarse_setup(gb300_matrix *A, const double *val, bool reuse)
   k_coarse_to_double<<<grid_for(m, 256, kReduceBlocks), 256, 0, st>>>(m, c->headroom, amax,
                                                                       c->inv.p);
   GB_CUDA(cudaGetLastError());
-  const void *key[4] = {c->inv.p, c->rbuf.p, c->cbuf.p, c->err.p};
-  if(!c->gj_exec || c->gj_nc != nc || memcmp(key, c->gj_key, sizeof(key)) != 0) {
-    if(c->gj_exec) cudaGraphExecDestroy(c->gj_exec);
-    c->gj_exec = nullptr;
-    cudaGraph_t graph;
-    GB_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-    k_gj_init<<<grid_for(nc, 256), 256, 0, st>>>(nc, c->inv.p, c->rbuf.p, c->cbuf.p);
-    const int g = grid_for(m, 256, kReduceBlocks * 2);
-    for(int k = 0; k < nc; k++)
-      k_gj_step<<<g, 256, 0, st>>>(nc, k, c->inv.p, c->rbuf.p, c->cbuf.p, c->err.p);
-    GB_CUDA(cudaStreamEndCapture(st, &graph));
-    cudaError_t e = cudaGraphInstantiate(&c->gj_exec, graph, 0);
-    cudaGraphDestroy(graph);
-    if(e != cudaSuccess) {
-      c->gj_exec = nullptr;
-      set_error("coarse matrix: graph instantiation failed: %s", cudaGetErrorString(e));
-      return GB300_ERR_CUDA;
-    }
-    c->gj_nc = nc;
-    memcpy(c->gj_key, key, sizeof(key));
+  const int nb = (nc + kSwB - 1) / kSwB;
+  double *P = c->panel.p, *Wp = P + (size_t)nc * kSwB, *dinv = Wp + (size_t)nc * kSwB;
+  for(int k = 0; k < nb; k++) {
+    k_sweep_panel<<<grid_for(nc, kSwRows), 256, 0, st>>>(nc, k * kSwB, c->inv.p, P, Wp, dinv,
+                                                         c->err.p);
+    k_sweep_update<<<nb * (nb + 1) / 2, 64, 0, st>>>(nc, k, c->inv.p, P, Wp, dinv, c->err.p);
   }
-  GB_CUDA(cudaGraphLaunch(c->gj_exec, st));
+  k_sweep_finish<<<dim3(nb, nb), 256, 0, st>>>(nc, c->inv.p, c->err.p);
+  GB_CUDA(cudaGetLastError());
   int err = 0;
   GB_CUDA(cudaMemcpyAsync(&err, c->err.p, sizeof(int), cudaMemcpyDeviceToHost, st));
   GB_CUDA(cudaStreamSynchronize(st));

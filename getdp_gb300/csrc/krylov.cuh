@@ -100,19 +100,10 @@ struct Coarse {
   bool ready = false;       // inv holds the inverse for the last values
   DevBuf<int> agg, aperm, aptr;   // aggregate of each row; rows by aggregate
   DevBuf<double> inv;             // nc x nc, row-major
-  DevBuf<double> rbuf, cbuf;      // Gauss-Jordan pivot rows and columns
+  DevBuf<double> panel;           // the inversion's panels (coarse.cu)
   DevBuf<double> rc, ec;          // coarse residual and correction
   DevBuf<int> err;
   DevBuf<double> amax;
-  // the nc pivot launches of the inversion, captured once in a CUDA graph
-  // (replayed while nc and the buffers stay the same)
-  cudaGraphExec_t gj_exec = nullptr;
-  const void *gj_key[4] = {nullptr, nullptr, nullptr, nullptr};
-  int gj_nc = 0;
-  ~Coarse()
-  {
-    if(gj_exec) cudaGraphExecDestroy(gj_exec);
-  }
 };
 void coarse_free(Coarse *c);
 bool coarse_valid(const gb300_matrix *A);

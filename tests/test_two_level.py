@@ -268,3 +268,43 @@ def test_spai_cycle_solves_to_the_oracle_solution():
     print(f"SPAI-1 cycle {i25['iterations']} steps, ILU(0) cycle {i21['iterations']}")
     assert i25["status"] == 0
     assert np.linalg.norm(x25 - xo) <= 1e-10 * np.linalg.norm(xo)
+
+
+@pytest.mark.parametrize("nc", [1, 2, 31, 32, 33, 63, 64, 65, 97, 200])
+def test_coarse_inverse_at_the_edges_of_its_blocks(nc):
+    """u^T C u against numpy's inverse, one row per aggregate (Ac = A up to
+    the numbering).  Forward error of an elimination without pivoting on an
+    SPD matrix: ~nc eps cond(Ac), here <= 200 * 1.1e-16 * 1e4."""
+    rng = np.random.default_rng(nc)
+    M = rng.standard_normal((nc, nc))
+    D = M @ M.T / max(nc, 1) + 1e-3 * np.eye(nc)
+    assert np.linalg.cond(D) < 1e4
+    S = sp.csr_matrix(D)
+    A = LA.gMatrix(nc)
+    A.set_csr(S.indptr, S.indices, S.data)
+    perm = rng.permutation(nc)
+    A.set_aggregates(perm, nc)
+    u = LA.gVector(nc)
+    uh = rng.standard_normal(nc)
+    u.set(uh)
+    out = ctypes.c_double()
+    _lib.check(_lib.load().gb300_matrix_coarse_energy(A.h, u.h, ctypes.byref(out)))
+    ref = uh @ np.linalg.solve(D, uh)
+    assert abs(out.value - ref) <= 200 * 1.1e-16 * 1e4 * abs(ref)
+
+
+@pytest.mark.parametrize("bad", [0, 31, 32, 40, 69])
+def test_first_bad_pivot_is_named(bad):
+    nc = 70
+    d = np.full(nc, 2.0)
+    d[bad] = -1.0
+    S = sp.diags(d).tocsr()
+    A = LA.gMatrix(nc)
+    A.set_csr(S.indptr, S.indices, S.data)
+    A.set_aggregates(np.arange(nc), nc)
+    u = LA.gVector(nc)
+    u.set(np.ones(nc))
+    out = ctypes.c_double()
+    rc = _lib.load().gb300_matrix_coarse_energy(A.h, u.h, ctypes.byref(out))
+    assert rc == 5
+    assert f"pivot {bad + 1} of {nc}" in _lib.load().gb300_last_error().decode()
