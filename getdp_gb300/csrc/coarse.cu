@@ -33,7 +33,6 @@
 #include <string.h>
 
 #include <algorithm>
-#include <functional>
 #include <vector>
 
 #include "common.cuh"
@@ -564,68 +563,75 @@ int coarse_setup(gb300_matrix *A, const double *val, bool reuse)
 // ---------------------------------------------------------------------------
 // application
 
-__global__ void k_add_into(int n, const double *__restrict__ t, double *__restrict__ z,
-                           const int *flag)
-{
-  if(flag && !*flag) return;
-  for(int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    z[i] += t[i];
-}
+// rc = P0^T t: one CTA of kRestrictThreads per aggregate, its rows in a fixed
+// order (a warp per aggregate had left a thousand gathers to 32 lanes)
+constexpr int kRestrictThreads = 128;
 
-// rc = P0^T t: one warp per aggregate, its rows in a fixed order
-__global__ void k_restrict(int nc, const int *__restrict__ aptr, const int *__restrict__ aperm,
-                           const double *__restrict__ t, double *__restrict__ rc,
-                           const int *flag)
+__global__ void __launch_bounds__(kRestrictThreads)
+k_restrict(const int *__restrict__ aptr, const int *__restrict__ aperm, const double *t,
+           double *rc, const int *flag)
 {
+  constexpr int U = 4;
+  const int k = blockIdx.x;
+  const int q0 = aptr[k] + threadIdx.x, e = aptr[k + 1];
+  int i[U];
+#pragma unroll
+  for(int u = 0; u < U; u++)
+    i[u] = q0 + u * kRestrictThreads < e ? aperm[q0 + u * kRestrictThreads] : -1;
+  chain_wait();
   if(flag && !*flag) return;
-  const int lane = threadIdx.x & 31;
-  for(int k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; k < nc;
-      k += (gridDim.x * blockDim.x) >> 5) {
-    double s = 0.;
-    for(int q = aptr[k] + lane; q < aptr[k + 1]; q += 32) s += t[aperm[q]];
-    s = warp_sum(s);
-    if(lane == 0) rc[k] = s;
-  }
+  double s = 0.;
+#pragma unroll
+  for(int u = 0; u < U; u++)
+    if(i[u] >= 0) s += t[i[u]];
+#pragma unroll 4
+  for(int q = q0 + U * kRestrictThreads; q < e; q += kRestrictThreads) s += t[aperm[q]];
+  s = block_sum<double, kRestrictThreads>(s);
+  if(threadIdx.x == 0) rc[k] = s;
 }
 
 // ec = Ainv rc: one warp per row
-__global__ void k_coarse_gemv(int nc, const double *__restrict__ inv,
-                              const double *__restrict__ rc, double *__restrict__ ec,
-                              const int *flag)
+__global__ void __launch_bounds__(256)
+k_coarse_gemv(int nc, const double *__restrict__ inv, const double *rc, double *ec,
+              const int *flag)
 {
-  if(flag && !*flag) return;
+  constexpr int U = 8;
   const int lane = threadIdx.x & 31;
-  for(int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < nc;
-      i += (gridDim.x * blockDim.x) >> 5) {
-    const double *row = inv + (size_t)i * nc;
-    double s = 0.;
-    for(int j = lane; j < nc; j += 32) s = fma(row[j], rc[j], s);
-    s = warp_sum(s);
-    if(lane == 0) ec[i] = s;
-  }
-}
-
-// z += P0 ec
-__global__ void k_prolong(int n, const int *__restrict__ agg, const double *__restrict__ ec,
-                          double *__restrict__ z, const int *flag)
-{
+  const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const double *row = inv + (size_t)(i < nc ? i : 0) * nc;
+  double a[U];
+#pragma unroll
+  for(int u = 0; u < U; u++) a[u] = lane + 32 * u < nc ? row[lane + 32 * u] : 0.;
+  chain_wait();
   if(flag && !*flag) return;
-  for(int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    z[i] += ec[agg[i]];
+  if(i >= nc) return;
+  double s = 0.;
+#pragma unroll
+  for(int u = 0; u < U; u++)
+    if(lane + 32 * u < nc) s = fma(a[u], rc[lane + 32 * u], s);
+#pragma unroll 8
+  for(int j = lane + 32 * U; j < nc; j += 32) s = fma(row[j], rc[j], s);
+  s = warp_sum(s);
+  if(lane == 0) ec[i] = s;
 }
 
-void coarse_correct(const gb300_matrix *A, const double *val, const double *v, double *z,
-                    double *t, const int *flag, cudaStream_t st)
+static void coarse_solve(const Coarse *c, const double *t, int n, const int *flag,
+                         cudaStream_t st)
+{
+  launch_chain(chain_early(n), k_restrict, c->nc, kRestrictThreads, st, c->aptr.p, c->aperm.p,
+               t, c->rc.p, flag);
+  launch_chain(chain_early(n), k_coarse_gemv, grid_for((long long)c->nc * 32, 256), 256, st,
+               c->nc, c->inv.p, c->rc.p, c->ec.p, flag);
+}
+
+void coarse_correct(const gb300_matrix *A, const double *val, const double *v,
+                    const double *z, double *out, double *t, const int *flag,
+                    cudaStream_t st)
 {
   const Coarse *c = A->coarse;
-  const int n = A->n, nc = c->nc;
-  const int g = grid_for(n, 256, kReduceBlocks * 4);
-  resid_guarded(A, val, z, v, t, flag, st);  // t = v - A z
-  k_restrict<<<grid_for((long long)nc * 32, 256), 256, 0, st>>>(nc, c->aptr.p, c->aperm.p,
-                                                                t, c->rc.p, flag);
-  k_coarse_gemv<<<grid_for((long long)nc * 32, 256), 256, 0, st>>>(nc, c->inv.p, c->rc.p,
-                                                                   c->ec.p, flag);
-  k_prolong<<<g, 256, 0, st>>>(n, c->agg.p, c->ec.p, z, flag);
+  product_chain(kChainRes, A, val, {z, v, t, nullptr, nullptr, nullptr, flag}, st);
+  coarse_solve(c, t, A->n, flag, st);
+  product_chain(kChainProlong, A, val, {z, v, t, c->agg.p, c->ec.p, out, flag}, st);
 }
 
 // one block: out = rc . ec over the nc coarse entries, in a fixed order
@@ -665,10 +671,7 @@ int coarse_energy_project(gb300_matrix *A, double *w, double *t, double *q, doub
   const Coarse *c = A->coarse;
   const int n = A->n, nc = c->nc;
   const int g = grid_for(n, 256, kReduceBlocks * 4);
-  k_restrict<<<grid_for((long long)nc * 32, 256), 256, 0, st>>>(nc, c->aptr.p, c->aperm.p,
-                                                                w, c->rc.p, nullptr);
-  k_coarse_gemv<<<grid_for((long long)nc * 32, 256), 256, 0, st>>>(nc, c->inv.p, c->rc.p,
-                                                                   c->ec.p, nullptr);
+  coarse_solve(c, w, n, nullptr, st);
   k_coarse_dot<<<1, 1024, 0, st>>>(nc, c->rc.p, c->ec.p, wcw);
   k_prolong_set<<<g, 256, 0, st>>>(n, c->agg.p, c->ec.p, t);
   spmv_plain(A, A->val.p, t, q, st);
@@ -682,27 +685,10 @@ int coarse_energy(gb300_matrix *A, const double *u, double *ucu_dev, cudaStream_
   GB_TRY(coarse_setup(A, A->val.p, true));
   const Coarse *c = A->coarse;
   const int nc = c->nc;
-  k_restrict<<<grid_for((long long)nc * 32, 256), 256, 0, st>>>(nc, c->aptr.p, c->aperm.p,
-                                                                u, c->rc.p, nullptr);
-  k_coarse_gemv<<<grid_for((long long)nc * 32, 256), 256, 0, st>>>(nc, c->inv.p, c->rc.p,
-                                                                   c->ec.p, nullptr);
+  coarse_solve(c, u, A->n, nullptr, st);
   k_coarse_dot<<<1, 1024, 0, st>>>(nc, c->rc.p, c->ec.p, ucu_dev);
   GB_CUDA(cudaGetLastError());
   return GB300_OK;
-}
-
-void two_level_apply(const gb300_matrix *A, const double *val, const double *v, double *z,
-                     double *t3, double *t4, const int *flag, cudaStream_t st,
-                     const std::function<void(const double *, double *)> &smooth,
-                     const std::function<void(const double *, double *)> &smooth_post)
-{
-  const int n = A->n;
-  const int g = grid_for(n, 256, kReduceBlocks * 4);
-  smooth(v, z);
-  coarse_correct(A, val, v, z, t3, flag, st);
-  resid_guarded(A, val, z, v, t3, flag, st);  // t3 = v - A z
-  smooth_post(t3, t4);
-  k_add_into<<<g, 256, 0, st>>>(n, t4, z, flag);
 }
 
 }  // namespace gb

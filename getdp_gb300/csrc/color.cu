@@ -39,6 +39,8 @@
 // every result computed with it, is deterministic.  For a
 // batch of independent systems (diagonal blocks) the rows are reordered
 // within each block only, so every block keeps its row range.
+#include <memory>
+
 #include "krylov.cuh"
 
 namespace gb {
@@ -381,6 +383,7 @@ static int permuted_structure(gb300_matrix *A, Colouring *C, cudaStream_t st)
   GB_CUDA(cudaStreamSynchronize(st));
   if(herr) return GB300_ERR_UNSUPPORTED;
   B->csr_valid = true;
+  B->order = C;
   choose_tpr(B);
   return GB300_OK;
 }
@@ -546,7 +549,6 @@ int precond_apply(gb300_matrix *A, const gb300_solver_params *p, const double *v
   const int n = A->n;
   const bool learned = precond_learned(p->preconditioner);
   const bool coarse = precond_two_level(p->preconditioner);
-  const bool learned_post = learned && p->preconditioner != kPrecondLearnedCoarsePre;
   const bool sai = (p->preconditioner == kPrecondLearnedSai ||
                     p->preconditioner == kPrecondSai);
   if(p->preconditioner != 6 && !learned && !coarse) {
@@ -563,15 +565,8 @@ int precond_apply(gb300_matrix *A, const gb300_solver_params *p, const double *v
   }
   const bool fp32 = (p->precision != 0);
   gb300_matrix *M = A;
-  DevBuf<double> vb, zb, t1, t2, t3, t4;
-  DevBuf<float> t32;
-  GB_TRY(t1.alloc(n));
-  GB_TRY(t2.alloc(n));
-  if(coarse) {
-    GB_TRY(t3.alloc(n));
-    GB_TRY(t4.alloc(n));
-  }
-  if(fp32) GB_TRY(t32.alloc(n));
+  DevBuf<double> vb, zb;
+  std::vector<std::unique_ptr<DevBuf<char>>> bufs;
   const double *vin = v;
   double *zout = z;
   Colouring *C = nullptr;
@@ -603,23 +598,17 @@ int precond_apply(gb300_matrix *A, const gb300_solver_params *p, const double *v
     set_error("Zero pivot on line %d in ILU", zr);
     return GB300_ERR_ZERO_PIVOT;
   }
-  auto smooth = [&](const double *vv, double *zz, bool corr) {
-    if(sai) {  // z = G v
-      spmv_guarded(M, M->corr.p, vv, zz, nullptr, st);
-      return;
-    }
-    ilu_apply(M, ilu_mode(p), vv, zz, fp32 ? t32.p : nullptr, nullptr, st);
-    if(corr) correction_apply(M, M->val.p, vv, zz, t1.p, t2.p, nullptr, st);
-  };
   if(p->preconditioner == kPrecondSai) GB_TRY(spai1(M, M->val.p));
-  if(coarse) {
-    GB_TRY(coarse_setup(M, M->val.p, p->re_use_lu != 0));
-    two_level_apply(M, M->val.p, vin, zout, t3.p, t4.p, nullptr, st,
-                    [&](const double *vv, double *zz) { smooth(vv, zz, learned); },
-                    [&](const double *vv, double *zz) { smooth(vv, zz, learned_post); });
-  }
-  else
-    smooth(vin, zout, learned);
+  if(!sai) GB_TRY(ilu_products(M, M->val.p));
+  if(coarse) GB_TRY(coarse_setup(M, M->val.p, p->re_use_lu != 0));
+  PrecondScratch ps;
+  GB_TRY(ps.alloc(p, n, [&](int, size_t bytes) -> void * {
+    bufs.emplace_back(new DevBuf<char>());
+    return bufs.back()->alloc(bytes) == GB300_OK ? bufs.back()->p : nullptr;
+  }));
+  // the chain reads matrix, factor and correction ahead of its waits
+  GB_CUDA(cudaStreamSynchronize(st));
+  precond_run(M, M->val.p, p, vin, zout, ps, nullptr, st);
   if(C) unpermute_solution(C, zout, z, st);
   GB_CUDA(cudaGetLastError());
   GB_CUDA(cudaStreamSynchronize(st));

@@ -168,24 +168,30 @@ template <int NT> __device__ __forceinline__ double block_sum8(const double (&a)
   return s;
 }
 
-// Completion of a grid-wide reduction inside the kernel that produces the
-// partials: every block calls arrive_last after its partials are stored;
-// exactly one block, the last to arrive, gets true and then sees every
+// Completion of a reduction inside the kernel that produces the partials:
+// every block (of the grid, or of the group that shares the counter) calls
+// arrive_last after its partials are stored; exactly one block, the last of
+// `arrivals` to arrive, gets true and then sees every
 // partial (read them with __ldcg).  It resets the counter for the next
 // launch.  Needs no co-residency and never waits.
-__device__ __forceinline__ bool arrive_last(unsigned *counter)
+__device__ __forceinline__ bool arrive_last(unsigned *counter, unsigned arrivals)
 {
   __shared__ int last;
   __threadfence();
   __syncthreads();
   if(threadIdx.x == 0) {
     unsigned t = atomicAdd(counter, 1u);
-    last = (t == gridDim.x * gridDim.y * gridDim.z - 1);
+    last = (t == arrivals - 1);
     if(last) *counter = 0u;
   }
   __syncthreads();
   if(last) __threadfence();
   return last != 0;
+}
+
+__device__ __forceinline__ bool arrive_last(unsigned *counter)
+{
+  return arrive_last(counter, gridDim.x * gridDim.y * gridDim.z);
 }
 
 // the kReduceBlocks partials summed in the fixed order of the one-block
@@ -248,6 +254,49 @@ __device__ __forceinline__ int find_col(const int *__restrict__ col, int lo,
   }
   return (lo < end && col[lo] == c) ? lo : -1;
 }
+
+// Programmatic dependent launch: a kernel launched with launch_chain and
+// `early` may start while its predecessor in the stream still runs.
+// chain_wait() returns when the predecessor has completed and its writes are
+// visible; before it a kernel reads only data no kernel of the sequence
+// writes (matrix structure and values, factors, permutations), so that those
+// loads overlap the predecessor's tail.  The next kernel is released after
+// the wait, so everything older than the direct predecessor is complete when
+// a kernel starts.  Every CTA calls it (a CTA that skipped the wait could let
+// the kernel after it overtake the predecessor); without `early` it returns
+// at once.  Data written inside the sequence is read with plain loads (no
+// __restrict__ const, no __ldg: the non-coherent path could return lines
+// cached before the wait).
+__device__ __forceinline__ void chain_wait()
+{
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+template <typename... K, typename... A>
+inline void launch_chain(bool early, void (*kernel)(K...), dim3 grid, dim3 block,
+                         cudaStream_t st, A... args)
+{
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = early ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, kernel, K(args)...);  // errors: cudaGetLastError
+}
+
+// whether a sequence over n rows gains from the early start.  Measured on
+// 2D meshes in the multicolour order, both sweeps / a product, early against
+// not: 14.2 / 2.8 against 15.4 / 3.4 us at 65,025 rows, but 25.3 / 7.0
+// against 19.3 / 7.6 at 261,121: the waiting CTAs of the next kernel take the
+// free slots of whichever SMs have them, and its load is uneven from then on
+// (the FP64-bound Gram-Schmidt kernels lose by that at every size and never
+// start early)
+inline bool chain_early(int n) { return n <= 131072; }
 
 inline int grid_for(long long work, int threads, int max_blocks = 1 << 30)
 {
@@ -322,6 +371,8 @@ struct gb300_matrix {
   // ILU solves (created on demand) remembers the version it was made for
   unsigned pattern_version = 0;
   gb::Colouring *mc = nullptr;
+  // on a permuted copy: the ordering it is the copy of (owned by the source)
+  const gb::Colouring *order = nullptr;
   // rows per unknown (2: complex system in real form, harmonic-interleaved)
   int block_rows = 1;
   // learned preconditioner correction on the pattern (valid while

@@ -63,6 +63,12 @@ struct ilu_data {
   DevBuf<int> lptr, uptr;           // level offsets (device copies)
   std::vector<int> hlptr, huptr;    // level offsets (host)
   std::vector<Segment> lseg, useg;
+  // a multicolour copy (one row per vertex): the levels are the colours, rows
+  // in order (lrows and urows stay empty), the sweeps run as a chain
+  bool by_colour = false;
+  int n0 = 0;                       // rows of colour 0
+  EllPart aell;                     // A's own rows, for the products
+  const double *aell_of = nullptr;  // the values it holds (ilu_products)
   DevBuf<double> lu64, inv64;
   DevBuf<float> lu32, inv32;
   bool fact64 = false, fact32 = false;  // a factor of that precision is held
@@ -183,13 +189,14 @@ static int make_levels(gb300_matrix *A, ilu_data *L, int *d_indeg,
   return GB300_OK;
 }
 
-// entries of row i's strictly lower (UPPER = 0) or upper part
+// entries of row i's strictly lower (UPPER = 0) or upper (1) part, or of the
+// whole row (2)
 template <int UPPER>
 __device__ __forceinline__ void part_range(int i, const int *rowptr, const int *diag,
                                            int &k0, int &cnt)
 {
-  k0 = UPPER ? diag[i] + 1 : rowptr[i];
-  cnt = UPPER ? rowptr[i + 1] - diag[i] - 1 : diag[i] - rowptr[i];
+  k0 = UPPER == 1 ? diag[i] + 1 : rowptr[i];
+  cnt = UPPER == 0 ? diag[i] - rowptr[i] : rowptr[i + 1] - (UPPER == 1 ? diag[i] + 1 : k0);
 }
 
 template <int UPPER>
@@ -202,7 +209,7 @@ __global__ void k_ell_width(int r0, int w, int nsl, int slice0, const int *__res
   int cnt = 0;
   if(t < w) {
     int k0;
-    part_range<UPPER>(rows[r0 + t], rowptr, diag, k0, cnt);
+    part_range<UPPER>(rows ? rows[r0 + t] : r0 + t, rowptr, diag, k0, cnt);
   }
   cnt = __reduce_max_sync(0xffffffffu, cnt);
   if((t & 31) == 0) width[slice0 + (t >> 5)] = cnt;
@@ -221,7 +228,7 @@ __global__ void k_ell_fill(int r0, int w, int nsl, int slice0, const int *__rest
   long long base = 32 * wscan[s] + lane;
   int W = width[s];
   int k0 = 0, cnt = 0;
-  if(t < w) part_range<UPPER>(rows[r0 + t], rowptr, diag, k0, cnt);
+  if(t < w) part_range<UPPER>(rows ? rows[r0 + t] : r0 + t, rowptr, diag, k0, cnt);
   for(int j = 0; j < W; j++) {
     bool in = j < cnt;
     ecol[base + 32LL * j] = in ? col[k0 + j] : -1;
@@ -321,11 +328,27 @@ static int ilu_setup(gb300_matrix *A)
     A->ilu = nullptr;
     return GB300_ERR_UNSUPPORTED;
   }
-  int rc = make_levels<0>(A, L, indl.p, L->lrows, L->lptr, L->hlptr, L->lseg);
-  if(rc == GB300_OK)
-    rc = make_levels<1>(A, L, indu.p, L->urows, L->uptr, L->huptr, L->useg);
+  int rc = GB300_OK;
+  const Colouring *C = A->order;
+  if(C && C->kind == 0 && C->bs == 1 && C->seg.size() == 2) {
+    // first-fit colours: a row of colour c has neighbours of every smaller
+    // colour, so the colours are the forward sweep's levels; backwards they
+    // are a valid schedule of the same length
+    L->by_colour = true;
+    L->n0 = C->voff[1];
+    for(int c = 0; c < C->ncolors; c++)
+      L->lseg.push_back({c, c + 1, false, C->voff[c + 1] - C->voff[c], C->voff[c]});
+    L->useg.assign(L->lseg.rbegin(), L->lseg.rend());
+  }
+  else {
+    rc = make_levels<0>(A, L, indl.p, L->lrows, L->lptr, L->hlptr, L->lseg);
+    if(rc == GB300_OK)
+      rc = make_levels<1>(A, L, indu.p, L->urows, L->uptr, L->huptr, L->useg);
+  }
   if(rc == GB300_OK) rc = build_ell<0>(A, L->lseg, L->lrows.p, L->diag.p, L->lell, st);
   if(rc == GB300_OK) rc = build_ell<1>(A, L->useg, L->urows.p, L->diag.p, L->uell, st);
+  if(rc == GB300_OK && L->by_colour)
+    rc = build_ell<2>(A, {{0, 0, false, n, 0}}, nullptr, L->diag.p, L->aell, st);
   if(rc != GB300_OK) {
     ilu_free(A->ilu);
     A->ilu = nullptr;
@@ -427,7 +450,7 @@ k_level_wide(int r0, int width, const int *__restrict__ rows,
   if(flag && !*flag) return;
   int t = blockIdx.x * blockDim.x + threadIdx.x;
   if(t >= width) return;
-  int i = rows[r0 + t];
+  int i = rows ? rows[r0 + t] : r0 + t;
   if(MODE != 0 && rmask && !rmask[i]) return;
   if(MODE == 0)
     row_fact<T>(i, rowptr, col, diag, lu, inv, zero_row);
@@ -451,7 +474,7 @@ k_level_ell(int r0, int w, int slice0, const int *__restrict__ rows,
   if(flag && !*flag) return;
   int t = blockIdx.x * blockDim.x + threadIdx.x;
   if(t >= w) return;
-  int i = rows[r0 + t];
+  int i = rows ? rows[r0 + t] : r0 + t;
   if(rmask && !rmask[i]) return;
   int s = slice0 + (t >> 5);
   long long e = 32 * wscan[s] + (t & 31);
@@ -560,6 +583,176 @@ int ilu_factor(gb300_matrix *A, const double *val, bool fp32, int *zero_row_out,
   return GB300_OK;
 }
 
+// The sweeps on a multicolour copy, one launch per colour in a chain
+// (launch_chain): forward through the colours, the last colour's rows
+// finished at once (they have no upper entries), then backward to colour 0.
+// Colour 0 has no lower entries, so its forward values are the right-hand
+// side itself, which the other colours read in place: 2 C - 2 launches
+// instead of 2 C, and no pass that converts the vector.  A row's first
+// kSweepU entries and its pivot are loaded before the wait for the preceding
+// colour, and the guard is tested once the gathers are on their way: one
+// memory latency and a store remain of each colour.  Both sweeps at 65,025
+// rows, 4 colours: 15.4 us, 27 with a launch per level and sweep (rows of a
+// level in the order the schedule's atomics left them).  The accumulation
+// order is that of lusol.
+//   PART 0: forward, x = value          PART 1: last colour, both sweeps
+//   PART 2: backward, from x            PART 3: backward, from src (colour 0)
+// OUT 1: final values also to z as doubles; 2: added into z
+constexpr int kSweepU = 8;
+
+template <int PART, int OUT, typename T, typename X>
+__global__ void __launch_bounds__(256)
+k_colour_sweep(int r0, int w, int slice0, const int *__restrict__ width,
+               const long long *__restrict__ wscan, const int *__restrict__ ecol,
+               const T *__restrict__ ev, const T *__restrict__ inv, int n0, const double *src,
+               X *x, double *z, const int *flag)
+{
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  const int i = r0 + t;
+  int W = 0;
+  long long e = 0;
+  T iv = (T)0, v[kSweepU];
+  int c[kSweepU];
+  if(t < w) {
+    const int s = slice0 + (t >> 5);
+    W = width[s];
+    e = 32 * wscan[s] + (t & 31);
+    if(PART != 0) iv = inv[i];
+  }
+#pragma unroll
+  for(int u = 0; u < kSweepU; u++) {
+    c[u] = u < W ? ecol[e + 32 * u] : -1;
+    v[u] = u < W ? ev[e + 32 * u] : (T)0;
+  }
+  chain_wait();
+  if(t >= w) return;
+  const int go = flag ? *flag : 1;
+  X acc = PART == 2 ? x[i] : (X)src[i];
+  auto gather = [&](int cc) -> X {
+    if(PART < 2 && cc < n0) return (X)src[cc];
+    return x[cc];
+  };
+  X xv[kSweepU];
+#pragma unroll
+  for(int u = 0; u < kSweepU; u++) xv[u] = c[u] >= 0 ? gather(c[u]) : (X)0;
+  if(!go) return;
+#pragma unroll
+  for(int u = 0; u < kSweepU; u++)
+    if(c[u] >= 0) acc = acc - (X)v[u] * xv[u];
+  for(int j = kSweepU; j < W; j++) {
+    const int cc = ecol[e + 32LL * j];
+    if(cc >= 0) acc = acc - (X)ev[e + 32LL * j] * gather(cc);
+  }
+  if(PART != 0) acc = (X)iv * acc;
+  x[i] = acc;
+  if(PART != 0 && OUT == 1) z[i] = (double)acc;
+  if(PART != 0 && OUT == 2) z[i] += (double)acc;
+}
+
+template <int OUT, typename T, typename X>
+static void colour_sweeps(const ilu_data *L, const T *inv, const double *src, X *x, double *z,
+                          const int *flag, cudaStream_t st)
+{
+  const int C = (int)L->lseg.size();
+  auto go = [&](auto kernel, const EllPart &E, const Segment &g, int slice0) {
+    launch_chain(chain_early(L->n), kernel, grid_for(g.width, 256), 256, st, g.r0, g.width,
+                 slice0, E.width.p, E.wscan.p, E.col.p, ell_vals<T>(E), inv, L->n0, src, x, z,
+                 flag);
+  };
+  for(int c = 1; c < C - 1; c++)
+    go(k_colour_sweep<0, OUT, T, X>, L->lell, L->lseg[c], L->lell.slice0[c]);
+  go(k_colour_sweep<1, OUT, T, X>, L->lell, L->lseg[C - 1], L->lell.slice0[C - 1]);
+  for(int q = 1; q < C; q++) {  // useg[q] is colour C - 1 - q
+    if(q < C - 1)
+      go(k_colour_sweep<2, OUT, T, X>, L->uell, L->useg[q], L->uell.slice0[q]);
+    else
+      go(k_colour_sweep<3, OUT, T, X>, L->uell, L->useg[q], L->uell.slice0[q]);
+  }
+}
+
+// A multicolour copy's products, one thread per row of a sliced-ELL copy of
+// A: GB300's FP64 pipe, not memory, bounds them from ~500,000 rows on (14 us
+// for the 7.3 M FMAs at 1,046,529 rows), and a row shared by two lanes issues
+// 10 FP64 instructions per 32 rows of 7 entries where a thread per row issues 7
+template <int MODE>
+__global__ void __launch_bounds__(256)
+k_ell_chain(int n, const int *__restrict__ width, const long long *__restrict__ wscan,
+            const int *__restrict__ ecol, const double *__restrict__ ev, ChainArgs a)
+{
+  constexpr int U = 8;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  int W = 0, c[U], g[U], grow = 0;
+  long long e = 0;
+  double v[U];
+  if(i < n) {
+    W = width[i >> 5];
+    e = 32 * wscan[i >> 5] + (i & 31);
+    if(MODE == kChainProlong) grow = a.agg[i];
+  }
+#pragma unroll
+  for(int u = 0; u < U; u++) {
+    c[u] = u < W ? ecol[e + 32 * u] : -1;
+    v[u] = u < W ? ev[e + 32 * u] : 0.;
+    if(MODE == kChainProlong) g[u] = c[u] >= 0 ? a.agg[c[u]] : 0;
+  }
+  chain_wait();
+  if(i >= n) return;
+  const int go = a.flag ? *a.flag : 1;
+  double xv[U];
+#pragma unroll
+  for(int u = 0; u < U; u++) {
+    xv[u] = c[u] >= 0 ? a.x[c[u]] : 0.;
+    if(MODE == kChainProlong && c[u] >= 0) xv[u] += a.ec[g[u]];
+  }
+  if(!go) return;
+  double sum = 0.;
+#pragma unroll
+  for(int u = 0; u < U; u++)
+    if(c[u] >= 0) sum += v[u] * xv[u];
+#pragma unroll 4
+  for(int j = U; j < W; j++) {
+    const int cc = ecol[e + 32LL * j];
+    if(cc >= 0) {
+      double x = a.x[cc];
+      if(MODE == kChainProlong) x += a.ec[a.agg[cc]];
+      sum += ev[e + 32LL * j] * x;
+    }
+  }
+  chain_store<MODE>(a, i, grow, sum);
+}
+
+int ilu_products(gb300_matrix *A, const double *val)
+{
+  ilu_data *L = A->ilu;
+  if(!L || !L->by_colour) return GB300_OK;
+  L->aell_of = nullptr;
+  GB_TRY(ell_values<double>(L->aell, val, L->aell.v64, A->ctx->stream));
+  L->aell_of = val;
+  return GB300_OK;
+}
+
+void product_chain(ChainMode mode, const gb300_matrix *A, const double *val,
+                   const ChainArgs &a, cudaStream_t st)
+{
+  const ilu_data *L = A->ilu;
+  if(!L || !L->by_colour || L->aell_of != val || L->aell.entries == 0) {
+    spmv_chain(mode, A, val, a, st);
+    return;
+  }
+  const EllPart &E = L->aell;
+  auto go = [&](auto kernel) {
+    launch_chain(chain_early(A->n), kernel, grid_for(A->n, 256), 256, st, A->n, E.width.p,
+                 E.wscan.p, E.col.p, E.v64.p, a);
+  };
+  switch(mode) {
+  case kChainMul: go(k_ell_chain<kChainMul>); break;
+  case kChainAdd: go(k_ell_chain<kChainAdd>); break;
+  case kChainRes: go(k_ell_chain<kChainRes>); break;
+  case kChainProlong: go(k_ell_chain<kChainProlong>); break;
+  case kChainAddBoth: go(k_ell_chain<kChainAddBoth>); break;
+  }
+}
+
 // z = M^-1 v for the ILU(0) factor: mode 0 FP64 factor and sweeps; 1 FP32
 // factor, sweeps on FP32 vectors in FP32 arithmetic; 2 FP32 factor, sweeps
 // in FP64 (the reference built with HAVE_ILU_FLOAT: lusol's float alu
@@ -634,6 +827,10 @@ int ilu_sys_levels(gb300_matrix *A, int nsys, const int *off, const SysLevels **
 {
   GB_TRY(ilu_setup(A));
   ilu_data *L = A->ilu;
+  if(L->by_colour) {  // (its callers go by the colours)
+    set_error("ILU(0): no level lists on a multicolour copy");
+    return GB300_ERR_UNSUPPORTED;
+  }
   if(L->sys && (int)L->sys->off.size() == nsys + 1 &&
      std::equal(off, off + nsys + 1, L->sys->off.begin())) {
     *out = L->sys.get();
@@ -685,6 +882,7 @@ void ilu_factor_arrays(const gb300_matrix *A, bool fp32, const void **lu, const 
 // GMRES device state and kernels
 // ---------------------------------------------------------------------------
 constexpr int kMaxKrylov = 128;
+constexpr int kDotCols = 8;  // columns of one group of dot products
 
 struct GmState {
   int active;       // whole solve still running
@@ -701,15 +899,20 @@ struct GmState {
   double res;       // fpar(5)
   double res6;      // fpar(6)
   double rtol;
-  double scale;     // 1 / h(k+1,k) for the new basis vector
+  double scale;     // 1 / ||r|| at a restart (V_0 is normalised)
+  // vector j of the algorithm is sc[j] V_j: the basis vectors are left with
+  // the norm h(j+1,j) they come out of the Gram-Schmidt step with, the
+  // preconditioner and the product act on them as they are, and the scalars
+  // carry the normalisation (no pass over the vector scales it)
+  double sc[kMaxKrylov + 1];
   double H[(kMaxKrylov + 1) * kMaxKrylov];  // column-major, (m+1) x m
   double cs[kMaxKrylov], sn[kMaxKrylov], g[kMaxKrylov + 1], y[kMaxKrylov];
-  double h1[kMaxKrylov + 1], h2[kMaxKrylov + 1];
+  double h1[kMaxKrylov + 1], h2[kMaxKrylov + 1];  // the column of each pass
   double nrm0;      // ||w||^2 before the Gram-Schmidt pass of this step
   int reorth;       // this step takes a second Gram-Schmidt pass
   int reorths;      // second passes taken so far
   // arrival counters of the kernels whose last CTA finishes a reduction
-  unsigned tick_dots0, tick_dots1, tick_upd0, tick_upd1;
+  unsigned tick_dots[2][kMaxKrylov / kDotCols + 1], tick_upd[2];
 };
 
 // restart: r = rhs - A x was computed with its partial norms
@@ -743,209 +946,259 @@ __global__ void k_gm_restart(GmState *S, const double *__restrict__ part, int m)
     return;
   }
   S->scale = 1. / alpha;
+  S->sc[0] = 1.;
   S->cycle = 1;
 }
 
-// y = s * x, guarded by the cycle flag
-__global__ void k_gm_scale(int n, const GmState *__restrict__ S,
-                           const double *__restrict__ x, double *__restrict__ y)
+// y = s * x (s = *scale, or 1), guarded by *flag
+__global__ void k_gm_scale(int n, const double *scale, const double *x, double *y,
+                           const int *flag)
 {
-  if(!S->cycle) return;
-  double s = S->scale;
+  chain_wait();
+  if(flag && !*flag) return;
+  const double s = scale ? *scale : 1.;
   for(long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
       i += (long long)gridDim.x * blockDim.x)
-    y[i] = s * x[i];
+    y[i] = scale ? s * x[i] : x[i];
 }
 
-// partial dots <V_j, w>, j < k, over a fixed grid; part[j * B + block].
-// PASS 0 also forms <w, w> (as column k), the norm the selective
-// re-orthogonalisation compares with; PASS 1 runs only when this step
-// takes the second Gram-Schmidt pass.
-// the partial dots of columns [j0, j0 + CNT) over this CTA's share of rows
-template <int CNT>
-__device__ __forceinline__ void dots_group(int n, int j0, const double *__restrict__ V,
-                                           size_t ldv, const double *__restrict__ w,
-                                           double *__restrict__ part)
+__global__ void k_gm_add(int n, const double *t, double *z, const int *flag)
 {
-  double acc[8];
-#pragma unroll
-  for(int u = 0; u < 8; u++) acc[u] = 0.;
+  chain_wait();
+  if(flag && !*flag) return;
   for(long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-      i += (long long)gridDim.x * blockDim.x) {
-    double wi = w[i];
+      i += (long long)gridDim.x * blockDim.x)
+    z[i] += t[i];
+}
+
+// The dot products <V_j, w>, j < k, of one Gram-Schmidt pass.  blockIdx.y
+// takes a group of at most kDotCols columns (the groups as even as they can
+// be), so the groups run side by side and each FMA issued is needed;
+// blockIdx.x a share of the rows, its partial of column j in
+// part[j * kReduceBlocks + blockIdx.x].  PASS 0 also forms <w, w> (column k:
+// V_k is w), the norm the selective re-orthogonalisation compares with; PASS
+// 1 runs only when this step takes the second pass.  The last CTA of each
+// group sums its columns, one warp per column, in a fixed order (one CTA
+// summing every group's had been 10 of 22 us at 65,025 rows and k = 49).
+// Bound by the FP64 pipe: a warp's block sum costs as many FP64 instructions
+// as two rows of a group, so the grid is one CTA per SM over all groups.
+// The first rows are loaded before the guard is known.
+template <int CNT>
+__device__ __forceinline__ void dots_group(int n, int j0, const double *V, size_t ldv,
+                                           const double *w, double *part, bool go)
+{
+  double acc[kDotCols], x[CNT], wi = 0.;
 #pragma unroll
-    for(int u = 0; u < CNT; u++) acc[u] += V[(size_t)(j0 + u) * ldv + i] * wi;
+  for(int u = 0; u < kDotCols; u++) acc[u] = 0.;
+  const int stride = gridDim.x * blockDim.x;
+  const double *Vj = V + (size_t)j0 * ldv;
+  int i = blockIdx.x * blockDim.x + threadIdx.x;
+  auto load = [&]() {
+    wi = i < n ? w[i] : 0.;
+#pragma unroll
+    for(int u = 0; u < CNT; u++) x[u] = i < n ? Vj[(size_t)u * ldv + i] : 0.;
+  };
+  load();
+  if(!go) return;
+  while(i < n) {
+    double xc[CNT], wc = wi;
+#pragma unroll
+    for(int u = 0; u < CNT; u++) xc[u] = x[u];
+    i += stride;
+    load();  // the next row, in flight during this one's FMAs
+#pragma unroll
+    for(int u = 0; u < CNT; u++) acc[u] += xc[u] * wc;
   }
-  double s = block_sum8<256>(acc);
+  const double s = block_sum8<256>(acc);
   if(threadIdx.x < CNT) part[(size_t)(j0 + threadIdx.x) * kReduceBlocks + blockIdx.x] = s;
 }
 
-// end of one Arnoldi step (thread 0), with rr = ||w||^2 after the
-// Gram-Schmidt pass: h(k+1,k), Givens rotations, stopping test
-__device__ void gm_step_tail(GmState *S, int k, int m, double rr)
-{
-  S->its += 1;
-  double *Hc = S->H + (size_t)(k - 1) * (kMaxKrylov + 1);  // column k
-  double nrm = sqrt(rr);
-  Hc[k] = nrm;
-  S->k = k;
-  S->did_cycle = 1;
-  if(!(nrm > 0.)) {  // mgsro ierr -3: the new vector depends on the others
-    S->breakdown = -3;
-    S->cycle = 0;
-    return;
-  }
-  // previous rotations on the new column, then a new one
-  for(int i = 0; i < k - 1; i++) {
-    double a = Hc[i], c = S->cs[i], s = S->sn[i];
-    Hc[i] = c * a + s * Hc[i + 1];
-    Hc[i + 1] = c * Hc[i + 1] - s * a;
-  }
-  double c, s;
-  givens_dev(&Hc[k - 1], &Hc[k], &c, &s);
-  S->cs[k - 1] = c;
-  S->sn[k - 1] = s;
-  double alpha = -s * S->g[k - 1];
-  S->g[k - 1] = c * S->g[k - 1];
-  S->g[k] = alpha;
-  alpha = fabs(alpha);
-  S->res = alpha;
-  S->scale = 1. / nrm;
-  if(!(k < m && !(alpha <= S->tol) && (S->maxit <= 0 || S->its < S->maxit)))
-    S->cycle = 0;  // end of this cycle after the scaling below is skipped
-}
-
-// Partial dots <V_j, w>, j < k, over a fixed grid (part[j * B + block]);
-// blockIdx.y selects a group of (at most) eight columns, so the groups run
-// side by side and each FMA issued is needed.  PASS 0 also forms <w, w>
-// (column k: V_k is w), the norm the selective re-orthogonalisation
-// compares with; PASS 1 runs only when this step takes the second pass.
-// The last CTA to finish sums the partials in a fixed order (one warp per
-// column): PASS 0 stores h1 (and the column of H) and ||w||^2, PASS 1
-// stores h2 and adds it to the column.
 template <int PASS>
 __global__ void __launch_bounds__(256)
-k_gm_dots(int n, int k, const double *__restrict__ V, size_t ldv,
-          const double *__restrict__ w, double *__restrict__ part, GmState *S, int nb)
+k_gm_dots(int n, int k, const double *V, size_t ldv, const double *w, double *part, GmState *S)
 {
-  if(!S->cycle || (PASS == 1 && !S->reorth)) return;  // the same in every CTA
+  chain_wait();
+  // the same in every CTA
+  const bool go = PASS == 0 ? S->cycle != 0 : (S->cycle != 0) & (S->reorth != 0);
   const int kk = PASS == 0 ? k + 1 : k;  // column k: V_k = w itself
-  const int j0 = blockIdx.y * 8;
-  switch(j0 >= kk ? 0 : kk - j0 < 8 ? kk - j0 : 8) {
-  case 0: break;
-  case 1: dots_group<1>(n, j0, V, ldv, w, part); break;
-  case 2: dots_group<2>(n, j0, V, ldv, w, part); break;
-  case 3: dots_group<3>(n, j0, V, ldv, w, part); break;
-  case 4: dots_group<4>(n, j0, V, ldv, w, part); break;
-  case 5: dots_group<5>(n, j0, V, ldv, w, part); break;
-  case 6: dots_group<6>(n, j0, V, ldv, w, part); break;
-  case 7: dots_group<7>(n, j0, V, ldv, w, part); break;
-  default: dots_group<8>(n, j0, V, ldv, w, part); break;
+  const int j0 = (int)(blockIdx.y * kk / gridDim.y);
+  const int cnt = (int)((blockIdx.y + 1) * kk / gridDim.y) - j0;
+  if(PASS == 1 && !go) return;  // (rarely taken: no loads ahead)
+  switch(cnt) {
+  case 1: dots_group<1>(n, j0, V, ldv, w, part, go); break;
+  case 2: dots_group<2>(n, j0, V, ldv, w, part, go); break;
+  case 3: dots_group<3>(n, j0, V, ldv, w, part, go); break;
+  case 4: dots_group<4>(n, j0, V, ldv, w, part, go); break;
+  case 5: dots_group<5>(n, j0, V, ldv, w, part, go); break;
+  case 6: dots_group<6>(n, j0, V, ldv, w, part, go); break;
+  case 7: dots_group<7>(n, j0, V, ldv, w, part, go); break;
+  default: dots_group<8>(n, j0, V, ldv, w, part, go); break;
   }
-  if(!arrive_last(PASS == 0 ? &S->tick_dots0 : &S->tick_dots1)) return;
-  __shared__ double sums[kMaxKrylov + 1];
-  __shared__ int abnormal;
-  int wp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for(int j = wp; j < kk; j += blockDim.x / 32) {
-    double v = 0.;
-    for(int b = lane; b < nb; b += 32) v += __ldcg(part + (size_t)j * kReduceBlocks + b);
-    v = warp_sum(v);
-    if(lane == 0) sums[j] = v;
-  }
-  __syncthreads();
-  if(threadIdx.x == 0) {
-    abnormal = 0;
-    if(PASS == 0) {
-      // mgsro's checks on ||w||^2 before it orthogonalises (iters.f:
-      // 3475-3600): zero (ierr -1) or abnormal (-2) leaves the column
-      // unwritten and ends the cycle; gmres then reports a break-down
-      const double nrm0 = sums[k];
-      S->nrm0 = nrm0;
-      if(!(nrm0 > 0. && 1. / nrm0 > 0.)) {
-        abnormal = 1;
-        S->its += 1;  // the Arnoldi step's product was formed
-        S->breakdown = (nrm0 <= 0.) ? -1 : -2;
-        S->cycle = 0;
-      }
-    }
-  }
-  __syncthreads();
-  if(abnormal) return;
-  for(int j = threadIdx.x; j < k; j += blockDim.x) {
-    if(PASS == 0) {
-      S->h1[j] = sums[j];
-      S->H[(size_t)(k - 1) * (kMaxKrylov + 1) + j] = sums[j];
-    }
-    else {
-      S->h2[j] = sums[j];
-      S->H[(size_t)(k - 1) * (kMaxKrylov + 1) + j] = S->h1[j] + sums[j];
+  if(!go) return;
+  const int wp = threadIdx.x >> 5, lane = threadIdx.x & 31, j = j0 + wp;
+  // (the scales, on their way while the ticket is drawn; after the first
+  // pass w has its own scale)
+  const double sw = PASS == 0 ? S->sc[k - 1] : 1.;
+  const double sc = sw * (j < k ? S->sc[j] : sw);
+  if(!arrive_last(&S->tick_dots[PASS][blockIdx.y], gridDim.x)) return;
+  static_assert(kDotCols == 256 / 32, "one warp per column");
+  if(wp >= cnt) return;
+  double v = 0.;
+#pragma unroll 5
+  for(int b = lane; b < gridDim.x; b += 32) v += __ldcg(part + (size_t)j * kReduceBlocks + b);
+  v = warp_sum(v);
+  if(lane) return;
+  v *= sc;
+  if(j < k)
+    (PASS == 0 ? S->h1 : S->h2)[j] = v;
+  else {
+    // mgsro's checks on ||w||^2 before it orthogonalises (iters.f:3475-3600):
+    // zero (ierr -1) or abnormal (-2) leaves the column unwritten and ends
+    // the cycle; gmres then reports a break-down
+    S->nrm0 = v;
+    if(!(v > 0. && 1. / v > 0.)) {
+      S->its += 1;  // the Arnoldi step's product was formed
+      S->breakdown = (v <= 0.) ? -1 : -2;
+      S->cycle = 0;
     }
   }
 }
 
 // w -= sum_j h_j V_j (h of pass `pass`) with the partials of ||w||^2 in pn.
-// The last CTA to finish sums them.  After pass 0 it applies the selective
-// re-orthogonalisation test with mgsro's constant (iters.f:3475-3600,
-// reorth = 0.98: mgsro repeats the projection on one basis vector when it
-// removed more than 98 % of the squared norm left; here the second
+// CTA nb, beside the nb that do so, applies the previous Givens rotations to
+// the new Hessenberg column: they need the column only, not the norm, and
+// their serial chain (one FMA per rotation) hides behind the update (done
+// by one thread at the end of the step it had cost 18 us at k = 49).  The
+// last CTA to finish sums the partials.  After pass 0 it applies the
+// selective re-orthogonalisation test with mgsro's constant (iters.f:
+// 3475-3600, reorth = 0.98: mgsro repeats the projection on one basis vector
+// when it removed more than 98 % of the squared norm left; here the second
 // classical Gram-Schmidt pass runs when the first pass removed more than
 // 98 % of ||w||^2, ||w'|| < 0.14 ||w||; the loss of orthogonality of one
 // pass grows like eps ||w|| / ||w'||, so a pass that keeps more than 2 %
-// leaves w' orthogonal to within ~10 eps) and, without a second pass, ends
-// the Arnoldi step; after pass 1 it ends the step.
+// leaves w' orthogonal to within ~10 eps); without a second pass, or after
+// it, it ends the Arnoldi step: h(k+1,k), the new rotation, the stopping test.
 __global__ void __launch_bounds__(256)
-k_gm_update(int n, int k, int m, const double *__restrict__ V, size_t ldv,
-            double *__restrict__ w, double *__restrict__ pn, GmState *S, int pass, int nb)
+k_gm_update(int n, int k, int m, const double *V, size_t ldv, double *w, double *pn,
+            GmState *S, int pass)
 {
+  chain_wait();
   if(!S->cycle || (pass == 1 && !S->reorth)) return;  // the same in every CTA
-  __shared__ double h[kMaxKrylov];
-  for(int j = threadIdx.x; j < k; j += blockDim.x)
-    h[j] = pass == 0 ? S->h1[j] : S->h2[j];
-  __syncthreads();
-  double v = 0.;
-  for(long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-      i += (long long)gridDim.x * blockDim.x) {
-    // four partial sums of h_j V_j: four independent FMA chains instead of
-    // one (the FP64 FMA latency otherwise serialises the k terms)
-    double s0 = 0., s1 = 0., s2 = 0., s3 = 0.;
-    int j = 0;
-    for(; j + 3 < k; j += 4) {
-      s0 += h[j] * V[(size_t)j * ldv + i];
-      s1 += h[j + 1] * V[(size_t)(j + 1) * ldv + i];
-      s2 += h[j + 2] * V[(size_t)(j + 2) * ldv + i];
-      s3 += h[j + 3] * V[(size_t)(j + 3) * ldv + i];
+  const int nb = gridDim.x - 1;
+  __shared__ double h[kMaxKrylov + 1];
+  __shared__ double rc[kMaxKrylov], rs[kMaxKrylov], ra[kMaxKrylov];
+  double *Hc = S->H + (size_t)(k - 1) * (kMaxKrylov + 1);  // column k
+  if(blockIdx.x == nb) {
+    // rotation i: (a, b) -> (c a + s b, c b - s a) with b = h(i+1), the second
+    // the next rotation's a.  Everything but that chain in parallel.
+    const int j = threadIdx.x;
+    double c = 0., s = 0., b = 0.;
+    if(j < k) {
+      h[j] = S->h1[j] + (pass == 0 ? 0. : S->h2[j]);
+      c = S->cs[j];
+      s = S->sn[j];
     }
-    for(; j < k; j++) s0 += h[j] * V[(size_t)j * ldv + i];
-    double wi = w[i] - ((s0 + s1) + (s2 + s3));
-    w[i] = wi;
-    v += wi * wi;
+    __syncthreads();
+    if(j < k - 1) {
+      b = h[j + 1];
+      rc[j] = c * b;
+      rs[j] = s;
+    }
+    __syncthreads();
+    if(j == 0) {
+      double a = h[0];
+#pragma unroll 4
+      for(int i = 0; i < k - 1; i++) {
+        ra[i] = a;
+        a = fma(-rs[i], a, rc[i]);
+      }
+      ra[k - 1] = a;
+    }
+    __syncthreads();
+    if(j < k) Hc[j] = j < k - 1 ? fma(c, ra[j], s * b) : ra[j];
   }
-  double s = block_sum<double, 256>(v);
-  if(threadIdx.x == 0) pn[blockIdx.x] = s;
-  if(!arrive_last(pass == 0 ? &S->tick_upd0 : &S->tick_upd1)) return;
+  else {
+    for(int j = threadIdx.x; j < k; j += blockDim.x)
+      h[j] = -S->sc[j] * (pass == 0 ? S->h1[j] : S->h2[j]);
+    const double sw = pass == 0 ? S->sc[k - 1] : 1.;
+    __syncthreads();
+    double v = 0.;
+    for(int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += nb * blockDim.x) {
+      // two chains of FMAs, k + 3 FP64 instructions per row in all (FP64
+      // instructions pace the kernel; four chains and a separate subtraction
+      // took k + 6)
+      const double *Vi = V + i;
+      double s0 = sw * w[i], s1 = 0.;
+      int j = 0;
+#pragma unroll 4
+      for(; j + 1 < k; j += 2, Vi += 2 * ldv) {
+        s0 = fma(h[j], Vi[0], s0);
+        s1 = fma(h[j + 1], Vi[ldv], s1);
+      }
+      if(j < k) s0 = fma(h[j], Vi[0], s0);
+      s0 += s1;
+      w[i] = s0;
+      v = fma(s0, s0, v);
+    }
+    const double s = block_sum<double, 256>(v);
+    if(threadIdx.x == 0) pn[blockIdx.x] = s;
+  }
+  // what the end of the step reads, on its way while the ticket is drawn
+  const double nrm0 = S->nrm0, tol = S->tol, g = S->g[k - 1];
+  const int its = S->its, maxit = S->maxit;
+  if(!arrive_last(&S->tick_upd[pass], gridDim.x)) return;
+  const double hk = __ldcg(Hc + k - 1);
   double rr = 0.;
+#pragma unroll 4
   for(int i = threadIdx.x; i < nb; i += blockDim.x) rr += __ldcg(pn + i);
   rr = block_sum<double, 256>(rr);
   if(threadIdx.x) return;
   if(pass == 0) {
-    S->reorth = !(rr >= 0.02 * S->nrm0);
-    if(S->reorth) {
+    const bool again = !(rr >= 0.02 * nrm0);
+    S->reorth = again;
+    if(again) {
       S->reorths += 1;
       return;  // the step ends after the second pass
     }
   }
-  gm_step_tail(S, k, m, rr);
-}
-
-// scale the new basis vector (runs only while the cycle continues)
-__global__ void k_gm_scale_next(int n, const GmState *__restrict__ S,
-                                double *__restrict__ w, int k)
-{
-  if(!S->cycle || S->k != k) return;
-  double s = S->scale;
-  for(long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-      i += (long long)gridDim.x * blockDim.x)
-    w[i] *= s;
+  S->its = its + 1;
+  S->k = k;
+  S->did_cycle = 1;
+  if(!(rr > 0.)) {
+    // mgsro ierr -3: the new vector depends on the others; the reference
+    // solves with the column as mgsro left it, no rotation applied
+    for(int j = 0; j < k; j++) Hc[j] = S->h1[j] + (pass == 0 ? 0. : S->h2[j]);
+    Hc[k] = sqrt(rr);
+    S->breakdown = -3;
+    S->cycle = 0;
+    return;
+  }
+  // the rotation of (hk, nrm): givens (iters.f:3235-3273) in terms of two
+  // independent reciprocal roots, a third of the serial chain of its root,
+  // divisions and root (an FP64 division takes about 0.8 us here)
+  const double r2 = fma(hk, hk, rr);
+  double c, s;
+  if(rr > 1e-280 && r2 < 1e280) {
+    const double ri = rsqrt(rr), q = rsqrt(r2);
+    S->sc[k] = ri;
+    c = hk * q;
+    s = rr * ri * q;
+    Hc[k - 1] = r2 * q;
+  }
+  else {
+    double x = hk, y = sqrt(rr);
+    S->sc[k] = 1. / y;
+    givens_dev(&x, &y, &c, &s);
+    Hc[k - 1] = x;
+  }
+  S->cs[k - 1] = c;
+  S->sn[k - 1] = s;
+  S->g[k - 1] = c * g;
+  S->g[k] = -s * g;
+  const double alpha = fabs(-s * g);
+  S->res = alpha;
+  if(!(k < m && !(alpha <= tol) && (maxit <= 0 || its + 1 < maxit)))
+    S->cycle = 0;  // the end of this cycle
 }
 
 // end of a cycle: solve H y = g (upper triangular, k x k) on one thread
@@ -979,7 +1232,8 @@ k_gm_combine(int n, const double *__restrict__ V, size_t ldv,
   if(!S->active || !S->did_cycle) return;
   __shared__ double y[kMaxKrylov];
   int k = S->k;
-  for(int j = threadIdx.x; j < k; j += blockDim.x) y[j] = S->y[j];
+  for(int j = threadIdx.x; j < k; j += blockDim.x)
+    y[j] = S->y[j] * S->sc[j];
   __syncthreads();
   for(long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
       i += (long long)gridDim.x * blockDim.x) {
@@ -1020,9 +1274,6 @@ __global__ void k_gm_after(GmState *S)
   }
 }
 
-// flag pointer for the preconditioner inside a cycle: S->cycle
-static const int *cycle_flag(GmState *S) { return &S->cycle; }
-
 __global__ void k_gm_apply_ok(GmState *S, int *ok)
 {
   // the update's preconditioner runs when a solution update is due
@@ -1034,14 +1285,93 @@ bool correction_valid(const gb300_matrix *A)
   return A->corr_version == A->pattern_version && A->corr.p && A->nnz > 0;
 }
 
-// z <- z + G (v - A z): the learned correction after the ILU(0) step (two
-// fused products: t1 = v - A z, then z += G t1; t2 is not needed)
-void correction_apply(const gb300_matrix *A, const double *val, const double *v,
-                      double *z, double *t1, double *t2, const int *flag, cudaStream_t st)
+int PrecondScratch::alloc(const gb300_solver_params *p, int n,
+                          const std::function<void *(int, size_t)> &get)
 {
-  (void)t2;
-  resid_guarded(A, val, z, v, t1, flag, st);
-  spmv_add_guarded(A, A->corr.p, t1, z, flag, st);
+  const size_t b64 = sizeof(double) * (size_t)(n > 0 ? n : 1);
+  bool ok = true;
+  auto vec = [&](int slot) {
+    double *q = (double *)get(slot, b64);
+    ok = ok && q;
+    return q;
+  };
+  if(p->precision != 0) {
+    t32 = (float *)get(5, b64 / 2);
+    ok = ok && t32;
+  }
+  if(precond_learned(p->preconditioner)) t1 = vec(8);
+  if(precond_two_level(p->preconditioner)) {
+    t3 = vec(13);
+    t4 = vec(14);
+    t5 = vec(15);
+  }
+  return ok ? GB300_OK : GB300_ERR_CUDA;
+}
+
+void precond_run(const gb300_matrix *A, const double *val, const gb300_solver_params *p,
+                 const double *v, double *z, const PrecondScratch &s, const int *flag,
+                 cudaStream_t st)
+{
+  const int n = A->n, pc = p->preconditioner;
+  const bool learned = precond_learned(pc);
+  const bool learned_post = learned && pc != kPrecondLearnedCoarsePre;
+  const bool sai = (pc == kPrecondLearnedSai || pc == kPrecondSai);
+  const bool ilu = (pc == 6 || learned || precond_two_level(pc)) && !sai;
+  const ilu_data *L = ilu ? A->ilu : nullptr;
+  const int gs = grid_for(n, 256, kReduceBlocks * 4);
+  const bool early = chain_early(n);
+  if(!ilu && !sai) {  // no preconditioner
+    launch_chain(early, k_gm_scale, gs, 256, st, n, nullptr, v, z, flag);
+    return;
+  }
+  // out = S in (+ G (in - A out)), or added into out through tmp
+  auto smooth = [&](const double *in, double *out, double *tmp, bool add, bool corr) {
+    if(sai) {
+      spmv_chain(add ? kChainAdd : kChainMul, A, A->corr.p,
+                 {in, nullptr, out, nullptr, nullptr, nullptr, flag}, st);
+      return;
+    }
+    double *x = add ? tmp : out;
+    const bool sweep_adds = add && !corr;
+    const int mode = ilu_mode(p);
+    if(!L->by_colour) {
+      ilu_apply(A, mode, in, x, s.t32, flag, st);
+      if(sweep_adds) launch_chain(early, k_gm_add, gs, 256, st, n, (const double *)x, out, flag);
+    }
+    else if(mode == 0) {
+      if(sweep_adds)
+        colour_sweeps<2, double, double>(L, L->inv64.p, in, x, out, flag, st);
+      else
+        colour_sweeps<0, double, double>(L, L->inv64.p, in, x, nullptr, flag, st);
+    }
+    else if(mode == 2) {
+      if(sweep_adds)
+        colour_sweeps<2, float, double>(L, L->inv32.p, in, x, out, flag, st);
+      else
+        colour_sweeps<0, float, double>(L, L->inv32.p, in, x, nullptr, flag, st);
+    }
+    else {
+      if(sweep_adds)
+        colour_sweeps<2, float, float>(L, L->inv32.p, in, s.t32, out, flag, st);
+      else
+        colour_sweeps<1, float, float>(L, L->inv32.p, in, s.t32, x, flag, st);
+    }
+    if(corr) {
+      // the learned correction: t1 = in - A x, then x += G t1 (or both added
+      // into out)
+      product_chain(kChainRes, A, val, {x, in, s.t1, nullptr, nullptr, nullptr, flag}, st);
+      spmv_chain(add ? kChainAddBoth : kChainAdd, A, A->corr.p,
+                 {s.t1, x, add ? out : x, nullptr, nullptr, nullptr, flag}, st);
+    }
+  };
+  if(!precond_two_level(pc)) {
+    smooth(v, z, nullptr, false, learned);
+    return;
+  }
+  // z = S v;  z += P0 Ac^-1 P0^T (v - A z);  z += S (v - A z)
+  smooth(v, s.t5, nullptr, false, learned && !sai);
+  coarse_correct(A, val, v, s.t5, z, s.t3, flag, st);
+  smooth(s.t3, z, s.t4, true, learned_post && !sai);
 }
 
 int gmres_solve(gb300_matrix *A, const double *val, const double *rhs,
@@ -1065,7 +1395,6 @@ int gmres_solve(gb300_matrix *A, const double *val, const double *rhs,
   // the two-level cycle on aggregates around ILU(0) (22: and the correction)
   const bool learned = precond_learned(p->preconditioner);
   const bool coarse = precond_two_level(p->preconditioner);
-  const bool learned_post = learned && p->preconditioner != kPrecondLearnedCoarsePre;
   // 24: G alone smooths, no ILU(0); 25: with G the SPAI-1 made here
   const bool sai = (p->preconditioner == kPrecondLearnedSai ||
                     p->preconditioner == kPrecondSai);
@@ -1088,7 +1417,6 @@ int gmres_solve(gb300_matrix *A, const double *val, const double *rhs,
     return GB300_ERR_ARG;
   }
   bool fp32 = (p->precision != 0);
-  const int imode = ilu_mode(p);
   if(precond) {
     int zr = 0;
     // the factor is on A's values as given to the solver (scaled if needed)
@@ -1100,23 +1428,19 @@ int gmres_solve(gb300_matrix *A, const double *val, const double *rhs,
     }
   }
   if(coarse) GB_TRY(coarse_setup(A, val, p->re_use_lu != 0));
+  if(precond) GB_TRY(ilu_products(A, val));
   size_t ldv = (size_t)n;
   double *V = (double *)W.vec(0, sizeof(double) * ldv * (m + 1));
   double *Z = flexible ? (double *)W.vec(1, sizeof(double) * ldv * m) : nullptr;
-  double *r = (double *)W.vec(2, sizeof(double) * n);
   double *u = (double *)W.vec(3, sizeof(double) * n);
   double *zt = (double *)W.vec(4, sizeof(double) * n);
-  float *t32 = fp32 ? (float *)W.vec(5, sizeof(float) * n) : nullptr;
+  PrecondScratch ps;
+  GB_TRY(ps.alloc(p, n, [&](int slot, size_t bytes) { return W.vec(slot, bytes); }));
   double *part = (double *)W.vec(6, sizeof(double) * kReduceBlocks * (m + 1));
   double *pn = (double *)W.vec(12, sizeof(double) * kReduceBlocks);
   GmState *S = (GmState *)W.state(sizeof(GmState));
   int *okflag = (int *)W.vec(7, sizeof(int));
-  double *t1 = learned ? (double *)W.vec(8, sizeof(double) * n) : nullptr;
-  double *t2 = learned ? (double *)W.vec(9, sizeof(double) * n) : nullptr;
-  double *t3 = coarse ? (double *)W.vec(13, sizeof(double) * n) : nullptr;
-  double *t4 = coarse ? (double *)W.vec(14, sizeof(double) * n) : nullptr;
-  if(!V || (flexible && !Z) || !r || !u || !zt || (fp32 && !t32) || !part || !pn || !S ||
-     (learned && (!t1 || !t2)) || (coarse && (!t3 || !t4)))
+  if(!V || (flexible && !Z) || !u || !zt || !part || !pn || !S || !okflag)
     return GB300_ERR_CUDA;
   GmState h0;
   memset(&h0, 0, sizeof(h0));
@@ -1129,52 +1453,39 @@ int gmres_solve(gb300_matrix *A, const double *val, const double *rhs,
   GB_CUDA(cudaMemsetAsync(x, 0, sizeof(double) * n, st));  // sol = 0
 
   int gs = grid_for(n, 256, kReduceBlocks * 4);
-  // partial-sum blocks of the Arnoldi dot products: one per SM at least,
-  // one per 2048 rows up to kReduceBlocks (small systems keep the
-  // one-block reductions short); fixed for a given n, so deterministic
-  const int nb = std::min(kReduceBlocks, std::max(152, (n + 2047) / 2048));
-  auto smooth = [&](const double *v, double *z, const int *flag, bool corr) {
-    if(sai) {  // z = G v
-      spmv_guarded(A, A->corr.p, v, z, flag, st);
-      return;
-    }
-    if(precond)
-      ilu_apply(A, imode, v, z, t32, flag, st);
-    else
-      k_cvt<double, double><<<grid_for(n, 256), 256, 0, st>>>(n, v, z, flag);
-    if(corr) correction_apply(A, val, v, z, t1, t2, flag, st);
+  // row shares of the Gram-Schmidt kernels, fixed for a given n and k, so
+  // deterministic.  Dots: the groups' CTAs fill the SMs once (see k_gm_dots),
+  // twice from 200,000 rows on, where the loads need more warps.  Update:
+  // whole waves of 152, as many as leave a thread some 6 rows (512 CTAs on
+  // 152 SMs, 4 on some and 3 on others, took 85 us at 1,046,529 rows, k = 25)
+  const int rows256 = (n + 255) / 256;
+  auto dots_shares = [&](int groups) {
+    return std::max(1, std::min({rows256, 152 * (n > 200000 ? 2 : 1) / groups, kReduceBlocks}));
   };
-  auto precond_apply = [&](const double *v, double *z, const int *flag) {
-    if(!coarse) {
-      smooth(v, z, flag, learned);
-      return;
-    }
-    two_level_apply(A, val, v, z, t3, t4, flag, st,
-                    [&](const double *vv, double *zz) { smooth(vv, zz, flag, learned); },
-                    [&](const double *vv, double *zz) { smooth(vv, zz, flag, learned_post); });
-  };
-
+  const int nbu = std::min(rows256, 152 * std::min(8, std::max(1, n / (152 * 256 * 6))));
   cudaGraph_t graph;
   cudaGraphExec_t exec;
   GB_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-  // restart: r = rhs - A x, its norm, v1 = r / ||r||
-  residual64(A, val, x, rhs, r, part, st);
+  // restart: V_0 = (rhs - A x) / ||rhs - A x||
+  residual64(A, val, x, rhs, V, part, st);
   k_gm_restart<<<1, 256, 0, st>>>(S, part, m);
-  k_gm_scale<<<gs, 256, 0, st>>>(n, S, r, V);
+  k_gm_scale<<<gs, 256, 0, st>>>(n, &S->scale, V, V, &S->cycle);
   for(int k = 1; k <= m; k++) {
     double *vk = V + (size_t)(k - 1) * ldv;
     double *w = V + (size_t)k * ldv;
     double *z = flexible ? Z + (size_t)(k - 1) * ldv : zt;
-    precond_apply(vk, z, cycle_flag(S));
-    spmv_guarded(A, val, z, w, &S->cycle, st);
+    precond_run(A, val, p, vk, z, ps, &S->cycle, st);
+    product_chain(kChainMul, A, val, {z, nullptr, w, nullptr, nullptr, nullptr, &S->cycle}, st);
     // classical Gram-Schmidt, a second pass only when the test after the
     // first asks for it; the reductions, the test and the end of the step
     // run in the last CTA of each kernel
-    k_gm_dots<0><<<dim3(nb, (k + 1 + 7) / 8), 256, 0, st>>>(n, k, V, ldv, w, part, S, nb);
-    k_gm_update<<<nb, 256, 0, st>>>(n, k, m, V, ldv, w, pn, S, 0, nb);
-    k_gm_dots<1><<<dim3(nb, (k + 7) / 8), 256, 0, st>>>(n, k, V, ldv, w, part, S, nb);
-    k_gm_update<<<nb, 256, 0, st>>>(n, k, m, V, ldv, w, pn, S, 1, nb);
-    k_gm_scale_next<<<gs, 256, 0, st>>>(n, S, w, k);
+    const int g0 = k / kDotCols + 1, g1 = (k - 1) / kDotCols + 1;
+    launch_chain(false, k_gm_dots<0>, dim3(dots_shares(g0), g0), 256, st, n, k, V, ldv, w, part,
+                 S);
+    launch_chain(false, k_gm_update, nbu + 1, 256, st, n, k, m, V, ldv, w, pn, S, 0);
+    launch_chain(false, k_gm_dots<1>, dim3(dots_shares(g1), g1), 256, st, n, k, V, ldv, w, part,
+                 S);
+    launch_chain(false, k_gm_update, nbu + 1, 256, st, n, k, m, V, ldv, w, pn, S, 1);
   }
   k_gm_solve_small<<<1, 32, 0, st>>>(S);
   if(flexible)
@@ -1182,7 +1493,7 @@ int gmres_solve(gb300_matrix *A, const double *val, const double *rhs,
   else {
     k_gm_combine<0><<<gs, 256, 0, st>>>(n, V, ldv, u, S);
     k_gm_apply_ok<<<1, 32, 0, st>>>(S, okflag);
-    precond_apply(u, zt, okflag);
+    precond_run(A, val, p, u, zt, ps, okflag, st);
     k_gm_addto<<<gs, 256, 0, st>>>(n, zt, x, S);
   }
   k_gm_after<<<1, 32, 0, st>>>(S);

@@ -114,8 +114,17 @@ constexpr int kAutoAggregates = 1024;
 int coarse_follow(const gb300_matrix *A, gb300_matrix *B, const Colouring *C,
                   cudaStream_t st);
 int coarse_setup(gb300_matrix *A, const double *val, bool reuse);
-void coarse_correct(const gb300_matrix *A, const double *val, const double *v, double *z,
-                    double *t, const int *flag, cudaStream_t st);
+// one coarse correction: t = v - A z, then out = z + P0 Ac^-1 P0^T t and
+// t = v - A out
+void coarse_correct(const gb300_matrix *A, const double *val, const double *v,
+                    const double *z, double *out, double *t, const int *flag,
+                    cudaStream_t st);
+// spmv_chain on A's values val: from the sliced-ELL copy of a multicolour
+// copy's rows where ilu_products has made one of val, else from the CSR
+void product_chain(ChainMode mode, const gb300_matrix *A, const double *val,
+                   const ChainArgs &a, cudaStream_t st);
+// (re)make that copy for the values val; A's ILU(0) is set up
+int ilu_products(gb300_matrix *A, const double *val);
 // w <- (I - A C) w and *wcw = w^T C w (device scalar), C = P0 Ac^-1 P0^T on
 // A's own values (the coarse inverse made once and then reused; t, q: n
 // doubles of scratch) -- the two-level form of the learned correction's loss
@@ -123,14 +132,21 @@ int coarse_energy_project(gb300_matrix *A, double *w, double *t, double *q, doub
                           cudaStream_t st);
 // *ucu_dev = u^T C u (same coarse inverse as coarse_energy_project)
 int coarse_energy(gb300_matrix *A, const double *u, double *ucu_dev, cudaStream_t st);
-// smooth: the first smoothing, smooth_post: the second
-void two_level_apply(const gb300_matrix *A, const double *val, const double *v, double *z,
-                     double *t3, double *t4, const int *flag, cudaStream_t st,
-                     const std::function<void(const double *, double *)> &smooth,
-                     const std::function<void(const double *, double *)> &smooth_post);
 bool correction_valid(const gb300_matrix *A);
-void correction_apply(const gb300_matrix *A, const double *val, const double *v,
-                      double *z, double *t1, double *t2, const int *flag, cudaStream_t st);
+// scratch vectors of one preconditioner application
+struct PrecondScratch {
+  float *t32 = nullptr;    // FP32 sweeps
+  double *t1 = nullptr;    // residual of the learned correction
+  double *t3 = nullptr, *t4 = nullptr, *t5 = nullptr;  // two-level cycle
+  // get(slot, bytes): a device buffer, or null
+  int alloc(const gb300_solver_params *p, int n, const std::function<void *(int, size_t)> &get);
+};
+// z = M^-1 v for the preconditioner of p (Preconditioner 0, 6, 20-25; the
+// factor, correction and coarse inverse already made), guarded by *flag
+// (null: always); z distinct from v
+void precond_run(const gb300_matrix *A, const double *val, const gb300_solver_params *p,
+                 const double *v, double *z, const PrecondScratch &s, const int *flag,
+                 cudaStream_t st);
 
 // ILU(0) of A's pattern on the values val (FP64, or FP32 storage), and its
 // application z = M^-1 v guarded by *flag (gmres.cu)

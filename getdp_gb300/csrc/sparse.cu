@@ -513,10 +513,6 @@ k_spmv(int n, const int *__restrict__ rowptr, const int *__restrict__ col,
         y[row] = r;
         red += r * r;
       }
-      else if(MODE == 3)  // y += A x
-        y[row] += sum;
-      else if(MODE == 4)  // y = b - A x, no partial sums
-        y[row] = b[row] - sum;
       else {
         y[row] = sum;
         if(MODE == 2) red += x[row] * sum;
@@ -537,7 +533,7 @@ static void launch_spmv(const gb300_matrix *A, const V *val, const XT *x,
   int n = A->n;
   int rows_per_block_64 = 256 / A->tpr;
   // modes with partial sums (1, 2) run on the fixed reduction grid
-  constexpr bool kFree = (MODE == 0 || MODE == 3 || MODE == 4);
+  constexpr bool kFree = (MODE == 0);
   int blocks = kFree ? grid_for(n, rows_per_block_64, 1 << 30) : kReduceBlocks;
   if(kFree && blocks > 152 * 64) blocks = 152 * 64;
   switch(A->tpr) {
@@ -589,20 +585,86 @@ void spmv_plain(const gb300_matrix *A, const double *val, const double *x,
 {
   launch_spmv<0, double, double>(A, val, x, nullptr, y, nullptr, st);
 }
-void spmv_guarded(const gb300_matrix *A, const double *val, const double *x,
-                  double *y, const int *flag, cudaStream_t st)
+// A row's first U entries per lane are loaded before the wait for the
+// preceding kernel (the matrix does not change during a solve), and the guard
+// is tested after the gathers are on their way: such a product is bound by its
+// chain of dependent loads, not by bytes, up to some 100,000 rows
+template <int TPR, int MODE>
+__global__ void __launch_bounds__(256)
+k_spmv_chain(int n, const int *__restrict__ rowptr, const int *__restrict__ col,
+             const double *__restrict__ val, ChainArgs a)
 {
-  launch_spmv<0, double, double>(A, val, x, nullptr, y, nullptr, st, flag);
+  constexpr int U = TPR >= 8 ? 2 : 4;
+  const int lane = threadIdx.x % TPR;
+  const long long row = (long long)blockIdx.x * (256 / TPR) + threadIdx.x / TPR;
+  int c[U], g[U], k0 = 0, e = 0;
+  double v[U];
+  if(row < n) {
+    k0 = rowptr[row] + lane;
+    e = rowptr[row + 1];
+  }
+  auto load = [&](int k) {
+#pragma unroll
+    for(int u = 0; u < U; u++) {
+      const int kk = k + u * TPR;
+      c[u] = kk < e ? __ldcs(col + kk) : -1;
+      v[u] = kk < e ? __ldcs(val + kk) : 0.;
+      if(MODE == kChainProlong) g[u] = kk < e ? a.agg[c[u]] : 0;
+    }
+  };
+  load(k0);
+  const int grow = (MODE == kChainProlong && row < n) ? a.agg[row] : 0;
+  chain_wait();
+  const int go = a.flag ? *a.flag : 1;
+  double sum = 0.;
+  for(;;) {
+    double xv[U];
+#pragma unroll
+    for(int u = 0; u < U; u++) {
+      xv[u] = c[u] >= 0 ? a.x[c[u]] : 0.;
+      if(MODE == kChainProlong && c[u] >= 0) xv[u] += a.ec[g[u]];
+    }
+    if(!go) return;  // (the same in every thread)
+#pragma unroll
+    for(int u = 0; u < U; u++)
+      if(c[u] >= 0) sum += v[u] * xv[u];
+    k0 += U * TPR;
+    if(k0 >= e) break;
+    load(k0);
+  }
+#pragma unroll
+  for(int o = TPR / 2; o > 0; o >>= 1) sum += __shfl_down_sync(0xffffffffu, sum, o, TPR);
+  if(lane == 0 && row < n) chain_store<MODE>(a, row, grow, sum);
 }
-void spmv_add_guarded(const gb300_matrix *A, const double *val, const double *x,
-                      double *y, const int *flag, cudaStream_t st)
+
+template <int MODE>
+static void launch_spmv_chain(const gb300_matrix *A, const double *val, const ChainArgs &a,
+                              cudaStream_t st)
 {
-  launch_spmv<3, double, double>(A, val, x, nullptr, y, nullptr, st, flag);
+  const int n = A->n;
+  auto go = [&](auto kernel, int tpr) {
+    launch_chain(chain_early(n), kernel, grid_for(n, 256 / tpr), 256, st, n, A->rowptr.p,
+                 A->col.p, val, a);
+  };
+  switch(A->tpr) {
+  case 2: go(k_spmv_chain<2, MODE>, 2); break;
+  case 4: go(k_spmv_chain<4, MODE>, 4); break;
+  case 8: go(k_spmv_chain<8, MODE>, 8); break;
+  case 16: go(k_spmv_chain<16, MODE>, 16); break;
+  default: go(k_spmv_chain<32, MODE>, 32); break;
+  }
 }
-void resid_guarded(const gb300_matrix *A, const double *val, const double *x,
-                   const double *b, double *r, const int *flag, cudaStream_t st)
+
+void spmv_chain(ChainMode mode, const gb300_matrix *A, const double *val, const ChainArgs &a,
+                cudaStream_t st)
 {
-  launch_spmv<4, double, double>(A, val, x, b, r, nullptr, st, flag);
+  switch(mode) {
+  case kChainMul: launch_spmv_chain<kChainMul>(A, val, a, st); break;
+  case kChainAdd: launch_spmv_chain<kChainAdd>(A, val, a, st); break;
+  case kChainRes: launch_spmv_chain<kChainRes>(A, val, a, st); break;
+  case kChainProlong: launch_spmv_chain<kChainProlong>(A, val, a, st); break;
+  case kChainAddBoth: launch_spmv_chain<kChainAddBoth>(A, val, a, st); break;
+  }
 }
 
 // sum of the fixed-size partial array, in a fixed order, into *out

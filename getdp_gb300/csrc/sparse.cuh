@@ -19,13 +19,40 @@ int build_csr_from_coo(gb300_matrix *A, long long m, const int *d_r,
 void spmv64(const gb300_matrix *A, const double *x, double *y, cudaStream_t st);
 void spmv_plain(const gb300_matrix *A, const double *val, const double *x,
                 double *y, cudaStream_t st);
-void spmv_guarded(const gb300_matrix *A, const double *val, const double *x,
-                  double *y, const int *flag, cudaStream_t st);
-// y += A x, and r = b - A x without partial sums (guarded by *flag)
-void spmv_add_guarded(const gb300_matrix *A, const double *val, const double *x,
-                      double *y, const int *flag, cudaStream_t st);
-void resid_guarded(const gb300_matrix *A, const double *val, const double *x,
-                   const double *b, double *r, const int *flag, cudaStream_t st);
+// The products of a Krylov step, launched as a chain (launch_chain) and
+// guarded by *flag (null: always):
+//   kChainMul     y = A x
+//   kChainAdd     y += A x
+//   kChainRes     y = b - A x
+//   kChainProlong x2 = x + ec[agg], y = b - A x2
+//   kChainAddBoth y += b + A x
+enum ChainMode { kChainMul, kChainAdd, kChainRes, kChainProlong, kChainAddBoth };
+struct ChainArgs {
+  const double *x, *b;
+  double *y;
+  const int *agg;
+  const double *ec;
+  double *x2;
+  const int *flag;
+};
+void spmv_chain(ChainMode mode, const gb300_matrix *A, const double *val, const ChainArgs &a,
+                cudaStream_t st);
+// the row's result (sum: its product), one thread per row
+template <int MODE>
+__device__ __forceinline__ void chain_store(const ChainArgs &a, size_t row, int grow,
+                                            double sum)
+{
+  if(MODE == kChainMul)
+    a.y[row] = sum;
+  else if(MODE == kChainAdd)
+    a.y[row] += sum;
+  else if(MODE == kChainAddBoth)
+    a.y[row] += a.b[row] + sum;
+  else {
+    a.y[row] = a.b[row] - sum;
+    if(MODE == kChainProlong) a.x2[row] = a.x[row] + a.ec[grow];
+  }
+}
 void residual64(const gb300_matrix *A, const double *val, const double *x,
                 const double *b, double *r, double *part, cudaStream_t st);
 void residual64_guarded(const gb300_matrix *A, const double *val,

@@ -1,0 +1,117 @@
+"""The Krylov step's kernels at the edges of their blocks: column groups of
+eight (restart lengths around multiples), row counts around warps and CTAs,
+one to twelve colours, rows longer than the entries a sweep loads ahead, the
+second Gram-Schmidt pass, and both sides of the early-start rule.
+
+Every matrix is strictly diagonally dominant by rows with unit diagonal and an
+off-diagonal row sum of at most 1/2, so ||A^-1||_inf <= 2 and ||A||_inf <= 3/2:
+a residual of 1e-12 ||b||_2 bounds the error by 2 sqrt(n) 1e-12 ||b||_2, and
+||b||_2 <= 1.5 sqrt(n) ||x||_2; the bound asserted is ten times 3 n 1e-12 or, for
+the large systems, measured against the solution the right-hand side was made of
+with the residual bound 1e-10."""
+import numpy as np
+import pytest
+import scipy.sparse as sp
+
+from getdp_gb300 import linalg as LA
+
+pytestmark = pytest.mark.gpu
+
+
+def _dominant(S, seed, weight=0.5):
+    """Random values on S's symmetric pattern, unit diagonal, off-diagonal row
+    sums of `weight`."""
+    S = sp.csr_matrix(S)
+    S.setdiag(0)
+    S.eliminate_zeros()
+    S = ((S + S.T) != 0).astype(float).tocsr()
+    rng = np.random.default_rng(seed)
+    S.data = rng.uniform(0.2, 1.0, S.nnz) * rng.choice([-1.0, 1.0], S.nnz)
+    s = np.asarray(abs(S).sum(axis=1)).ravel()
+    S = sp.diags(weight / np.where(s > 0, s, 1.0)) @ S
+    A = (S + sp.identity(S.shape[0])).tocsr()
+    A.sort_indices()
+    return A
+
+
+def _grid(m, diagonals):
+    T = sp.diags([np.ones(m - 1), np.ones(m - 1)], [-1, 1])
+    E = sp.identity(m)
+    S = sp.kron(E, T) + sp.kron(T, E)
+    if diagonals:
+        S = S + sp.kron(sp.diags([np.ones(m - 1)], [1]), sp.diags([np.ones(m - 1)], [1]))
+    return S
+
+
+def _solve(A, par, seed=1):
+    n = A.shape[0]
+    x0 = np.random.default_rng(seed).standard_normal(n)
+    G, b, x = LA.gMatrix(n), LA.gVector(n), LA.gVector(n)
+    G.set_csr(A.indptr, A.indices, A.data)
+    b.set(A @ x0)
+    S = LA.LinAlg_CreateSolver(None)
+    for k, v in dict(Algorithm=8, Preconditioner=6, Krylov_Size=30, Nb_Iter_Max=2000,
+                     Renumbering_Technique=1).items():
+        S.set(k, par.get(k, v))
+    S.set("Precision", par.get("Precision", 0))
+    S["stopping_test"] = 1e-12
+    info = LA.LinAlg_Solve(G, b, S, x)
+    # (one colour: the factor is exact and the first step may end with a vector
+    # of exactly zero, mgsro's code -3, at the solution)
+    exact = info["status"] == -3 and info["true_residual"] <= 1e-13 * info["rhs_norm"]
+    assert info["status"] == 0 or exact, info
+    assert info["true_residual"] <= 1e-10 * info["rhs_norm"], info
+    assert np.linalg.norm(x.numpy() - x0) <= 30 * max(n, 34) * 1e-12 * np.linalg.norm(x0)
+    return info
+
+
+PATTERNS = {
+    "one": lambda: sp.identity(1),
+    "diagonal": lambda: sp.identity(77),
+    "path31": lambda: sp.diags([np.ones(30)], [1]),
+    "path257": lambda: sp.diags([np.ones(256)], [1]),
+    "grid5": lambda: _grid(23, False),
+    "grid7": lambda: _grid(33, True),
+    "cliques": lambda: sp.kron(sp.identity(27), np.ones((12, 12))) +
+    sp.kron(sp.diags([np.ones(26)], [1]), np.eye(12)),
+}
+
+
+@pytest.mark.parametrize("name", sorted(PATTERNS))
+@pytest.mark.parametrize("algorithm,precision", [(8, 0), (9, 0), (9, 1), (8, 2)])
+def test_colour_sweeps(name, algorithm, precision):
+    _solve(_dominant(PATTERNS[name](), 3), {"Algorithm": algorithm, "Precision": precision})
+
+
+@pytest.mark.parametrize("m", [2, 7, 8, 9, 15, 16, 17, 64, 128])
+def test_restart_lengths(m):
+    # a weakly dominant system takes enough steps to fill the groups
+    _solve(_dominant(_grid(31, True), 5, 0.5), {"Krylov_Size": m, "Preconditioner": 0})
+
+
+def test_second_pass():
+    # A near the identity: a step's product lies almost in the span of the
+    # basis, so the first pass removes more than 98 % of it every time
+    info = _solve(_dominant(_grid(40, True), 7, 0.05), {"Preconditioner": 0, "Krylov_Size": 20})
+    assert info["iterations"] > 3
+
+
+@pytest.mark.parametrize("side", [361, 363])
+def test_both_sides_of_the_early_start(side):
+    # 130,321 and 131,769 rows: the chain starts early up to 131,072
+    A = _dominant(_grid(side, True), 11)
+    n = A.shape[0]
+    x0 = np.random.default_rng(2).standard_normal(n)
+    G, b, x = LA.gMatrix(n), LA.gVector(n), LA.gVector(n)
+    G.set_csr(A.indptr, A.indices, A.data)
+    b.set(A @ x0)
+    S = LA.LinAlg_CreateSolver(None)
+    for k, v in dict(Algorithm=8, Preconditioner=6, Krylov_Size=30, Nb_Iter_Max=500,
+                     Renumbering_Technique=1).items():
+        S.set(k, v)
+    S["stopping_test"] = 1e-12
+    info = LA.LinAlg_Solve(G, b, S, x)
+    assert info["status"] == 0 and info["true_residual"] <= 1e-10 * info["rhs_norm"], info
+    # 2-norm: ||A^-1||_2 <= 2 sqrt(n) would be far from sharp; the residual
+    # bound and the condition number of a dominant matrix (<= 3) give
+    assert np.linalg.norm(x.numpy() - x0) <= 10 * 3 * 1e-10 * np.linalg.norm(x0)
