@@ -950,16 +950,19 @@ __global__ void k_gm_restart(GmState *S, const double *__restrict__ part, int m)
   S->cycle = 1;
 }
 
-// y = s * x (s = *scale, or 1), guarded by *flag
-__global__ void k_gm_scale(int n, const double *scale, const double *x, double *y,
+// y = x, or y = y2 = s x with s = *scale, guarded by *flag
+__global__ void k_gm_scale(int n, const double *scale, const double *x, double *y, double *y2,
                            const int *flag)
 {
   chain_wait();
   if(flag && !*flag) return;
   const double s = scale ? *scale : 1.;
   for(long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-      i += (long long)gridDim.x * blockDim.x)
-    y[i] = scale ? s * x[i] : x[i];
+      i += (long long)gridDim.x * blockDim.x) {
+    const double v = scale ? s * x[i] : x[i];
+    y[i] = v;
+    if(y2) y2[i] = v;
+  }
 }
 
 __global__ void k_gm_add(int n, const double *t, double *z, const int *flag)
@@ -971,35 +974,36 @@ __global__ void k_gm_add(int n, const double *t, double *z, const int *flag)
     z[i] += t[i];
 }
 
-// The dot products <V_j, w>, j < k, of one Gram-Schmidt pass.  blockIdx.y
-// takes a group of at most kDotCols columns (the groups as even as they can
-// be), so the groups run side by side and each FMA issued is needed;
-// blockIdx.x a share of the rows, its partial of column j in
-// part[j * kReduceBlocks + blockIdx.x].  PASS 0 also forms <w, w> (column k:
+// The dot products <V_j, w>, j < k, of one Gram-Schmidt pass, k - 1 the steps
+// taken in this cycle (read from the state, so that one captured step serves
+// them all).  The CTAs are dealt to groups of at most kDotCols columns (the
+// groups as even as they can be), which run side by side, and within a group
+// to shares of the rows, the partial of column j and share b in
+// part[j * kReduceBlocks + b]; CTAs left over return.  PASS 0 also forms <w, w> (column k:
 // V_k is w), the norm the selective re-orthogonalisation compares with; PASS
 // 1 runs only when this step takes the second pass.  The last CTA of each
 // group sums its columns, one warp per column, in a fixed order (one CTA
 // summing every group's had been 10 of 22 us at 65,025 rows and k = 49).
 // Bound by the FP64 pipe: a warp's block sum costs as many FP64 instructions
 // as two rows of a group, so the grid is one CTA per SM over all groups.
-// The first rows are loaded before the guard is known.
 template <int CNT>
-__device__ __forceinline__ void dots_group(int n, int j0, const double *V, size_t ldv,
-                                           const double *w, double *part, bool go)
+__device__ __forceinline__ void dots_group(int n, int j0, int k, int share, int shares,
+                                           const double *V, size_t ldv, const double *w,
+                                           double *part)
 {
   double acc[kDotCols], x[CNT], wi = 0.;
 #pragma unroll
   for(int u = 0; u < kDotCols; u++) acc[u] = 0.;
-  const int stride = gridDim.x * blockDim.x;
+  const int stride = shares * blockDim.x;
   const double *Vj = V + (size_t)j0 * ldv;
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
+  int i = share * blockDim.x + threadIdx.x;
   auto load = [&]() {
     wi = i < n ? w[i] : 0.;
 #pragma unroll
-    for(int u = 0; u < CNT; u++) x[u] = i < n ? Vj[(size_t)u * ldv + i] : 0.;
+    for(int u = 0; u < CNT; u++)  // column k is w
+      x[u] = i < n ? (u == CNT - 1 && j0 + u == k ? wi : Vj[(size_t)u * ldv + i]) : 0.;
   };
   load();
-  if(!go) return;
   while(i < n) {
     double xc[CNT], wc = wi;
 #pragma unroll
@@ -1010,42 +1014,45 @@ __device__ __forceinline__ void dots_group(int n, int j0, const double *V, size_
     for(int u = 0; u < CNT; u++) acc[u] += xc[u] * wc;
   }
   const double s = block_sum8<256>(acc);
-  if(threadIdx.x < CNT) part[(size_t)(j0 + threadIdx.x) * kReduceBlocks + blockIdx.x] = s;
+  if(threadIdx.x < CNT) part[(size_t)(j0 + threadIdx.x) * kReduceBlocks + share] = s;
 }
 
 template <int PASS>
 __global__ void __launch_bounds__(256)
-k_gm_dots(int n, int k, const double *V, size_t ldv, const double *w, double *part, GmState *S)
+k_gm_dots(int n, const double *V, size_t ldv, const double *w, double *part, GmState *S)
 {
   chain_wait();
-  // the same in every CTA
-  const bool go = PASS == 0 ? S->cycle != 0 : (S->cycle != 0) & (S->reorth != 0);
-  const int kk = PASS == 0 ? k + 1 : k;  // column k: V_k = w itself
-  const int j0 = (int)(blockIdx.y * kk / gridDim.y);
-  const int cnt = (int)((blockIdx.y + 1) * kk / gridDim.y) - j0;
-  if(PASS == 1 && !go) return;  // (rarely taken: no loads ahead)
+  const int go = S->cycle, again = S->reorth, k = S->k + 1;
+  if(!go || (PASS == 1 && !again)) return;  // the same in every CTA
+  const int kk = PASS == 0 ? k + 1 : k;     // column k: V_k = w itself
+  const int groups = (kk - 1) / kDotCols + 1;
+  const int grp = (int)blockIdx.x % groups, share = (int)blockIdx.x / groups;
+  const int rows256 = (n + 255) / 256, most = (int)gridDim.x / groups;
+  const int shares = rows256 < most ? rows256 : most;
+  if(share >= shares) return;
+  const int j0 = grp * kk / groups;
+  const int cnt = (grp + 1) * kk / groups - j0;
   switch(cnt) {
-  case 1: dots_group<1>(n, j0, V, ldv, w, part, go); break;
-  case 2: dots_group<2>(n, j0, V, ldv, w, part, go); break;
-  case 3: dots_group<3>(n, j0, V, ldv, w, part, go); break;
-  case 4: dots_group<4>(n, j0, V, ldv, w, part, go); break;
-  case 5: dots_group<5>(n, j0, V, ldv, w, part, go); break;
-  case 6: dots_group<6>(n, j0, V, ldv, w, part, go); break;
-  case 7: dots_group<7>(n, j0, V, ldv, w, part, go); break;
-  default: dots_group<8>(n, j0, V, ldv, w, part, go); break;
+  case 1: dots_group<1>(n, j0, k, share, shares, V, ldv, w, part); break;
+  case 2: dots_group<2>(n, j0, k, share, shares, V, ldv, w, part); break;
+  case 3: dots_group<3>(n, j0, k, share, shares, V, ldv, w, part); break;
+  case 4: dots_group<4>(n, j0, k, share, shares, V, ldv, w, part); break;
+  case 5: dots_group<5>(n, j0, k, share, shares, V, ldv, w, part); break;
+  case 6: dots_group<6>(n, j0, k, share, shares, V, ldv, w, part); break;
+  case 7: dots_group<7>(n, j0, k, share, shares, V, ldv, w, part); break;
+  default: dots_group<8>(n, j0, k, share, shares, V, ldv, w, part); break;
   }
-  if(!go) return;
   const int wp = threadIdx.x >> 5, lane = threadIdx.x & 31, j = j0 + wp;
   // (the scales, on their way while the ticket is drawn; after the first
   // pass w has its own scale)
   const double sw = PASS == 0 ? S->sc[k - 1] : 1.;
   const double sc = sw * (j < k ? S->sc[j] : sw);
-  if(!arrive_last(&S->tick_dots[PASS][blockIdx.y], gridDim.x)) return;
+  if(!arrive_last(&S->tick_dots[PASS][grp], shares)) return;
   static_assert(kDotCols == 256 / 32, "one warp per column");
   if(wp >= cnt) return;
   double v = 0.;
 #pragma unroll 5
-  for(int b = lane; b < gridDim.x; b += 32) v += __ldcg(part + (size_t)j * kReduceBlocks + b);
+  for(int b = lane; b < shares; b += 32) v += __ldcg(part + (size_t)j * kReduceBlocks + b);
   v = warp_sum(v);
   if(lane) return;
   v *= sc;
@@ -1064,7 +1071,10 @@ k_gm_dots(int n, int k, const double *V, size_t ldv, const double *w, double *pa
   }
 }
 
-// w -= sum_j h_j V_j (h of pass `pass`) with the partials of ||w||^2 in pn.
+// V_k = cur = w - sum_j h_j V_j (h of pass `pass`; pass 1: w is cur) with the
+// partials of ||V_k||^2 in pn.  cur is the copy of the newest basis vector
+// that the next step's preconditioner reads at a fixed address; for FGMRES
+// pass 0 also keeps the preconditioned vector zt as Z_{k-1}.
 // CTA nb, beside the nb that do so, applies the previous Givens rotations to
 // the new Hessenberg column: they need the column only, not the norm, and
 // their serial chain (one FMA per rotation) hides behind the update (done
@@ -1079,11 +1089,12 @@ k_gm_dots(int n, int k, const double *V, size_t ldv, const double *w, double *pa
 // leaves w' orthogonal to within ~10 eps); without a second pass, or after
 // it, it ends the Arnoldi step: h(k+1,k), the new rotation, the stopping test.
 __global__ void __launch_bounds__(256)
-k_gm_update(int n, int k, int m, const double *V, size_t ldv, double *w, double *pn,
-            GmState *S, int pass)
+k_gm_update(int n, int m, double *V, size_t ldv, const double *w, double *cur,
+            const double *zt, double *Z, double *pn, GmState *S, int pass)
 {
   chain_wait();
-  if(!S->cycle || (pass == 1 && !S->reorth)) return;  // the same in every CTA
+  const int go = S->cycle, again = S->reorth, k = S->k + 1;
+  if(!go || (pass == 1 && !again)) return;  // the same in every CTA
   const int nb = gridDim.x - 1;
   __shared__ double h[kMaxKrylov + 1];
   __shared__ double rc[kMaxKrylov], rs[kMaxKrylov], ra[kMaxKrylov];
@@ -1137,7 +1148,9 @@ k_gm_update(int n, int k, int m, const double *V, size_t ldv, double *w, double 
       }
       if(j < k) s0 = fma(h[j], Vi[0], s0);
       s0 += s1;
-      w[i] = s0;
+      V[(size_t)k * ldv + i] = s0;
+      cur[i] = s0;
+      if(Z && pass == 0) Z[(size_t)(k - 1) * ldv + i] = zt[i];
       v = fma(s0, s0, v);
     }
     const double s = block_sum<double, 256>(v);
@@ -1154,9 +1167,9 @@ k_gm_update(int n, int k, int m, const double *V, size_t ldv, double *w, double 
   rr = block_sum<double, 256>(rr);
   if(threadIdx.x) return;
   if(pass == 0) {
-    const bool again = !(rr >= 0.02 * nrm0);
-    S->reorth = again;
-    if(again) {
+    const bool more = !(rr >= 0.02 * nrm0);
+    S->reorth = more;
+    if(more) {
       S->reorths += 1;
       return;  // the step ends after the second pass
     }
@@ -1321,7 +1334,7 @@ void precond_run(const gb300_matrix *A, const double *val, const gb300_solver_pa
   const int gs = grid_for(n, 256, kReduceBlocks * 4);
   const bool early = chain_early(n);
   if(!ilu && !sai) {  // no preconditioner
-    launch_chain(early, k_gm_scale, gs, 256, st, n, nullptr, v, z, flag);
+    launch_chain(early, k_gm_scale, gs, 256, st, n, nullptr, v, z, nullptr, flag);
     return;
   }
   // out = S in (+ G (in - A out)), or added into out through tmp
@@ -1433,6 +1446,8 @@ int gmres_solve(gb300_matrix *A, const double *val, const double *rhs,
   double *V = (double *)W.vec(0, sizeof(double) * ldv * (m + 1));
   double *Z = flexible ? (double *)W.vec(1, sizeof(double) * ldv * m) : nullptr;
   double *u = (double *)W.vec(3, sizeof(double) * n);
+  double *cur = (double *)W.vec(2, sizeof(double) * n);
+  double *w = (double *)W.vec(9, sizeof(double) * n);
   double *zt = (double *)W.vec(4, sizeof(double) * n);
   PrecondScratch ps;
   GB_TRY(ps.alloc(p, n, [&](int slot, size_t bytes) { return W.vec(slot, bytes); }));
@@ -1440,7 +1455,7 @@ int gmres_solve(gb300_matrix *A, const double *val, const double *rhs,
   double *pn = (double *)W.vec(12, sizeof(double) * kReduceBlocks);
   GmState *S = (GmState *)W.state(sizeof(GmState));
   int *okflag = (int *)W.vec(7, sizeof(int));
-  if(!V || (flexible && !Z) || !u || !zt || !part || !pn || !S || !okflag)
+  if(!V || (flexible && !Z) || !u || !cur || !w || !zt || !part || !pn || !S || !okflag)
     return GB300_ERR_CUDA;
   GmState h0;
   memset(&h0, 0, sizeof(h0));
@@ -1453,64 +1468,82 @@ int gmres_solve(gb300_matrix *A, const double *val, const double *rhs,
   GB_CUDA(cudaMemsetAsync(x, 0, sizeof(double) * n, st));  // sol = 0
 
   int gs = grid_for(n, 256, kReduceBlocks * 4);
-  // row shares of the Gram-Schmidt kernels, fixed for a given n and k, so
+  // row shares of the Gram-Schmidt kernels, fixed for a given n and step, so
   // deterministic.  Dots: the groups' CTAs fill the SMs once (see k_gm_dots),
   // twice from 200,000 rows on, where the loads need more warps.  Update:
   // whole waves of 152, as many as leave a thread some 6 rows (512 CTAs on
   // 152 SMs, 4 on some and 3 on others, took 85 us at 1,046,529 rows, k = 25)
   const int rows256 = (n + 255) / 256;
-  auto dots_shares = [&](int groups) {
-    return std::max(1, std::min({rows256, 152 * (n > 200000 ? 2 : 1) / groups, kReduceBlocks}));
-  };
+  const int nbd = std::min(152 * (n > 200000 ? 2 : 1), rows256 * (m / kDotCols + 1));
   const int nbu = std::min(rows256, 152 * std::min(8, std::max(1, n / (152 * 256 * 6))));
-  cudaGraph_t graph;
-  cudaGraphExec_t exec;
-  GB_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-  // restart: V_0 = (rhs - A x) / ||rhs - A x||
-  residual64(A, val, x, rhs, V, part, st);
-  k_gm_restart<<<1, 256, 0, st>>>(S, part, m);
-  k_gm_scale<<<gs, 256, 0, st>>>(n, &S->scale, V, V, &S->cycle);
-  for(int k = 1; k <= m; k++) {
-    double *vk = V + (size_t)(k - 1) * ldv;
-    double *w = V + (size_t)k * ldv;
-    double *z = flexible ? Z + (size_t)(k - 1) * ldv : zt;
-    precond_run(A, val, p, vk, z, ps, &S->cycle, st);
-    product_chain(kChainMul, A, val, {z, nullptr, w, nullptr, nullptr, nullptr, &S->cycle}, st);
+  const double *no_z = nullptr;
+
+  // One graph holds a few Arnoldi steps (they find their place in the cycle
+  // in the state) and is replayed through the cycle, another the end of the
+  // cycle and the restart: a graph of all m steps had cost 1 to 3 ms per
+  // solve to capture and instantiate, more than 50 steps of a small system.
+  constexpr int kChunk = 5;
+  auto restart = [&]() {  // V_0 = cur = (rhs - A x) / ||rhs - A x||
+    residual64(A, val, x, rhs, V, part, st);
+    k_gm_restart<<<1, 256, 0, st>>>(S, part, m);
+    k_gm_scale<<<gs, 256, 0, st>>>(n, &S->scale, V, V, cur, &S->cycle);
+  };
+  auto step = [&]() {
+    precond_run(A, val, p, cur, zt, ps, &S->cycle, st);
+    product_chain(kChainMul, A, val, {zt, nullptr, w, nullptr, nullptr, nullptr, &S->cycle}, st);
     // classical Gram-Schmidt, a second pass only when the test after the
     // first asks for it; the reductions, the test and the end of the step
     // run in the last CTA of each kernel
-    const int g0 = k / kDotCols + 1, g1 = (k - 1) / kDotCols + 1;
-    launch_chain(false, k_gm_dots<0>, dim3(dots_shares(g0), g0), 256, st, n, k, V, ldv, w, part,
-                 S);
-    launch_chain(false, k_gm_update, nbu + 1, 256, st, n, k, m, V, ldv, w, pn, S, 0);
-    launch_chain(false, k_gm_dots<1>, dim3(dots_shares(g1), g1), 256, st, n, k, V, ldv, w, part,
-                 S);
-    launch_chain(false, k_gm_update, nbu + 1, 256, st, n, k, m, V, ldv, w, pn, S, 1);
-  }
-  k_gm_solve_small<<<1, 32, 0, st>>>(S);
-  if(flexible)
-    k_gm_combine<1><<<gs, 256, 0, st>>>(n, Z, ldv, x, S);
-  else {
-    k_gm_combine<0><<<gs, 256, 0, st>>>(n, V, ldv, u, S);
-    k_gm_apply_ok<<<1, 32, 0, st>>>(S, okflag);
-    precond_run(A, val, p, u, zt, ps, okflag, st);
-    k_gm_addto<<<gs, 256, 0, st>>>(n, zt, x, S);
-  }
-  k_gm_after<<<1, 32, 0, st>>>(S);
-  GB_CUDA(cudaStreamEndCapture(st, &graph));
-  GB_CUDA(cudaGraphInstantiate(&exec, graph, 0));
-
+    launch_chain(false, k_gm_dots<0>, nbd, 256, st, n, V, ldv, w, part, S);
+    launch_chain(false, k_gm_update, nbu + 1, 256, st, n, m, V, ldv, w, cur, zt, Z, pn, S, 0);
+    launch_chain(false, k_gm_dots<1>, nbd, 256, st, n, V, ldv, cur, part, S);
+    launch_chain(false, k_gm_update, nbu + 1, 256, st, n, m, V, ldv, cur, cur, no_z, Z, pn, S, 1);
+  };
+  auto turn = [&]() {
+    k_gm_solve_small<<<1, 32, 0, st>>>(S);
+    if(flexible)
+      k_gm_combine<1><<<gs, 256, 0, st>>>(n, Z, ldv, x, S);
+    else {
+      k_gm_combine<0><<<gs, 256, 0, st>>>(n, V, ldv, u, S);
+      k_gm_apply_ok<<<1, 32, 0, st>>>(S, okflag);
+      precond_run(A, val, p, u, zt, ps, okflag, st);
+      k_gm_addto<<<gs, 256, 0, st>>>(n, zt, x, S);
+    }
+    k_gm_after<<<1, 32, 0, st>>>(S);
+    restart();
+  };
+  struct Graph {
+    cudaGraph_t g = nullptr;
+    cudaGraphExec_t e = nullptr;
+    ~Graph()
+    {
+      if(e) cudaGraphExecDestroy(e);
+      if(g) cudaGraphDestroy(g);
+    }
+  } steps, turns;
+  auto capture = [&](Graph &G, auto body) -> int {
+    GB_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
+    body();
+    GB_CUDA(cudaStreamEndCapture(st, &G.g));
+    GB_CUDA(cudaGraphInstantiate(&G.e, G.g, 0));
+    return GB300_OK;
+  };
+  restart();
+  GB_TRY(capture(steps, [&]() {
+    for(int q = 0; q < std::min(m, kChunk); q++) step();
+  }));
+  GB_TRY(capture(turns, turn));
+  const int replays = (m + kChunk - 1) / kChunk;
   int active = 1, launches = 0;
   int max_launches = p->nb_iter_max > 0 ? p->nb_iter_max + 2 : 1 << 30;
   while(active && launches < max_launches) {
-    GB_CUDA(cudaGraphLaunch(exec, st));
+    for(int q = 0; q < replays; q++) GB_CUDA(cudaGraphLaunch(steps.e, st));
+    GB_CUDA(cudaGraphLaunch(turns.e, st));
     launches++;
     GB_CUDA(cudaMemcpyAsync(&active, &S->active, sizeof(int),
                             cudaMemcpyDeviceToHost, st));
     GB_CUDA(cudaStreamSynchronize(st));
   }
-  cudaGraphExecDestroy(exec);
-  cudaGraphDestroy(graph);
   GB_CUDA(cudaMemcpyAsync(&h0, S, sizeof(GmState), cudaMemcpyDeviceToHost, st));
   GB_CUDA(cudaStreamSynchronize(st));
   info->status = active ? -1 : h0.status;
