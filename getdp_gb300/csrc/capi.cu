@@ -20,6 +20,23 @@ void set_error(const char *fmt, ...)
   g_error = buf;
 }
 
+thread_local gb300_ctx *t_pool_ctx = nullptr;
+
+cudaError_t pool_alloc(void **p, size_t bytes, cudaStream_t *stream)
+{
+  gb300_ctx *c = t_pool_ctx;
+  if(!c->pool) return cudaMalloc(p, bytes);
+  cudaError_t e = cudaMallocFromPoolAsync(p, bytes, c->pool, c->stream);
+  if(e == cudaErrorMemoryAllocation) {  // what the pool holds in other sizes
+    cudaGetLastError();
+    cudaStreamSynchronize(c->stream);
+    cudaMemPoolTrimTo(c->pool, 0);
+    e = cudaMallocFromPoolAsync(p, bytes, c->pool, c->stream);
+  }
+  if(e == cudaSuccess) *stream = c->stream;
+  return e;
+}
+
 template <typename T> static int check(T *p, const char *what)
 {
   if(!p) {
@@ -85,6 +102,17 @@ int gb300_ctx_create(int device, gb300_ctx **out)
     set_error("cudaStreamCreate failed: %s", cudaGetErrorString(e));
     return GB300_ERR_CUDA;
   }
+  cudaMemPoolProps props = {};
+  props.allocType = cudaMemAllocationTypePinned;
+  props.location.type = cudaMemLocationTypeDevice;
+  props.location.id = device;
+  unsigned long long keep = gb::kPoolKeep;
+  if(cudaMemPoolCreate(&c->pool, &props) != cudaSuccess ||
+     cudaMemPoolSetAttribute(c->pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+    cudaGetLastError();  // no pool: cudaMalloc instead
+    if(c->pool) cudaMemPoolDestroy(c->pool);
+    c->pool = nullptr;
+  }
   *out = c;
   return GB300_OK;
 }
@@ -95,6 +123,8 @@ int gb300_ctx_destroy(gb300_ctx *ctx)
   cudaStreamSynchronize(ctx->stream);
   gb::gen_cache_free(ctx->gen);
   ctx->gen = nullptr;
+  cudaStreamSynchronize(ctx->stream);  // (the frees above are in its order)
+  if(ctx->pool) cudaMemPoolDestroy(ctx->pool);
   cudaStreamDestroy(ctx->stream);
   delete ctx;
   return GB300_OK;
@@ -124,7 +154,14 @@ int gb300_device_alloc(gb300_ctx *ctx, size_t bytes, void **out)
 {
   GB_TRY(check(ctx, "ctx"));
   GB_TRY(check(out, "out"));
-  GB_CUDA(cudaMalloc(out, bytes ? bytes : 1));
+  cudaError_t e = cudaMalloc(out, bytes ? bytes : 1);
+  if(e == cudaErrorMemoryAllocation && ctx->pool) {
+    cudaGetLastError();
+    cudaStreamSynchronize(ctx->stream);
+    cudaMemPoolTrimTo(ctx->pool, 0);
+    e = cudaMalloc(out, bytes ? bytes : 1);
+  }
+  GB_CUDA(e);
   return GB300_OK;
 }
 
@@ -365,6 +402,7 @@ int gb300_vector_norm2(const gb300_vector *v, double *norm)
 {
   GB_TRY(check(v, "vector"));
   GB_TRY(check(norm, "norm"));
+  gb::PoolScope pool_scope(v->ctx);
   Work W;
   return norm2_dev(v->n, v->d.p, norm, W, v->ctx->stream);
 }
@@ -395,6 +433,7 @@ int gb300_vector_add_values(gb300_vector *v, int count, const int *idx,
                             const double *val)
 {
   GB_TRY(check(v, "vector"));
+  gb::PoolScope pool_scope(v->ctx);
   if(count <= 0) return GB300_OK;
   GB_TRY(check(idx, "idx"));
   GB_TRY(check(val, "val"));
@@ -509,6 +548,7 @@ int gb300_matrix_assemble(gb300_matrix *A)
 {
   gb::NvtxRange nvtx_range("gb300_matrix_assemble");
   GB_TRY(check(A, "matrix"));
+  gb::PoolScope pool_scope(A->ctx);
   if(A->hr.empty() && A->csr_valid) return GB300_OK;
   cudaStream_t st = A->ctx->stream;
   long long m = (long long)A->hr.size();
@@ -557,6 +597,7 @@ int gb300_matrix_assemble(gb300_matrix *A)
 int gb300_matrix_zero(gb300_matrix *A)
 {
   GB_TRY(check(A, "matrix"));
+  gb::PoolScope pool_scope(A->ctx);
   GB_TRY(gb300_matrix_assemble(A));
   cudaStream_t st = A->ctx->stream;
   if(A->nnz > 0) GB_CUDA(cudaMemsetAsync(A->val.p, 0, sizeof(double) * A->nnz, st));
@@ -682,6 +723,7 @@ int gb300_generate_pattern(gb300_matrix *A, const gb300_term_batch *t)
   gb::NvtxRange nvtx_range("gb300_generate_pattern");
   GB_TRY(check(A, "matrix"));
   GB_TRY(check(t, "term batch"));
+  gb::PoolScope pool_scope(A->ctx);
   // a Generate makes a new matrix (GetDP's ZeroMatrix): no factor survives it
   if(A->ilu) {
     ilu_free(A->ilu);
@@ -698,6 +740,7 @@ int gb300_generate_values(gb300_matrix *A, gb300_vector *b,
   GB_TRY(check(A, "matrix"));
   GB_TRY(check(b, "rhs"));
   GB_TRY(check(t, "term batch"));
+  gb::PoolScope pool_scope(A->ctx);
   return generate_values(A, b, t, nullptr);
 }
 
@@ -709,6 +752,7 @@ int gb300_generate_values_at(gb300_matrix *A, gb300_vector *b,
   GB_TRY(check(b, "rhs"));
   GB_TRY(check(t, "term batch"));
   GB_TRY(check(x, "solution"));
+  gb::PoolScope pool_scope(A->ctx);
   return generate_values(A, b, t, x);
 }
 
@@ -867,6 +911,7 @@ int gb300_solve(gb300_matrix *A, const gb300_vector *b,
   GB_TRY(check(b, "rhs"));
   GB_TRY(check(p, "params"));
   GB_TRY(check(x, "solution"));
+  gb::PoolScope pool_scope(A->ctx);
   GB_TRY(gb300_matrix_assemble(A));
   return solve(A, b, p, x, info);
 }
@@ -911,6 +956,7 @@ int gb300_matrix_coarse_energy(gb300_matrix *A, const gb300_vector *u, double *u
   GB_TRY(check(A, "matrix"));
   GB_TRY(check(u, "vector"));
   GB_TRY(check(ucu, "result"));
+  gb::PoolScope pool_scope(A->ctx);
   GB_TRY(gb300_matrix_assemble(A));
   if(u->n != A->n) {
     set_error("coarse energy: vector size %d, matrix size %d", u->n, A->n);
@@ -954,6 +1000,7 @@ int gb300_precond_apply(gb300_matrix *A, const gb300_solver_params *p,
   GB_TRY(check(p, "params"));
   GB_TRY(check(v, "v"));
   GB_TRY(check(z, "z"));
+  gb::PoolScope pool_scope(A->ctx);
   GB_TRY(gb300_matrix_assemble(A));
   if(v->n != A->n || z->n != A->n || v == z) {
     set_error("preconditioner apply: sizes or aliasing");
@@ -969,6 +1016,7 @@ int gb300_post_elements(const gb300_term_batch *t, const gb300_vector *x,
   GB_TRY(check(t, "term batch"));
   GB_TRY(check(x, "solution"));
   GB_TRY(check(out, "out"));
+  gb::PoolScope pool_scope(x->ctx);
   return post_elements(t, x, out);
 }
 
@@ -979,6 +1027,7 @@ int gb300_post_points(const gb300_term_batch *t, const gb300_vector *x, int npts
   GB_TRY(check(t, "term batch"));
   GB_TRY(check(x, "solution"));
   if(npts > 0) GB_TRY(check(xyz, "xyz"));
+  gb::PoolScope pool_scope(x->ctx);
   return post_points(t, x, npts, xyz, field, curl, elem);
 }
 
@@ -1017,6 +1066,7 @@ int gb300_solve_batch(gb300_matrix *A, const gb300_vector *b,
   GB_TRY(check(x, "solution"));
   GB_TRY(check(offsets, "offsets"));
   GB_TRY(check(infos, "infos"));
+  gb::PoolScope pool_scope(A->ctx);
   GB_TRY(gb300_matrix_assemble(A));
   return solve_batch(A, b, p, x, nsys, offsets, infos);
 }

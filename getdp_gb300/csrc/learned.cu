@@ -761,6 +761,7 @@ int gb300_mpnn_infer(gb300_mpnn *net, gb300_matrix *A)
     set_error("network: null argument");
     return GB300_ERR_ARG;
   }
+  gb::PoolScope pool_scope(A->ctx);
   GB_TRY(gb300_matrix_assemble(A));
   GB_TRY(mp_prepare(net, A));
   GB_TRY(mp_forward(net, A));
@@ -781,6 +782,7 @@ int gb300_mpnn_loss_grad(gb300_mpnn *net, gb300_matrix *A, const gb300_vector *r
     set_error("network: null argument");
     return GB300_ERR_ARG;
   }
+  gb::PoolScope pool_scope(A->ctx);
   GB_TRY(gb300_matrix_assemble(A));
   if(r1->n != A->n || (e1 && e1->n != A->n)) {
     set_error("network: vector sizes do not match the matrix");
