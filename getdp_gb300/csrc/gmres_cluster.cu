@@ -44,17 +44,14 @@ namespace cg = cooperative_groups;
 namespace gb {
 
 // CTAs per cluster (one cluster per system): Batch_Kernel 1, 2, 4, 8 (the
-// portable maximum) or 16 (a non-portable size this GPU allows).  Measured
-// on 512 complex systems of 1,922..51,842 rows (ILU(0)-GMRES(40) in the
-// multicolour order, FP64 / FP32 factor): 1 CTA 2.32 / 2.07 s, 2 1.29 /
-// 1.14, 4 0.958 / 0.856, 8 1.11 / 0.99, against 1.19 / 1.235 s for the
-// per-kernel form: few CTAs leave the largest systems' steps to one or two
-// SMs, many CTAs leave fewer systems running at once and make each cluster
-// barrier dearer.  256-thread CTAs measured the same at the same threads
-// per system (8 CTAs: 0.938 / 0.843 s) and slower at fewer (4 CTAs: 1.22 /
-// 1.10 s)
-constexpr int kCThreads = 512;
-constexpr int kCWarps = kCThreads / 32;
+// portable maximum) or 16 (a non-portable size this GPU allows); 512 threads
+// each, two CTAs to an SM.  On 512 complex systems of 1,922..51,842 rows
+// (ILU(0)-GMRES(40) in the multicolour order) four were the fastest: few CTAs
+// leave the largest systems' steps to one or two SMs, many CTAs leave fewer
+// systems running at once and make each cluster barrier dearer.  Fewer
+// systems want larger clusters (see where the default is chosen).  1024
+// threads in one CTA per SM leave half as many clusters: 322 against 240 ms
+// on 64 systems.
 constexpr int kCMaxKrylov = 64;
 // most levels of one system in either triangular sweep (one cluster
 // barrier each); systems in GetDP's own order (~2n levels on an n x n grid)
@@ -91,16 +88,17 @@ struct CArgs {
 
 // the sums over the cluster's CTAs, in rank order, of the nv partials each
 // CTA left in buf: every CTA gets the same values in out
-template <int CS>
+template <int CS, int NT>
 __device__ __forceinline__ void cluster_sum(cg::cluster_group &cl, double *buf, int nv,
                                             double *out)
 {
   cl.sync();
-  for(int j = threadIdx.x; j < nv; j += kCThreads) {
-    double s = 0.;
+  for(int j = threadIdx.x; j < nv; j += NT) {
+    // four chains over the ranks (an FP64 addition takes some 85 ns)
+    double s[4] = {0., 0., 0., 0.};
 #pragma unroll
-    for(int r = 0; r < CS; r++) s += cl.map_shared_rank(buf, r)[j];
-    out[j] = s;
+    for(int r = 0; r < CS; r++) s[r & 3] += cl.map_shared_rank(buf, r)[j];
+    out[j] = (s[0] + s[1]) + (s[2] + s[3]);
   }
   __syncthreads();
 }
@@ -138,161 +136,388 @@ __device__ __forceinline__ T row_acc(int k0, int k1, const int *__restrict__ col
   return s;
 }
 
-// the sum over the cluster's CTAs and their warps, in (rank, warp) order, of
-// the one partial per warp each CTA left in buf[0 .. kCWarps): every CTA
-// gets the same value in out[0] (no CTA-wide sum first)
-template <int CS>
+// the sum over the cluster's CTAs and their warps of the one partial per warp
+// each CTA left in buf[0 .. NT / 32), in a fixed order (a tree over a CTA's
+// warps, then one over the ranks: summing rank after rank cost 7 us on 16
+// CTAs): every CTA gets the same value in out[0]
+template <int CS, int NT>
 __device__ __forceinline__ void cluster_sum_warps(cg::cluster_group &cl, double *buf,
                                                   double *out)
 {
+  __syncthreads();
+  if(threadIdx.x < 32) {
+    const double v = warp_sum(threadIdx.x < NT / 32 ? buf[threadIdx.x] : 0.);
+    if(threadIdx.x == 0) buf[0] = v;
+  }
   cl.sync();
   if(threadIdx.x < 32) {
-    double s = 0.;
-    for(int r = 0; r < CS; r++) {
-      double v = threadIdx.x < kCWarps ? cl.map_shared_rank(buf, r)[threadIdx.x] : 0.;
-      s += warp_sum(v);  // lane 0 holds the rank's sum
-    }
-    if(threadIdx.x == 0) out[0] = s;
+    const double v = warp_sum(threadIdx.x < CS ? *cl.map_shared_rank(buf, threadIdx.x) : 0.);
+    if(threadIdx.x == 0) out[0] = v;
   }
   __syncthreads();
 }
 
-// w = A z on the rows [lo, hi) (two lanes per row, as k_b_spmv); with RES,
-// w = rhs - A z and the partial ||w||^2 (and ||rhs||^2 in bb)
-template <int RES>
-__device__ __forceinline__ double c_spmv(const CArgs &P, int lo, int hi, const double *z,
+// The three passes below run over some 2,000 rows per CTA from L2, so what
+// paces them is how many loads a thread has in flight: each keeps 16 or more
+// (with four, 64 systems of up to 50,562 rows took 243 ms instead of 230).
+
+// w = A z on the rows [lo, hi), one thread per row, the next row's bounds
+// loaded ahead; with RES, w = rhs - A z and the partial ||w||^2 (and
+// ||rhs||^2 in bb)
+template <int RES, int NT>
+__device__ __noinline__ double c_spmv(const CArgs &P, int lo, int hi, const double *z,
                                          double *w, double *bb)
 {
-  const int l2 = threadIdx.x & 1, sub = threadIdx.x >> 1;
+  constexpr int U = 8;
   double acc = 0., accb = 0.;
-  for(int i = lo + sub; i - sub < hi; i += kCThreads / 2) {
-    double s = 0.;
-    if(i < hi) s = row_acc<2, false>(P.rowptr[i] + l2, P.rowptr[i + 1], P.col, P.val, z, s);
-    s += __shfl_down_sync(0xffffffffu, s, 1, 2);
-    if(l2 == 0 && i < hi) {
-      if(RES) {
-        double ri = P.rhs[i] - s;
-        if(w) w[i] = ri;
-        acc += ri * ri;
-        accb += P.rhs[i] * P.rhs[i];
-      }
-      else
-        w[i] = s;
+  int i = lo + threadIdx.x, k = 0, e = 0;
+  if(i < hi) {
+    k = P.rowptr[i];
+    e = P.rowptr[i + 1];
+  }
+  while(i < hi) {
+    const int in = i + NT;
+    int kn = 0, en = 0;
+    if(in < hi) {
+      kn = P.rowptr[in];
+      en = P.rowptr[in + 1];
     }
+    double s = 0.;
+    for(; k < e; k += U) {
+      int c[U];
+      double v[U], zv[U];
+#pragma unroll
+      for(int u = 0; u < U; u++) {
+        c[u] = k + u < e ? P.col[k + u] : -1;
+        v[u] = k + u < e ? P.val[k + u] : 0.;
+      }
+#pragma unroll
+      for(int u = 0; u < U; u++) zv[u] = c[u] >= 0 ? __ldcg(z + c[u]) : 0.;
+#pragma unroll
+      for(int u = 0; u < U; u++)
+        if(c[u] >= 0) s += v[u] * zv[u];
+    }
+    if(RES) {
+      const double bi = P.rhs[i], ri = bi - s;
+      if(w) w[i] = ri;
+      acc += ri * ri;
+      accb += bi * bi;
+    }
+    else
+      w[i] = s;
+    i = in;
+    k = kn;
+    e = en;
   }
   if(bb) *bb = accb;
   return acc;
 }
 
-// partial <V_j, w> over the rows [lo, hi) for j < kk, one warp per column
-// (a fixed order per column), into buf[j]
-__device__ __forceinline__ void c_dots(const CArgs &P, int lo, int hi, const double *w,
+// partial <V_j, w> over the rows [lo, hi) for j < kk, two columns per warp at
+// a time (a fixed order per column), into buf[j]
+template <int NT>
+__device__ __noinline__ void c_dots(const CArgs &P, int lo, int hi, const double *w,
                                        int kk, double *buf)
 {
+  constexpr int U = 8, NW = NT / 32;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for(int j = warp; j < kk; j += kCWarps) {
-    const double *vj = P.Vb + (size_t)j * P.ldv;
-    double s = 0.;
+  for(int j = warp; j < kk; j += 2 * NW) {
+    const bool two = j + NW < kk;  // the same in the whole warp
+    const double *va = P.Vb + (size_t)j * P.ldv;
+    const double *vb = P.Vb + (size_t)(two ? j + NW : j) * P.ldv;
+    double sa = 0., sb = 0.;
+    for(int i = lo + lane; i < hi; i += 32 * U) {
+      double a[U], b[U], x[U];
+#pragma unroll
+      for(int u = 0; u < U; u++) {
+        const int r = i + 32 * u;
+        x[u] = r < hi ? __ldcg(w + r) : 0.;
+        a[u] = r < hi ? __ldcg(va + r) : 0.;
+        b[u] = two && r < hi ? __ldcg(vb + r) : 0.;
+      }
+#pragma unroll
+      for(int u = 0; u < U; u++) sa += a[u] * x[u];
+      if(two)
+#pragma unroll
+        for(int u = 0; u < U; u++) sb += b[u] * x[u];
+    }
+    sa = warp_sum(sa);
+    if(lane == 0) buf[j] = sa;
+    if(two) {
+      sb = warp_sum(sb);
+      if(lane == 0) buf[j + NW] = sb;
+    }
+  }
+}
+
+// The previous rotations on column k (h, into Hc): they need the column only,
+// so warp 0 runs them ahead of its share of the update, everything but their
+// chain (one FMA each, some 85 ns) in parallel; k <= 64
+__device__ __noinline__ void c_rotate(const double *h, const double *cs, const double *sn,
+                                         int k, double *ra, double *Hc)
+{
+  const int lane = threadIdx.x;  // warp 0
+  double t[2], q[2];
+#pragma unroll
+  for(int u = 0; u < 2; u++) {
+    const int j = lane + 32 * u;
+    const double b = j < k - 1 ? h[j + 1] : 0.;
+    t[u] = j < k - 1 ? cs[j] * b : 0.;
+    q[u] = j < k - 1 ? sn[j] * b : 0.;
+    if(j < k - 1) ra[j] = t[u];
+  }
+  __syncwarp();
+  if(lane == 0) {
+    double a = h[0];
 #pragma unroll 4
-    for(int i = lo + lane; i < hi; i += 32) s += __ldcg(vj + i) * __ldcg(w + i);
-    s = warp_sum(s);
-    if(lane == 0) buf[j] = s;
+    for(int i = 0; i < k - 1; i++) {
+      const double ti = ra[i];
+      ra[i] = a;
+      a = fma(-sn[i], a, ti);
+    }
+    ra[k - 1] = a;
+  }
+  __syncwarp();
+#pragma unroll
+  for(int u = 0; u < 2; u++) {
+    const int j = lane + 32 * u;
+    if(j < k) Hc[j] = j < k - 1 ? fma(cs[j], ra[j], q[u]) : ra[j];
   }
 }
 
 // w -= sum_{j<k} h_j V_j on the rows [lo, hi); the partial ||w||^2
-__device__ __forceinline__ double c_update(const CArgs &P, int lo, int hi, double *w,
+template <int NT>
+__device__ __noinline__ double c_update(const CArgs &P, int lo, int hi, double *w,
                                            const double *h, int k)
 {
+  // two rows at a time, one FMA chain each, k + 1 FP64 instructions per row
+  // (they pace the kernel once the loads do not)
+  constexpr int U = 8;
   double v = 0.;
-  for(int i = lo + threadIdx.x; i < hi; i += kCThreads) {
-    // four independent FMA chains (as k_b_update)
-    double s0 = 0., s1 = 0., s2 = 0., s3 = 0.;
-    int j = 0;
-    for(; j + 3 < k; j += 4) {
-      s0 += h[j] * __ldcg(P.Vb + (size_t)j * P.ldv + i);
-      s1 += h[j + 1] * __ldcg(P.Vb + (size_t)(j + 1) * P.ldv + i);
-      s2 += h[j + 2] * __ldcg(P.Vb + (size_t)(j + 2) * P.ldv + i);
-      s3 += h[j + 3] * __ldcg(P.Vb + (size_t)(j + 3) * P.ldv + i);
+  for(int i = lo + threadIdx.x; i < hi; i += 2 * NT) {
+    const bool two = i + NT < hi;
+    const double *va = P.Vb + i, *vb = va + (two ? NT : 0);
+    double s0 = __ldcg(w + i), s1 = two ? __ldcg(w + i + NT) : 0.;
+    for(int j = 0; j < k; j += U) {
+      double a[U], b[U];
+#pragma unroll
+      for(int u = 0; u < U; u++) {
+        a[u] = j + u < k ? __ldcg(va + (size_t)(j + u) * P.ldv) : 0.;
+        b[u] = two && j + u < k ? __ldcg(vb + (size_t)(j + u) * P.ldv) : 0.;
+      }
+#pragma unroll
+      for(int u = 0; u < U; u++)
+        if(j + u < k) {
+          s0 = fma(-h[j + u], a[u], s0);
+          if(two) s1 = fma(-h[j + u], b[u], s1);
+        }
     }
-    for(; j < k; j++) s0 += h[j] * __ldcg(P.Vb + (size_t)j * P.ldv + i);
-    double wi = __ldcg(w + i) - ((s0 + s1) + (s2 + s3));
-    w[i] = wi;
-    v += wi * wi;
+    w[i] = s0;
+    v = fma(s0, s0, v);
+    if(two) {
+      w[i + NT] = s1;
+      v = fma(s1, s1, v);
+    }
   }
   return v;
+}
+
+// One row's strictly lower or upper entries: the first kAhead columns and
+// values in registers, loaded before a cluster barrier so that only the
+// gathers of x follow it, the rest read when they are needed
+constexpr int kAhead = 4;
+template <typename T> struct RowAhead {
+  int k0, k1, c[kAhead];
+  T v[kAhead];
+  __device__ __forceinline__ void load(int a, int b, const int *__restrict__ col,
+                                       const T *__restrict__ lu)
+  {
+    k0 = a;
+    k1 = b;
+#pragma unroll
+    for(int u = 0; u < kAhead; u++) {
+      c[u] = a + u < b ? col[a + u] : -1;
+      v[u] = a + u < b ? lu[a + u] : (T)0;
+    }
+  }
+  template <typename X> __device__ __forceinline__ void gather(const X *x, X (&xv)[kAhead]) const
+  {
+#pragma unroll
+    for(int u = 0; u < kAhead; u++) xv[u] = c[u] >= 0 ? __ldcg(x + c[u]) : (X)0;
+  }
+  // s - sum over the entries, in their order
+  template <typename X>
+  __device__ __forceinline__ T apply(const int *__restrict__ col, const T *__restrict__ lu,
+                                     const X *x, const X (&xv)[kAhead], T s) const
+  {
+#pragma unroll
+    for(int u = 0; u < kAhead; u++)
+      if(c[u] >= 0) s = s - v[u] * xv[u];
+    return k0 + kAhead < k1 ? row_acc<1, true>(k0 + kAhead, k1, col, lu, x, s) : s;
+  }
+};
+
+// dst = M^-1 src colour by colour (the multicolour order): a colour's vertices
+// share no entry, so its rows are independent but for the two real rows of a
+// complex unknown (bs = 2), which sit in adjacent lanes and exchange their
+// values by shuffles, the coupling entry l (row 2v + 1 on 2v) forward and u
+// (2v on 2v + 1) backward.  The last colour's rows have no other upper
+// entries, so both sweeps finish them at once: one barrier per colour and
+// sweep but one.  A thread's first row of the next colour is loaded between
+// the barrier's arrive and its wait: a colour costs a gather, a short FMA
+// chain and the barrier (with the row's structure read after the barrier and
+// a vertex's rows one after the other, 5 us a colour on 16 CTAs).
+// src must be complete but for a cluster barrier; dst is complete on return.
+template <typename T, int CS, int NT>
+__device__ __noinline__ void c_colour_sweeps(const CArgs &P, cg::cluster_group &cl, int p, int rank,
+                                const double *src, double *dst)
+{
+  const T *__restrict__ lu = (const T *)P.lu, *__restrict__ inv = (const T *)P.inv;
+  const int *__restrict__ col = P.col;
+  T *x = sizeof(T) == 8 ? (T *)dst : (T *)P.t32;
+  const int *vo = P.voff + (size_t)p * (P.ncol + 1);
+  const int bs = P.bs, C = P.ncol;
+  const bool odd = bs == 2 && (threadIdx.x & 1), even = bs == 2 && !(threadIdx.x & 1);
+  RowAhead<T> R;
+  T cpl = (T)0, iv = (T)0;  // coupling entry with the partner row, pivot inverse
+  int m0 = 0, m1 = 0;       // the entries' bounds, one colour further ahead
+  auto bounds = [&](int c, int &r0, int &r1) {
+    const int a = vo[c], cnt = vo[c + 1] - a;
+    r0 = (a + (int)((long long)cnt * rank / CS)) * bs;
+    r1 = (a + (int)((long long)cnt * (rank + 1) / CS)) * bs;
+  };
+  // bounds of row i's strictly lower or upper entries
+  auto meta = [&](bool up, int i, bool in) {
+    m0 = !in ? 0 : up ? P.diag[i] + 1 : P.rowptr[i];
+    m1 = !in ? 0 : up ? P.rowptr[i + 1] : P.diag[i];
+  };
+  auto meta_first = [&](bool up, int c) {
+    int r0, r1;
+    bounds(c, r0, r1);
+    meta(up, r0 + threadIdx.x, r0 + (int)threadIdx.x < r1);
+  };
+  // the entries within the bounds, the partner's taken out: the last of row
+  // 2v + 1's lower ones, the first of row 2v's upper ones
+  auto load = [&](bool up, int i, bool in) {
+    cpl = (T)0;
+    iv = up && in ? inv[i] : (T)0;
+    if(up && even && m0 < m1 && col[m0] == i + 1) cpl = lu[m0++];
+    if(!up && odd && m0 < m1 && col[m1 - 1] == i - 1) cpl = lu[--m1];
+    R.load(m0, m1, col, lu);
+  };
+  auto put = [&](int i, T v, bool last) {
+    x[i] = v;
+    if(sizeof(T) == 4 && last) dst[i] = (double)v;
+  };
+  // v: this row's backward value before its partner's part and the pivot
+  auto pivot = [&](T v, T u, T ivv) {
+    const T w = ivv * v;
+    const T wo = __shfl_down_sync(0xffffffffu, w, 1);
+    return even ? ivv * (v - u * wo) : w;
+  };
+  cl.barrier_arrive();
+  meta_first(false, 0);
+  for(int c = 0; c < C; c++) {
+    int r0, r1;
+    bounds(c, r0, r1);
+    int i = r0 + threadIdx.x;
+    load(false, i, i < r1);
+    if(c < C - 1)
+      meta_first(false, c + 1);
+    else if(C > 1)
+      meta_first(true, C - 2);
+    const int n0 = m0, n1 = m1;  // the next colour's
+    cl.barrier_wait();
+    for(int base = r0; base < r1; base += NT) {  // the same in every thread
+      i = base + threadIdx.x;
+      const bool in = i < r1;
+      if(base > r0) {
+        meta(false, i, in);
+        load(false, i, in);
+      }
+      T s = in ? (T)__ldcg(src + i) : (T)0;
+      T xv[kAhead];
+      R.gather((const T *)x, xv);
+      s = R.apply(col, lu, (const T *)x, xv, s);
+      const T se = __shfl_up_sync(0xffffffffu, s, 1);
+      if(odd) s = s - cpl * se;
+      if(c == C - 1) {
+        T u = (T)0, ivv = in ? inv[i] : (T)0;
+        if(even && in) {
+          const int k = P.diag[i] + 1;
+          if(k < P.rowptr[i + 1] && col[k] == i + 1) u = lu[k];
+        }
+        s = pivot(s, u, ivv);
+      }
+      if(in) put(i, s, c == C - 1);
+    }
+    cl.barrier_arrive();
+    m0 = n0;
+    m1 = n1;
+  }
+  for(int c = C - 2; c >= 0; c--) {
+    int r0, r1;
+    bounds(c, r0, r1);
+    int i = r0 + threadIdx.x;
+    load(true, i, i < r1);
+    if(c > 0) meta_first(true, c - 1);
+    const int n0 = m0, n1 = m1;
+    cl.barrier_wait();
+    for(int base = r0; base < r1; base += NT) {
+      i = base + threadIdx.x;
+      const bool in = i < r1;
+      if(base > r0) {
+        meta(true, i, in);
+        load(true, i, in);
+      }
+      T s = in ? __ldcg(x + i) : (T)0;
+      T xv[kAhead];
+      R.gather((const T *)x, xv);
+      if(sizeof(T) == 8) {
+        s = R.apply(col, lu, (const T *)x, xv, s);
+        s = pivot(s, cpl, iv);
+      }
+      else {
+        // FP32 sums in lusol's order, in which the partner comes first (the
+        // FP64 ones put it last: no second FMA chain after the partner's)
+        T w = (T)0;
+        if(!even) w = iv * R.apply(col, lu, (const T *)x, xv, s);
+        const T wo = __shfl_down_sync(0xffffffffu, w, 1);
+        s = even ? iv * R.apply(col, lu, (const T *)x, xv, s - cpl * wo) : w;
+      }
+      if(in) put(i, s, true);
+    }
+    cl.barrier_arrive();
+    m0 = n0;
+    m1 = n1;
+  }
+  cl.barrier_wait();
 }
 
 // dst = M^-1 src for system p: the ILU(0) sweeps level by level, each
 // level's rows split over the cluster (a barrier after each level), or a
 // copy without a preconditioner.  src must be complete (all CTAs) on entry;
 // dst is complete on return.
-template <typename T, int CS>
-__device__ void c_precond(const CArgs &P, cg::cluster_group &cl, int p, int rank, int lo,
+template <typename T, int CS, int NT>
+__device__ __noinline__ void c_precond(const CArgs &P, cg::cluster_group &cl, int p, int rank, int lo,
                           int hi, const double *src, double *dst)
 {
   if(!P.precond) {
-    for(int i = lo + threadIdx.x; i < hi; i += kCThreads) dst[i] = __ldcg(src + i);
+    for(int i = lo + threadIdx.x; i < hi; i += NT) dst[i] = __ldcg(src + i);
     cl.sync();
     return;
   }
   const T *lu = (const T *)P.lu, *inv = (const T *)P.inv;
-  cl.sync();  // src written by every CTA
   if(P.ncol > 0) {
-    // colour by colour: a colour's vertices share no entry, so they are
-    // independent; a vertex's bs rows (a complex unknown's two real rows)
-    // go in order in one thread, forward first to last, backward last to
-    // first: one barrier per colour instead of one per level
-    const int *vo = P.voff + (size_t)p * (P.ncol + 1);
-    const int bs = P.bs;
-    for(int c = 0; c < P.ncol; c++) {
-      const int a = vo[c], cnt = vo[c + 1] - a;
-      if(cnt == 0) continue;  // the same for every CTA
-      const int t0 = a + (int)((long long)cnt * rank / CS);
-      const int t1 = a + (int)((long long)cnt * (rank + 1) / CS);
-      for(int v = t0 + threadIdx.x; v < t1; v += kCThreads)
-        for(int q = 0; q < bs; q++) {
-          const int i = v * bs + q;
-          if constexpr(sizeof(T) == 8)
-            dst[i] = row_acc<1, true>(P.rowptr[i], P.diag[i], P.col, lu,
-                                      (const double *)dst, __ldcg(src + i));
-          else
-            P.t32[i] = row_acc<1, true>(P.rowptr[i], P.diag[i], P.col, lu,
-                                        (const float *)P.t32, (float)__ldcg(src + i));
-        }
-      cl.sync();
-    }
-    for(int c = P.ncol - 1; c >= 0; c--) {
-      const int a = vo[c], cnt = vo[c + 1] - a;
-      if(cnt == 0) continue;
-      const int t0 = a + (int)((long long)cnt * rank / CS);
-      const int t1 = a + (int)((long long)cnt * (rank + 1) / CS);
-      for(int v = t0 + threadIdx.x; v < t1; v += kCThreads)
-        for(int q = bs - 1; q >= 0; q--) {
-          const int i = v * bs + q;
-          const int ke = P.rowptr[i + 1];
-          if constexpr(sizeof(T) == 8) {
-            double s = row_acc<1, true>(P.diag[i] + 1, ke, P.col, lu, (const double *)dst,
-                                        __ldcg(dst + i));
-            dst[i] = inv[i] * s;
-          }
-          else {
-            float s = row_acc<1, true>(P.diag[i] + 1, ke, P.col, lu, (const float *)P.t32,
-                                       __ldcg(P.t32 + i));
-            float w = inv[i] * s;
-            P.t32[i] = w;
-            dst[i] = (double)w;
-          }
-        }
-      cl.sync();
-    }
+    c_colour_sweeps<T, CS, NT>(P, cl, p, rank, src, dst);
     return;
   }
+  cl.sync();  // src written by every CTA
   for(int l = P.llb[p]; l + 1 < P.llb[p + 1]; l++) {
     const int a = P.llev[l], cnt = P.llev[l + 1] - a;
     const int t0 = a + (int)((long long)cnt * rank / CS);
     const int t1 = a + (int)((long long)cnt * (rank + 1) / CS);
-    for(int t = t0 + threadIdx.x; t < t1; t += kCThreads) {
+    for(int t = t0 + threadIdx.x; t < t1; t += NT) {
       const int i = P.lrows[t];
       const int ke = P.diag[i];
       if constexpr(sizeof(T) == 8)
@@ -308,7 +533,7 @@ __device__ void c_precond(const CArgs &P, cg::cluster_group &cl, int p, int rank
     const int a = P.ulev[l], cnt = P.ulev[l + 1] - a;
     const int t0 = a + (int)((long long)cnt * rank / CS);
     const int t1 = a + (int)((long long)cnt * (rank + 1) / CS);
-    for(int t = t0 + threadIdx.x; t < t1; t += kCThreads) {
+    for(int t = t0 + threadIdx.x; t < t1; t += NT) {
       const int i = P.urows[t];
       const int ke = P.rowptr[i + 1];
       if constexpr(sizeof(T) == 8) {
@@ -328,8 +553,8 @@ __device__ void c_precond(const CArgs &P, cg::cluster_group &cl, int p, int rank
   }
 }
 
-template <typename T, int CS>
-__global__ void __launch_bounds__(kCThreads, 1024 / kCThreads) k_c_solve(CArgs P)
+template <typename T, int CS, int NT>
+__global__ void __launch_bounds__(NT, 1024 / NT) k_c_solve(CArgs P)
 {
   cg::cluster_group cl = cg::this_cluster();
   const int rank = (int)cl.block_rank();
@@ -338,6 +563,7 @@ __global__ void __launch_bounds__(kCThreads, 1024 / kCThreads) k_c_solve(CArgs P
   __shared__ double sH[(kCMaxKrylov + 1) * kCMaxKrylov];  // column-major, ld m + 1
   __shared__ double scs[kCMaxKrylov], ssn[kCMaxKrylov], sy[kCMaxKrylov];
   __shared__ double sg[kCMaxKrylov + 1], sh1[kCMaxKrylov + 1], sdot[kCMaxKrylov + 1];
+  __shared__ double sra[kCMaxKrylov];
   __shared__ double xbuf[2][kCMaxKrylov + 2];  // partials read by the other CTAs
   __shared__ CState S;
   __shared__ int s_q;
@@ -365,9 +591,9 @@ __global__ void __launch_bounds__(kCThreads, 1024 / kCThreads) k_c_solve(CArgs P
       // restart: r = b - A x into V_0, ||r||
       cl.sync();  // x complete
       {
-        double rr = warp_sum(c_spmv<1>(P, lo, hi, P.x, P.Vb, nullptr));
+        double rr = warp_sum(c_spmv<1, NT>(P, lo, hi, P.x, P.Vb, nullptr));
         if((tid & 31) == 0) xbuf[xb][tid >> 5] = rr;
-        cluster_sum_warps<CS>(cl, xbuf[xb], sdot);
+        cluster_sum_warps<CS, NT>(cl, xbuf[xb], sdot);
         xb ^= 1;
       }
       if(tid == 0) {
@@ -396,18 +622,18 @@ __global__ void __launch_bounds__(kCThreads, 1024 / kCThreads) k_c_solve(CArgs P
       }
       __syncthreads();
       if(!S.cycle) break;  // converged at the restart
-      for(int i = lo + tid; i < hi; i += kCThreads) P.Vb[i] = S.scale * P.Vb[i];
+      for(int i = lo + tid; i < hi; i += NT) P.Vb[i] = S.scale * P.Vb[i];
 
       for(int k = 1; k <= m && S.cycle; k++) {
         double *vk = P.Vb + (size_t)(k - 1) * P.ldv;
         double *w = P.Vb + (size_t)k * P.ldv;
         double *z = P.flexible ? P.Z + (size_t)(k - 1) * P.ldv : P.zt;
-        c_precond<T, CS>(P, cl, p, rank, lo, hi, vk, z);
-        c_spmv<0>(P, lo, hi, z, w, nullptr);
+        c_precond<T, CS, NT>(P, cl, p, rank, lo, hi, vk, z);
+        c_spmv<0, NT>(P, lo, hi, z, w, nullptr);
         __syncthreads();
         // first Gram-Schmidt pass: <V_j, w> for j < k and <w, w>
-        c_dots(P, lo, hi, w, k + 1, xbuf[xb]);
-        cluster_sum<CS>(cl, xbuf[xb], k + 1, sdot);
+        c_dots<NT>(P, lo, hi, w, k + 1, xbuf[xb]);
+        cluster_sum<CS, NT>(cl, xbuf[xb], k + 1, sdot);
         xb ^= 1;
         if(tid == 0) {
           S.nrm0 = sdot[k];
@@ -420,16 +646,15 @@ __global__ void __launch_bounds__(kCThreads, 1024 / kCThreads) k_c_solve(CArgs P
             S.reorth = 0;
           }
         }
-        if(tid < k) {
-          sh1[tid] = sdot[tid];
-          sH[(k - 1) * (m + 1) + tid] = sdot[tid];
-        }
+        if(tid < k) sh1[tid] = sdot[tid];
         __syncthreads();
         if(!S.cycle) break;
+        double *Hc = sH + (size_t)(k - 1) * (m + 1);
+        if(tid < 32) c_rotate(sh1, scs, ssn, k, sra, Hc);
         {
-          double v = warp_sum(c_update(P, lo, hi, w, sh1, k));
+          double v = warp_sum(c_update<NT>(P, lo, hi, w, sh1, k));
           if((tid & 31) == 0) xbuf[xb][tid >> 5] = v;
-          cluster_sum_warps<CS>(cl, xbuf[xb], sdot);
+          cluster_sum_warps<CS, NT>(cl, xbuf[xb], sdot);
           xb ^= 1;
         }
         if(tid == 0) {
@@ -439,14 +664,15 @@ __global__ void __launch_bounds__(kCThreads, 1024 / kCThreads) k_c_solve(CArgs P
         __syncthreads();
         if(S.reorth) {
           // second pass
-          c_dots(P, lo, hi, w, k, xbuf[xb]);
-          cluster_sum<CS>(cl, xbuf[xb], k, sdot);
+          c_dots<NT>(P, lo, hi, w, k, xbuf[xb]);
+          cluster_sum<CS, NT>(cl, xbuf[xb], k, sdot);
           xb ^= 1;
-          if(tid < k) sH[(k - 1) * (m + 1) + tid] = sh1[tid] + sdot[tid];
+          if(tid < k) sh1[tid] += sdot[tid];
           __syncthreads();
-          double v = warp_sum(c_update(P, lo, hi, w, sdot, k));
+          if(tid < 32) c_rotate(sh1, scs, ssn, k, sra, Hc);
+          double v = warp_sum(c_update<NT>(P, lo, hi, w, sdot, k));
           if((tid & 31) == 0) xbuf[xb][tid >> 5] = v;
-          cluster_sum_warps<CS>(cl, xbuf[xb], sdot);
+          cluster_sum_warps<CS, NT>(cl, xbuf[xb], sdot);
           xb ^= 1;
           if(tid == 0) S.rr = sdot[0];
           __syncthreads();
@@ -454,23 +680,33 @@ __global__ void __launch_bounds__(kCThreads, 1024 / kCThreads) k_c_solve(CArgs P
         // end of the Arnoldi step: h(k+1,k), rotations, stopping test
         if(tid == 0) {
           S.its += 1;
-          double *Hc = sH + (size_t)(k - 1) * (m + 1);
-          double nrm = sqrt(S.rr);
-          Hc[k] = nrm;
           S.k = k;
           S.did_cycle = 1;
-          if(!(nrm > 0.)) {
+          if(!(S.rr > 0.)) {
+            // the column without rotations, as the reference leaves it
+            for(int j = 0; j < k; j++) Hc[j] = sh1[j];
+            Hc[k] = sqrt(S.rr);
             S.breakdown = -3;
             S.cycle = 0;
           }
           else {
-            for(int i = 0; i < k - 1; i++) {
-              double a = Hc[i], c = scs[i], s = ssn[i];
-              Hc[i] = c * a + s * Hc[i + 1];
-              Hc[i + 1] = c * Hc[i + 1] - s * a;
-            }
+            const double rr = S.rr, hk = Hc[k - 1], r2 = fma(hk, hk, rr);
             double c, s;
-            givens_dev(&Hc[k - 1], &Hc[k], &c, &s);
+            if(rr > 1e-280 && r2 < 1e280) {
+              // the rotation by two independent reciprocal roots (as
+              // k_gm_update: a third of the serial chain of givens)
+              const double ri = rsqrt(rr), q = rsqrt(r2);
+              S.scale = ri;
+              c = hk * q;
+              s = rr * ri * q;
+              Hc[k - 1] = r2 * q;
+            }
+            else {
+              double x = hk, y = sqrt(rr);
+              S.scale = 1. / y;
+              givens_dev(&x, &y, &c, &s);
+              Hc[k - 1] = x;
+            }
             scs[k - 1] = c;
             ssn[k - 1] = s;
             double alpha = -s * sg[k - 1];
@@ -478,14 +714,13 @@ __global__ void __launch_bounds__(kCThreads, 1024 / kCThreads) k_c_solve(CArgs P
             sg[k] = alpha;
             alpha = fabs(alpha);
             S.res = alpha;
-            S.scale = 1. / nrm;
             if(!(k < m && !(alpha <= S.tol) && (P.maxit <= 0 || S.its < P.maxit)))
               S.cycle = 0;
           }
         }
         __syncthreads();
         if(S.cycle)
-          for(int i = lo + tid; i < hi; i += kCThreads) w[i] = S.scale * w[i];
+          for(int i = lo + tid; i < hi; i += NT) w[i] = S.scale * w[i];
       }
 
       // end of the cycle: H y = g (upper triangular), then the update.
@@ -520,20 +755,20 @@ __global__ void __launch_bounds__(kCThreads, 1024 / kCThreads) k_c_solve(CArgs P
       if(upd) {
         const int k = S.k;
         if(P.flexible) {
-          for(int i = lo + tid; i < hi; i += kCThreads) {
+          for(int i = lo + tid; i < hi; i += NT) {
             double s = P.x[i];
             for(int j = 0; j < k; j++) s += sy[j] * __ldcg(P.Z + (size_t)j * P.ldv + i);
             P.x[i] = s;
           }
         }
         else {
-          for(int i = lo + tid; i < hi; i += kCThreads) {
+          for(int i = lo + tid; i < hi; i += NT) {
             double s = 0.;
             for(int j = 0; j < k; j++) s += sy[j] * __ldcg(P.Vb + (size_t)j * P.ldv + i);
             P.u[i] = s;
           }
-          c_precond<T, CS>(P, cl, p, rank, lo, hi, P.u, P.zt);
-          for(int i = lo + tid; i < hi; i += kCThreads) P.x[i] += __ldcg(P.zt + i);
+          c_precond<T, CS, NT>(P, cl, p, rank, lo, hi, P.u, P.zt);
+          for(int i = lo + tid; i < hi; i += NT) P.x[i] += __ldcg(P.zt + i);
         }
       }
       __syncthreads();
@@ -564,14 +799,14 @@ __global__ void __launch_bounds__(kCThreads, 1024 / kCThreads) k_c_solve(CArgs P
     cl.sync();
     {
       double bb = 0.;
-      double rr = c_spmv<1>(P, lo, hi, P.x, nullptr, &bb);
-      rr = block_sum<double, kCThreads>(rr);
-      bb = block_sum<double, kCThreads>(bb);
+      double rr = c_spmv<1, NT>(P, lo, hi, P.x, nullptr, &bb);
+      rr = block_sum<double, NT>(rr);
+      bb = block_sum<double, NT>(bb);
       if(tid == 0) {
         xbuf[xb][0] = rr;
         xbuf[xb][1] = bb;
       }
-      cluster_sum<CS>(cl, xbuf[xb], 2, sdot);
+      cluster_sum<CS, NT>(cl, xbuf[xb], 2, sdot);
       xb ^= 1;
     }
     if(rank == 0 && tid == 0) {
@@ -585,11 +820,11 @@ __global__ void __launch_bounds__(kCThreads, 1024 / kCThreads) k_c_solve(CArgs P
   }
 }
 
-template <typename T, int CS>
+template <typename T, int CS, int NT = 512>
 static int launch_c(const CArgs &a, cudaStream_t st, int *nclusters)
 {
   if(CS > 8 &&
-     cudaFuncSetAttribute(k_c_solve<T, CS>, cudaFuncAttributeNonPortableClusterSizeAllowed,
+     cudaFuncSetAttribute(k_c_solve<T, CS, NT>, cudaFuncAttributeNonPortableClusterSizeAllowed,
                           1) != cudaSuccess) {
     cudaGetLastError();
     *nclusters = 0;
@@ -602,13 +837,13 @@ static int launch_c(const CArgs &a, cudaStream_t st, int *nclusters)
   attr[0].val.clusterDim.x = CS;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
-  cfg.blockDim = dim3(kCThreads, 1, 1);
+  cfg.blockDim = dim3(NT, 1, 1);
   cfg.dynamicSmemBytes = 0;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   cfg.gridDim = dim3(CS, 1, 1);
   int nc = 0;
-  cudaError_t e = cudaOccupancyMaxActiveClusters(&nc, (void *)k_c_solve<T, CS>, &cfg);
+  cudaError_t e = cudaOccupancyMaxActiveClusters(&nc, (void *)k_c_solve<T, CS, NT>, &cfg);
   if(e != cudaSuccess || nc < 1) {
     cudaGetLastError();
     *nclusters = 0;
@@ -617,7 +852,7 @@ static int launch_c(const CArgs &a, cudaStream_t st, int *nclusters)
   if(nc > a.nsys) nc = a.nsys;
   *nclusters = nc;
   cfg.gridDim = dim3((unsigned)(nc * CS), 1, 1);
-  if(cudaLaunchKernelEx(&cfg, k_c_solve<T, CS>, a) != cudaSuccess) {
+  if(cudaLaunchKernelEx(&cfg, k_c_solve<T, CS, NT>, a) != cudaSuccess) {
     // a launch the device refuses (nothing ran): the per-kernel form runs
     cudaGetLastError();
     *nclusters = 0;
@@ -631,7 +866,7 @@ int gmres_solve_batch_cluster(gb300_matrix *A, const double *val, const double *
                               bool *used, const Colouring *mc)
 {
   *used = false;
-  const int cs = p->batch_kernel;
+  int cs = p->batch_kernel;
   if(cs != 1 && cs != 2 && cs != 4 && cs != 8 && cs != 16) return GB300_OK;
   if((p->algorithm != 8 && p->algorithm != 9) ||
      (p->preconditioner != 0 && p->preconditioner != 6))
@@ -642,6 +877,16 @@ int gmres_solve_batch_cluster(gb300_matrix *A, const double *val, const double *
   if(m > kCMaxKrylov || p->nb_iter_max <= 0 || p->nb_iter_max > 100000000 || nsys < 1 ||
      p->precision == 2)
     return GB300_OK;
+  if(cs == 4) {
+    // the default: larger clusters where a few systems would leave SMs idle,
+    // while the largest system has a row per thread of its cluster.
+    // Measured (ms, 4 / 8 / 16 CTAs): 64 systems of 1,922..50,562 rows 466 /
+    // 231 / 230; 12 of 1,058..28,322 154 / 77 / 48; 32 of 450..6,962 20.4 /
+    // 13.3 / 17.8; 200 of 1,922..19,602 124 / 130 / 213
+    int most = 0;
+    for(int q = 0; q < nsys; q++) most = std::max(most, off[q + 1] - off[q]);
+    while(cs < 16 && (long long)nsys * cs < 768 && most / (2 * cs) >= 512) cs *= 2;
+  }
   int dev = 0, can = 0;
   GB_CUDA(cudaGetDevice(&dev));
   if(cudaDeviceGetAttribute(&can, cudaDevAttrClusterLaunch, dev) != cudaSuccess || !can) {

@@ -100,7 +100,8 @@ typedef struct gb300_solver_params {
   int batch_kernel;       /* Batch_Kernel: form of gb300_solve_batch: c = 1, 2,
                              4 (default), 8 or 16: one launch for the whole
                              batch, a thread-block cluster of c CTAs per
-                             system (GMRES/FGMRES, Nb_Iter_Max > 0,
+                             system (the default takes 8 or 16 for a batch of
+                             few, large systems) (GMRES/FGMRES, Nb_Iter_Max > 0,
                              Krylov_Size <= 64, at most 64 ILU(0) levels per
                              system, e.g. Renumbering_Technique 1); 0, or
                              where that does not apply: one launch per Krylov
