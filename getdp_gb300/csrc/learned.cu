@@ -27,7 +27,8 @@
 // Kernels: the forward layers on the tensor cores over 16-node tiles
 // (k_mp_layer_mma); one warp per node (lane = channel) for the input, the
 // output head and the backward pass; weight gradients accumulate per warp in
-// registers and are added with FP32 atomics (their order varies, so
+// registers, per CTA in shared memory, and are added with FP32 atomics once
+// per CTA (their order varies, so
 // gradients agree with the FP64 CPU check to FP32 rounding, not bit for
 // bit).
 #include <cuda_bf16.h>
@@ -64,6 +65,7 @@ struct MpnnGraph {
   long long nnz = 0;
   unsigned version = ~0u;
   DevBuf<float> ehat, feat, dscale;  // e_ij (nnz), f_i (n x 4), 1/sqrt(a_ii)
+  DevBuf<double> dinv;               // 1/sqrt(a_ii) in FP64
   DevBuf<int> diag, tpos;            // position of a_ii, of (j,i) for entry (i,j)
   DevBuf<float> h, m;                // (L+1) x n x H, L x n x H
   DevBuf<float> dh, dm;              // n x H work for the backward pass
@@ -90,12 +92,13 @@ __global__ void k_round_bf16(int n, const float *__restrict__ w, float *__restri
   if(i < n) q[i] = bf16_round(w[i]);
 }
 
-// e_ij, node features, 1/sqrt(a_ii), diagonal and transpose positions
+// 1/sqrt(a_ii), diagonal positions; then e_ij, node features and transpose
+// positions.  e_ij is formed from the two inverse roots: a root and a division
+// per entry were some 40 FP64 instructions (at 65,025 rows 30 us).
 __global__ void k_mp_features(int n, const int *__restrict__ rowptr,
                               const int *__restrict__ col, const double *__restrict__ val,
-                              float *__restrict__ ehat, float *__restrict__ feat,
-                              float *__restrict__ dscale, int *__restrict__ diag,
-                              int *__restrict__ tpos, int *__restrict__ bad)
+                              float *__restrict__ dscale, double *__restrict__ dinv,
+                              int *__restrict__ diag, int *__restrict__ bad)
 {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if(i >= n) return;
@@ -106,24 +109,25 @@ __global__ void k_mp_features(int n, const int *__restrict__ rowptr,
     return;
   }
   diag[i] = di;
-  dscale[i] = (float)(1. / sqrt(val[di]));
+  const double r = 1. / sqrt(val[di]);
+  dinv[i] = r;
+  dscale[i] = (float)r;
 }
 
 __global__ void k_mp_edges(int n, const int *__restrict__ rowptr,
                            const int *__restrict__ col, const double *__restrict__ val,
-                           const int *__restrict__ diag, float *__restrict__ ehat,
+                           const double *__restrict__ dinv, float *__restrict__ ehat,
                            float *__restrict__ feat, int *__restrict__ tpos,
                            int *__restrict__ bad)
 {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if(i >= n) return;
   int s = rowptr[i], e = rowptr[i + 1];
-  double aii = val[diag[i]];
+  const double di = dinv[i];
   float sum = 0.f, mx = 0.f;
   for(int k = s; k < e; k++) {
     int j = col[k];
-    double ajj = val[diag[j]];
-    float v = (float)(val[k] / sqrt(aii * ajj));
+    float v = (float)(val[k] * di * dinv[j]);
     ehat[k] = v;
     int t = find_col(col, rowptr[j], rowptr[j + 1], i);
     if(t < 0) atomicExch(bad, 1);
@@ -389,6 +393,24 @@ __global__ void k_mp_dg(int n, const int *__restrict__ rowptr, const int *__rest
   }
 }
 
+// The warps' sums of one value per lane, added to g[lane * stride] once per
+// CTA (a warp's own atomics on those few addresses had been most of the small
+// kernels' time: 9,728 warps on 160 addresses, 198 us at 16,384 nodes)
+__device__ __forceinline__ void cta_add(float v, float *g, int stride)
+{
+  __shared__ float s[kNodeWarps][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  __syncthreads();  // (the previous call's reads)
+  s[warp][lane] = v;
+  __syncthreads();
+  if(warp == 0) {
+    float t = 0.f;
+#pragma unroll
+    for(int w = 0; w < kNodeWarps; w++) t += s[w][lane];
+    atomicAdd(g + lane * stride, t);
+  }
+}
+
 // backward of the output head: weight gradients and dh of the last layer
 __global__ void __launch_bounds__(32 * kNodeWarps)
 k_mp_output_bwd(int n, const int *__restrict__ rowptr, const int *__restrict__ col,
@@ -422,11 +444,19 @@ k_mp_output_bwd(int n, const int *__restrict__ rowptr, const int *__restrict__ c
     }
     dh[(size_t)i * kH + lane] = dhi;
   }
-  atomicAdd(&grad[kOffWo + lane], gwo);
-  atomicAdd(&grad[kOffWd + lane], gwd);
-  if(lane == 0) {
-    atomicAdd(&grad[kOffCo], gco);
-    atomicAdd(&grad[kOffBd], gbd);
+  cta_add(gwo, grad + kOffWo, 1);
+  cta_add(gwd, grad + kOffWd, 1);
+  // the two scalars (lane 0's) through lanes 0 and 1
+  const float gb1 = __shfl_sync(0xffffffffu, gbd, 0);
+  static_assert(kOffBd - kOffCo == kH + 1, "lane 1 adds to b_d");
+  __shared__ float sc[kNodeWarps][2];
+  if(lane < 2) sc[threadIdx.x >> 5][lane] = lane ? gb1 : gco;
+  __syncthreads();
+  if(threadIdx.x < 2) {
+    float t = 0.f;
+#pragma unroll
+    for(int w = 0; w < kNodeWarps; w++) t += sc[w][threadIdx.x];
+    atomicAdd(&grad[threadIdx.x ? kOffBd : kOffCo], t);
   }
 }
 
@@ -439,12 +469,14 @@ k_mp_layer_bwd1(int n, const float *__restrict__ wl, const float *__restrict__ h
                 float *__restrict__ dhin, float *__restrict__ gl)
 {
   __shared__ float Ws[kH][kH + 1], Wn[kH][kH + 1];
-  __shared__ float acc[kLayerSize];  // the CTA's weight gradients
+  // the CTA's weight gradients, [input channel][output channel]: a warp's
+  // lanes are output channels, so they meet 32 banks (in the weights' own
+  // order all 32 met one bank, 50 of this kernel's 64 us at 16,384 nodes)
+  __shared__ float acc[2 * kH + 1][kH + 1];
   for(int t = threadIdx.x; t < kH * kH; t += blockDim.x) {
     Ws[t / kH][t % kH] = wl[t];
     Wn[t / kH][t % kH] = wl[kH * kH + t];
   }
-  for(int t = threadIdx.x; t < kLayerSize; t += blockDim.x) acc[t] = 0.f;
   __syncthreads();
   int lane = threadIdx.x & 31;
   float gws[kH], gwn[kH], gb = 0.f;
@@ -470,14 +502,23 @@ k_mp_layer_bwd1(int n, const float *__restrict__ wl, const float *__restrict__ h
     dm[o] = dmi;
     dhin[o] = dsi;
   }
+  // the warps one after the other, without atomics
+  for(int w = 0; w < kNodeWarps; w++) {
+    if((threadIdx.x >> 5) == w) {
 #pragma unroll
-  for(int d = 0; d < kH; d++) {
-    atomicAdd(&acc[lane * kH + d], gws[d]);
-    atomicAdd(&acc[kH * kH + lane * kH + d], gwn[d]);
+      for(int d = 0; d < kH; d++) {
+        acc[d][lane] = (w ? acc[d][lane] : 0.f) + gws[d];
+        acc[kH + d][lane] = (w ? acc[kH + d][lane] : 0.f) + gwn[d];
+      }
+      acc[2 * kH][lane] = (w ? acc[2 * kH][lane] : 0.f) + gb;
+    }
+    __syncthreads();
   }
-  atomicAdd(&acc[2 * kH * kH + lane], gb);
-  __syncthreads();
-  for(int t = threadIdx.x; t < kLayerSize; t += blockDim.x) atomicAdd(&gl[t], acc[t]);
+  for(int t = threadIdx.x; t < 2 * kH * kH; t += blockDim.x) {
+    const int half = t / (kH * kH), c = (t / kH) % kH, d = t % kH;
+    atomicAdd(&gl[t], acc[half * kH + d][c]);
+  }
+  if(threadIdx.x < kH) atomicAdd(&gl[2 * kH * kH + threadIdx.x], acc[2 * kH][threadIdx.x]);
 }
 
 // pass 2: dh_in_i += sum_{j != i} e_ji dm_j  (e symmetric in the pattern:
@@ -514,8 +555,8 @@ k_mp_input_bwd(int n, const float *__restrict__ feat, const float *__restrict__ 
     for(int f = 0; f < kFin; f++) gw[f] += dz * feat[4 * i + f];
   }
 #pragma unroll
-  for(int f = 0; f < kFin; f++) atomicAdd(&grad[kOffWin + lane * kFin + f], gw[f]);
-  atomicAdd(&grad[kOffBin + lane], gb);
+  for(int f = 0; f < kFin; f++) cta_add(gw[f], grad + kOffWin + f, kFin);
+  cta_add(gb, grad + kOffBin, 1);
 }
 
 __global__ void k_adam(int np, float *__restrict__ w, const float *__restrict__ g,
@@ -544,6 +585,7 @@ static int mp_prepare(gb300_mpnn *net, const gb300_matrix *A)
   GB_TRY(g.ehat.alloc(A->nnz));
   GB_TRY(g.feat.alloc((size_t)n * 4));
   GB_TRY(g.dscale.alloc(n));
+  GB_TRY(g.dinv.alloc(n));
   GB_TRY(g.diag.alloc(n));
   GB_TRY(g.tpos.alloc(A->nnz));
   GB_TRY(g.h.alloc((size_t)(kLayers + 1) * n * kH));
@@ -555,11 +597,9 @@ static int mp_prepare(gb300_mpnn *net, const gb300_matrix *A)
   GB_TRY(bad.alloc(1));
   GB_CUDA(cudaMemsetAsync(bad.p, 0, sizeof(int), st));
   k_mp_features<<<grid_for(n, 256), 256, 0, st>>>(n, A->rowptr.p, A->col.p, A->val.p,
-                                                   g.ehat.p, g.feat.p, g.dscale.p,
-                                                   g.diag.p, g.tpos.p, bad.p);
-  k_mp_edges<<<grid_for(n, 256), 256, 0, st>>>(n, A->rowptr.p, A->col.p, A->val.p,
-                                                g.diag.p, g.ehat.p, g.feat.p, g.tpos.p,
-                                                bad.p);
+                                                   g.dscale.p, g.dinv.p, g.diag.p, bad.p);
+  k_mp_edges<<<grid_for(n, 128), 128, 0, st>>>(n, A->rowptr.p, A->col.p, A->val.p, g.dinv.p,
+                                                g.ehat.p, g.feat.p, g.tpos.p, bad.p);
   int hb = 0;
   GB_CUDA(cudaMemcpyAsync(&hb, bad.p, sizeof(int), cudaMemcpyDeviceToHost, st));
   GB_CUDA(cudaStreamSynchronize(st));
@@ -646,12 +686,13 @@ static int mp_loss_backward(gb300_mpnn *net, gb300_matrix *A, const double *r1,
   k_mp_dg<<<grid_for(n, 256), 256, 0, st>>>(n, A->rowptr.p, A->col.p, g.dscale.p, w.p, r1,
                                             1. / S, dg.p);
   int grid = grid_for(n, kNodeWarps, kReduceBlocks);
+  // the weight gradients are added once per CTA: no more CTAs than the work
+  // needs (eight nodes a warp, at most two CTAs per SM)
+  const int gw = grid_for(n, 8 * kNodeWarps, 2 * 152);
   float *dhA = g.dh.p, *dhB = g.dh.p + (size_t)n * kH;
-  k_mp_output_bwd<<<grid, 32 * kNodeWarps, 0, st>>>(
+  k_mp_output_bwd<<<gw, 32 * kNodeWarps, 0, st>>>(
     n, A->rowptr.p, A->col.p, g.ehat.p, g.tpos.p, net->wq.p,
     g.h.p + (size_t)kLayers * n * kH, dg.p, dhA, net->grad.p);
-  // few CTAs for the weight-gradient pass: each CTA adds its sums once
-  const int gw = grid_for(n, kNodeWarps, 2 * 152);
   for(int l = kLayers - 1; l >= 0; l--) {
     const float *wl = net->wq.p + kOffLayer + l * kLayerSize;
     k_mp_layer_bwd1<<<gw, 32 * kNodeWarps, 0, st>>>(
@@ -662,7 +703,7 @@ static int mp_loss_backward(gb300_mpnn *net, gb300_matrix *A, const double *r1,
                                                        g.tpos.p, g.dm.p, dhB);
     std::swap(dhA, dhB);
   }
-  k_mp_input_bwd<<<grid, 32 * kNodeWarps, 0, st>>>(n, g.feat.p, g.h.p, dhA, net->grad.p);
+  k_mp_input_bwd<<<gw, 32 * kNodeWarps, 0, st>>>(n, g.feat.p, g.h.p, dhA, net->grad.p);
   GB_CUDA(cudaGetLastError());
   GB_CUDA(cudaStreamSynchronize(st));
   *loss = hl / E;
