@@ -271,7 +271,7 @@ k_bsr_spmv(int nn, const int *__restrict__ ptr, const int *__restrict__ col,
         part[b] = 0.;
     // MODE 2 with dot_out: the last block to finish sums <p, y> itself
     if(MODE == 2 && dot_out && arrive_last(counter)) {
-      double d = sum_partials_l2<256>(part);
+      double d = sum_partials_l2<256>(part, gridDim.x);
       if(threadIdx.x == 0) *dot_out = d;
     }
   }
@@ -391,7 +391,7 @@ k_bsr_spmv_pf(int nn, const int *__restrict__ ptr, const int *__restrict__ col,
       for(int b = gridDim.x + threadIdx.x; b < kReduceBlocks; b += blockDim.x)
         part[b] = 0.;
     if(MODE == 2 && dot_out && arrive_last(counter)) {
-      double d = sum_partials_l2<256>(part);
+      double d = sum_partials_l2<256>(part, gridDim.x);
       if(threadIdx.x == 0) *dot_out = d;
     }
   }
@@ -625,7 +625,7 @@ k_bsr_spmv_tma(int nn, const int *__restrict__ ptr, const int *__restrict__ col,
     if(blockIdx.x == 0)
       for(int b = gridDim.x + tid; b < kReduceBlocks; b += blockDim.x) part[b] = 0.;
     if(MODE == 2 && dot_out && arrive_last(counter)) {
-      double d = sum_partials_l2<kTmaThreads>(part);
+      double d = sum_partials_l2<kTmaThreads>(part, gridDim.x);
       if(tid == 0) *dot_out = d;
     }
   }
@@ -666,7 +666,9 @@ static void launch_plain(const Bsr3 &B, const T *val, const T *p, const T *b,
 {
   static int grid = 0;  // per instantiation
   if(!grid) grid = resident_grid(k_bsr_spmv<MODE, T, L, U, C, M>, 256, 0);
-  k_bsr_spmv<MODE, T, L, U, C, M><<<grid, 256, 0, st>>>(
+  // (no CTA without rows: each would still arrive at the sum's counter)
+  const int g = grid_for(B.nn, 256 / L, grid);
+  k_bsr_spmv<MODE, T, L, U, C, M><<<g, 256, 0, st>>>(
     B.nn, B.ptr.p, B.col.p, val, B.pstride, p, b, y, part, flag, dot_out, counter);
 }
 
@@ -677,7 +679,8 @@ static void launch_pf(const Bsr3 &B, const T *val, const T *p, const T *b, T *y,
 {
   static int grid = 0;  // per instantiation
   if(!grid) grid = resident_grid(k_bsr_spmv_pf<MODE, T, L, U, M>, 256, 0);
-  k_bsr_spmv_pf<MODE, T, L, U, M><<<grid, 256, 0, st>>>(
+  const int g = grid_for(B.nn, 256 / L, grid);
+  k_bsr_spmv_pf<MODE, T, L, U, M><<<g, 256, 0, st>>>(
     B.nn, B.ptr.p, B.col.p, val, B.pstride, p, b, y, part, flag, dot_out, counter);
 }
 

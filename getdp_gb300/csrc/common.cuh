@@ -153,9 +153,10 @@ template <typename T, int NT> __device__ __forceinline__ T block_sum(T v)
   v = warp_sum(v);
   if((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
   __syncthreads();
+  // the warps' sums in a tree as well (one after the other, eight FP64
+  // additions of some 85 ns each stood at the end of every reduction)
   T s = 0;
-  if(threadIdx.x == 0)
-    for(int w = 0; w < NT / 32; w++) s += red[w];
+  if(threadIdx.x < 32) s = warp_sum(threadIdx.x < NT / 32 ? red[threadIdx.x] : (T)0);
   __syncthreads();
   return s;
 }
@@ -230,12 +231,13 @@ __device__ __forceinline__ bool arrive_last(unsigned *counter)
   return arrive_last(counter, gridDim.x * gridDim.y * gridDim.z);
 }
 
-// the kReduceBlocks partials summed in the fixed order of the one-block
-// control kernels (NT threads), read through L2
-template <int NT> __device__ __forceinline__ double sum_partials_l2(const double *part)
+// the first np partials summed in a fixed order (NT threads), read through L2
+template <int NT>
+__device__ __forceinline__ double sum_partials_l2(const double *part, int np)
 {
   double s = 0.;
-  for(int i = threadIdx.x; i < kReduceBlocks; i += NT) s += __ldcg(part + i);
+#pragma unroll 5
+  for(int i = threadIdx.x; i < np; i += NT) s += __ldcg(part + i);
   return block_sum<double, NT>(s);
 }
 

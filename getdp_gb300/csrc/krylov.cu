@@ -13,6 +13,8 @@
 //
 // Dot products use fixed-size partial-sum grids summed in a fixed order, so
 // a solve is bit-reproducible run to run.
+#include <algorithm>
+
 #include "krylov.cuh"
 
 namespace gb {
@@ -145,19 +147,12 @@ __device__ __forceinline__ void st4(double *p, long long i4, const double (&v)[4
   reinterpret_cast<double2 *>(p)[2 * i4 + 1] = make_double2(v[2], v[3]);
 }
 
-// brkdn (iters.f:3368-3402) on <p, Ap>: 0, or the ipar(1) code
+// brkdn (iters.f:3368-3402) on <p, Ap>: 0, or the ipar(1) code (its tests on
+// 1 / pq come down to pq being finite: no division)
 __device__ __forceinline__ int cg_breakdown(double pq)
 {
-  if(pq > 0.) {
-    double b = 1. / pq;
-    return (b > 0.) ? 0 : -9;
-  }
-  if(pq < 0.) {
-    double b = 1. / pq;
-    return (b < 0.) ? 0 : -9;
-  }
   if(pq == 0.) return -3;
-  return -9;
+  return fabs(pq) <= 1.7976931348623157e308 ? 0 : -9;
 }
 
 // the stopping test of the FP64 CG (stopbis: the iteration cap first, then
@@ -176,8 +171,8 @@ __device__ void cg_check_tail(CgState *S, double rr)
     S->active = 0;
     return;
   }
-  S->beta = S->res * S->res / S->rho;
-  S->rho = S->res * S->res;
+  S->beta = rr / S->rho;  // (beside the root, not after it)
+  S->rho = rr;
 }
 
 // the reliable-update test of the mixed CG: replace the residual when the
@@ -211,9 +206,21 @@ k_cg_step(int n, CgState *__restrict__ S, T *__restrict__ x, T *__restrict__ r,
 {
   if(!S->go) return;
   // alpha and the breakdown test once per CTA: FP64 divisions in every
-  // thread would keep the FP64 pipe busier than the vector traffic
+  // thread would keep the FP64 pipe busier than the vector traffic.  The
+  // first entries are on their way meanwhile.  Vectors are cudaMalloc'ed
+  // (256-byte aligned): groups of four, then the n % 4 remainder
   __shared__ T s_alpha;
   __shared__ int s_bad;
+  const long long stride = (long long)gridDim.x * blockDim.x;
+  const long long n4 = n / 4, first = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  long long i4 = first;
+  T xv[4], rv[4], pv[4], qv[4];
+  if(i4 < n4) {
+    ld4(x, i4, xv);
+    ld4(r, i4, rv);
+    ld4(p, i4, pv);
+    ld4(q, i4, qv);
+  }
   const double pq = S->pq, rho = S->rho;
   if(threadIdx.x == 0) {
     s_bad = cg_breakdown(pq);
@@ -223,18 +230,8 @@ k_cg_step(int n, CgState *__restrict__ S, T *__restrict__ x, T *__restrict__ r,
   const int bad = s_bad;
   typename Acc<T>::type v = 0;
   if(!bad) {
-    // vectors are cudaMalloc'ed (256-byte aligned): groups of four, then
-    // the n % 4 remainder
     const T a = s_alpha;
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    const long long n4 = n / 4;
-    for(long long i4 = (long long)blockIdx.x * blockDim.x + threadIdx.x; i4 < n4;
-        i4 += stride) {
-      T xv[4], rv[4], pv[4], qv[4];
-      ld4(x, i4, xv);
-      ld4(r, i4, rv);
-      ld4(p, i4, pv);
-      ld4(q, i4, qv);
+    while(i4 < n4) {
 #pragma unroll
       for(int c = 0; c < 4; c++) {
         xv[c] += a * pv[c];
@@ -243,9 +240,15 @@ k_cg_step(int n, CgState *__restrict__ S, T *__restrict__ x, T *__restrict__ r,
       }
       st4(x, i4, xv);
       st4(r, i4, rv);
+      i4 += stride;
+      if(i4 < n4) {
+        ld4(x, i4, xv);
+        ld4(r, i4, rv);
+        ld4(p, i4, pv);
+        ld4(q, i4, qv);
+      }
     }
-    for(long long i = 4 * n4 + (long long)blockIdx.x * blockDim.x + threadIdx.x;
-        i < n; i += stride) {
+    for(long long i = 4 * n4 + first; i < n; i += stride) {
       x[i] += a * p[i];
       T ri = r[i] - a * q[i];
       r[i] = ri;
@@ -257,7 +260,7 @@ k_cg_step(int n, CgState *__restrict__ S, T *__restrict__ x, T *__restrict__ r,
   if(blockIdx.x == 0)
     for(int b = gridDim.x + threadIdx.x; b < kReduceBlocks; b += blockDim.x) part[b] = 0.;
   if(!arrive_last(&S->tick_step)) return;
-  double rr = sum_partials_l2<256>(part);
+  double rr = sum_partials_l2<256>(part, gridDim.x);
   if(threadIdx.x == 0) {
     S->its += 1;
     if(bad) {
@@ -336,7 +339,7 @@ k_cg_spmv(int n, const int *__restrict__ rowptr, const int *__restrict__ col,
   double s = block_sum<double, 256>((double)red);
   if(threadIdx.x == 0) part[blockIdx.x] = s;
   if(arrive_last(&S->tick_dot)) {
-    double d = sum_partials_l2<256>(part);
+    double d = sum_partials_l2<256>(part, gridDim.x);
     if(threadIdx.x == 0) S->pq = d;
   }
 }
@@ -346,12 +349,13 @@ static void cg_spmv(const gb300_matrix *A, const V *val, const XT *p, XT *q,
                     double *part, CgState *S, cudaStream_t st)
 {
   int n = A->n;
+  const int g = grid_for(n, 256 / A->tpr, kReduceBlocks);
   switch(A->tpr) {
-  case 2: k_cg_spmv<2><<<kReduceBlocks, 256, 0, st>>>(n, A->rowptr.p, A->col.p, val, p, q, part, S); break;
-  case 4: k_cg_spmv<4><<<kReduceBlocks, 256, 0, st>>>(n, A->rowptr.p, A->col.p, val, p, q, part, S); break;
-  case 8: k_cg_spmv<8><<<kReduceBlocks, 256, 0, st>>>(n, A->rowptr.p, A->col.p, val, p, q, part, S); break;
-  case 16: k_cg_spmv<16><<<kReduceBlocks, 256, 0, st>>>(n, A->rowptr.p, A->col.p, val, p, q, part, S); break;
-  default: k_cg_spmv<32><<<kReduceBlocks, 256, 0, st>>>(n, A->rowptr.p, A->col.p, val, p, q, part, S); break;
+  case 2: k_cg_spmv<2><<<g, 256, 0, st>>>(n, A->rowptr.p, A->col.p, val, p, q, part, S); break;
+  case 4: k_cg_spmv<4><<<g, 256, 0, st>>>(n, A->rowptr.p, A->col.p, val, p, q, part, S); break;
+  case 8: k_cg_spmv<8><<<g, 256, 0, st>>>(n, A->rowptr.p, A->col.p, val, p, q, part, S); break;
+  case 16: k_cg_spmv<16><<<g, 256, 0, st>>>(n, A->rowptr.p, A->col.p, val, p, q, part, S); break;
+  default: k_cg_spmv<32><<<g, 256, 0, st>>>(n, A->rowptr.p, A->col.p, val, p, q, part, S); break;
   }
 }
 
@@ -384,7 +388,10 @@ static int cg_core(cudaStream_t st, int n, SPMV spmv_dot, const T *rhs, T *y,
 
   // capture a batch of iterations once
   const int batch = n > 200000 ? 16 : 32;
-  const int step_grid = resident_grid(k_cg_step<T, false>, 256, 0);
+  // no CTA without rows: each would still arrive at the counter the step's
+  // sums wait for (1,216 CTAs for 46 CTAs' rows at 34,914 unknowns)
+  const int step_grid =
+    std::min(resident_grid(k_cg_step<T, false>, 256, 0), grid_for((n + 3) / 4, 256));
   cudaGraph_t graph;
   cudaGraphExec_t exec;
   GB_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
@@ -619,7 +626,8 @@ static int cg_mixed_core(cudaStream_t st, int n, SPMV32 spmv32, RES64 res64,
   // resumes.  The iterations and their arithmetic are those of the one-graph
   // sequence; only the place where the update kernels run moves.
   const int batch = n > 200000 ? 16 : 32;
-  const int step_grid = resident_grid(k_cg_step<float, true>, 256, 0);
+  const int step_grid =
+    std::min(resident_grid(k_cg_step<float, true>, 256, 0), grid_for((n + 3) / 4, 256));
   cudaGraph_t graph, ugraph;
   cudaGraphExec_t exec, uexec;
   GB_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
