@@ -1063,9 +1063,7 @@ int generate_pattern(gb300_matrix *A, const gb300_term_batch *t)
       t->n_elems, B.p_coef2, B.cflag.p);
     flag = B.cflag.p;
   }
-  A->hr.clear();
-  A->hc.clear();
-  A->hv.clear();
+  A->drop_staged();
   const long long nent = (long long)t->n_elems * nloc;
   GenCache *G = A->ctx->gen;
   // the same element table as the cached pattern's: reuse it

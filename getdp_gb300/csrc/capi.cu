@@ -1,6 +1,7 @@
 // The C ABI (include/getdp_gb300.h): handles, parameters, vectors,
 // matrices, the batched element loop and the solve entry point.
 #include <cctype>
+#include <utility>
 #include <cstring>
 #include <string>
 
@@ -57,6 +58,69 @@ __global__ void k_add_values(int count, const int *__restrict__ idx,
     int i = idx[k];
     if(i >= 0 && i < n) v[i] += val[k];
   }
+}
+
+// the first entry with an index outside [0, n), if any
+__global__ void k_bad_entry(long long m, int n, const int *__restrict__ r,
+                            const int *__restrict__ c, unsigned long long *__restrict__ first)
+{
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if(t < m && ((unsigned)r[t] >= (unsigned)n || (unsigned)c[t] >= (unsigned)n))
+    atomicMin(first, (unsigned long long)t);
+}
+
+// Bulk adds of this many entries and more go to the device at once, where
+// their indices are checked (1.6 M entries: 2.0 ms in the host's range check
+// and copies, 0.17 ms here); smaller ones are staged on the host.
+constexpr long long kBulkAdd = 16384;
+
+// room for `extra` more staged entries, the present ones kept
+template <typename T>
+static int grow(DevBuf<T> &b, long long have, long long extra, cudaStream_t st)
+{
+  if((size_t)(have + extra) <= b.n) return GB300_OK;
+  if(have == 0) return b.alloc(extra);
+  DevBuf<T> t;
+  GB_TRY(t.alloc((have + extra) * 3 / 2));
+  GB_CUDA(cudaMemcpyAsync(t.p, b.p, sizeof(T) * have, cudaMemcpyDeviceToDevice, st));
+  std::swap(t.p, b.p);
+  std::swap(t.n, b.n);
+  std::swap(t.from, b.from);
+  return GB300_OK;  // (t's memory is freed in the stream's order)
+}
+
+static int stage_bulk(gb300_matrix *A, long long count, const int *i, const int *j,
+                      const double *v)
+{
+  PoolScope pool_scope(A->ctx);
+  cudaStream_t st = A->ctx->stream;
+  const long long host = (long long)A->hr.size(), at = A->staged + host;
+  GB_TRY(grow(A->sr, A->staged, host + count, st));
+  GB_TRY(grow(A->sc, A->staged, host + count, st));
+  GB_TRY(grow(A->sv, A->staged, host + count, st));
+  if(host > 0) {  // entries staged on the host were added before
+    GB_TRY(fetch_pageable(A->ctx, A->sr.p + A->staged, A->hr.data(), sizeof(int) * host));
+    GB_TRY(fetch_pageable(A->ctx, A->sc.p + A->staged, A->hc.data(), sizeof(int) * host));
+    GB_TRY(fetch_pageable(A->ctx, A->sv.p + A->staged, A->hv.data(), sizeof(double) * host));
+  }
+  GB_TRY(fetch_pageable(A->ctx, A->sr.p + at, i, sizeof(int) * count));
+  GB_TRY(fetch_pageable(A->ctx, A->sc.p + at, j, sizeof(int) * count));
+  GB_TRY(fetch_pageable(A->ctx, A->sv.p + at, v, sizeof(double) * count));
+  DevBuf<unsigned long long> first;
+  GB_TRY(first.alloc(1));
+  GB_CUDA(cudaMemsetAsync(first.p, 0xff, sizeof(unsigned long long), st));
+  k_bad_entry<<<grid_for(count, 256), 256, 0, st>>>(count, A->n, A->sr.p + at, A->sc.p + at,
+                                                    first.p);
+  unsigned long long h = 0;
+  GB_CUDA(cudaMemcpyAsync(&h, first.p, sizeof(h), cudaMemcpyDeviceToHost, st));
+  GB_CUDA(cudaStreamSynchronize(st));  // the caller's arrays have been read
+  if(h != ~0ull) {  // nothing of this call is added
+    set_error("entry %lld (%d, %d) out of range [0, %d)", (long long)h, i[h], j[h], A->n);
+    return GB300_ERR_ARG;
+  }
+  A->drop_staged_host();
+  A->staged = at + count;
+  return GB300_OK;
 }
 
 __global__ void k_add_diag(int n, const int *__restrict__ rowptr,
@@ -480,9 +544,7 @@ int gb300_matrix_destroy(gb300_matrix *A)
 int gb300_matrix_reset(gb300_matrix *A)
 {
   GB_TRY(check(A, "matrix"));
-  A->hr.clear();
-  A->hc.clear();
-  A->hv.clear();
+  A->drop_staged();
   A->csr_valid = false;
   A->val32_valid = false;
   gb::coarse_values_changed(A);
@@ -533,6 +595,7 @@ int gb300_matrix_add_coo(gb300_matrix *A, long long count, const int *i,
   GB_TRY(check(i, "i"));
   GB_TRY(check(j, "j"));
   GB_TRY(check(v, "v"));
+  if(count >= kBulkAdd) return stage_bulk(A, count, i, j, v);
   for(long long k = 0; k < count; k++)
     if(i[k] < 0 || i[k] >= A->n || j[k] < 0 || j[k] >= A->n) {
       set_error("entry %lld (%d, %d) out of range [0, %d)", k, i[k], j[k], A->n);
@@ -549,48 +612,36 @@ int gb300_matrix_assemble(gb300_matrix *A)
   gb::NvtxRange nvtx_range("gb300_matrix_assemble");
   GB_TRY(check(A, "matrix"));
   gb::PoolScope pool_scope(A->ctx);
-  if(A->hr.empty() && A->csr_valid) return GB300_OK;
+  if(A->hr.empty() && A->staged == 0 && A->csr_valid) return GB300_OK;
   cudaStream_t st = A->ctx->stream;
-  long long m = (long long)A->hr.size();
   // existing device entries come first: they were added before
-  std::vector<int> r, c;
-  std::vector<double> v;
-  if(A->csr_valid && A->nnz > 0) {
-    std::vector<int> rp(A->n + 1), cc(A->nnz);
-    std::vector<double> vv(A->nnz);
-    GB_CUDA(cudaMemcpyAsync(rp.data(), A->rowptr.p, sizeof(int) * (A->n + 1), cudaMemcpyDeviceToHost, st));
-    GB_CUDA(cudaMemcpyAsync(cc.data(), A->col.p, sizeof(int) * A->nnz, cudaMemcpyDeviceToHost, st));
-    GB_CUDA(cudaMemcpyAsync(vv.data(), A->val.p, sizeof(double) * A->nnz, cudaMemcpyDeviceToHost, st));
-    GB_CUDA(cudaStreamSynchronize(st));
-    for(int row = 0; row < A->n; row++)
-      for(int k = rp[row]; k < rp[row + 1]; k++) {
-        r.push_back(row);
-        c.push_back(cc[k]);
-        v.push_back(vv[k]);
-      }
-  }
-  r.insert(r.end(), A->hr.begin(), A->hr.end());
-  c.insert(c.end(), A->hc.begin(), A->hc.end());
-  v.insert(v.end(), A->hv.begin(), A->hv.end());
-  m = (long long)r.size();
+  const long long old = A->csr_valid ? A->nnz : 0, have = old + A->staged;
+  const long long added = (long long)A->hr.size(), m = have + added;
   DevBuf<int> dr, dc;
   DevBuf<double> dv;
   GB_TRY(dr.alloc(m > 0 ? m : 1));
   GB_TRY(dc.alloc(m > 0 ? m : 1));
   GB_TRY(dv.alloc(m > 0 ? m : 1));
-  if(m > 0) {
-    GB_CUDA(cudaMemcpyAsync(dr.p, r.data(), sizeof(int) * m, cudaMemcpyHostToDevice, st));
-    GB_CUDA(cudaMemcpyAsync(dc.p, c.data(), sizeof(int) * m, cudaMemcpyHostToDevice, st));
-    GB_CUDA(cudaMemcpyAsync(dv.p, v.data(), sizeof(double) * m, cudaMemcpyHostToDevice, st));
+  if(old > 0) GB_TRY(csr_triplets(A, dr.p, dc.p, dv.p));
+  if(A->staged > 0) {
+    GB_CUDA(cudaMemcpyAsync(dr.p + old, A->sr.p, sizeof(int) * A->staged,
+                            cudaMemcpyDeviceToDevice, st));
+    GB_CUDA(cudaMemcpyAsync(dc.p + old, A->sc.p, sizeof(int) * A->staged,
+                            cudaMemcpyDeviceToDevice, st));
+    GB_CUDA(cudaMemcpyAsync(dv.p + old, A->sv.p, sizeof(double) * A->staged,
+                            cudaMemcpyDeviceToDevice, st));
+  }
+  if(added > 0) {
+    GB_TRY(fetch_pageable(A->ctx, dr.p + have, A->hr.data(), sizeof(int) * added));
+    GB_TRY(fetch_pageable(A->ctx, dc.p + have, A->hc.data(), sizeof(int) * added));
+    GB_TRY(fetch_pageable(A->ctx, dv.p + have, A->hv.data(), sizeof(double) * added));
   }
   if(A->ilu) {
     ilu_free(A->ilu);
     A->ilu = nullptr;
   }
   GB_TRY(build_csr_from_coo(A, m, dr.p, dc.p, dv.p));
-  A->hr.clear();
-  A->hc.clear();
-  A->hv.clear();
+  A->drop_staged();
   return GB300_OK;
 }
 
@@ -686,9 +737,7 @@ int gb300_matrix_set_csr(gb300_matrix *A, long long nnz, const int *rowptr,
   A->block3 = false;
   A->node_blocks = false;
   A->bsr_var32 = A->bsr_var64 = -1;
-  A->hr.clear();
-  A->hc.clear();
-  A->hv.clear();
+  A->drop_staged();
   if(A->ilu) {
     ilu_free(A->ilu);
     A->ilu = nullptr;

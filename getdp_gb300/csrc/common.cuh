@@ -392,6 +392,26 @@ struct gb300_matrix {
   // host staging of LinAlg-style scalar adds, in call order
   std::vector<int> hr, hc;
   std::vector<double> hv;
+  // bulk adds, staged on the device before the host's entries
+  gb::DevBuf<int> sr, sc;
+  gb::DevBuf<double> sv;
+  long long staged = 0;
+  void drop_staged_host()
+  {
+    hr.clear();
+    hc.clear();
+    hv.clear();
+  }
+  void drop_staged()
+  {
+    drop_staged_host();
+    staged = 0;
+    if(sv.n > (1u << 26)) {  // more than 1 GB is not kept for the next adds
+      sr.release();
+      sc.release();
+      sv.release();
+    }
+  }
   // device CSR (0-based, rows sorted by column)
   gb::DevBuf<int> rowptr, col;
   gb::DevBuf<double> val;

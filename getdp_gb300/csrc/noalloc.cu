@@ -126,7 +126,7 @@ extern "C" int gb300_residual_noalloc(gb300_matrix *A, const gb300_vector *x,
               kMaxBlocks);
     return GB300_ERR_CAPACITY;
   }
-  if(!A->csr_valid || !A->hr.empty()) {
+  if(!A->csr_valid || !A->hr.empty() || A->staged > 0) {
     set_error("gb300_residual_noalloc: the matrix must be assembled first "
               "(assembling would allocate)");
     return GB300_ERR_ARG;

@@ -15,6 +15,9 @@ int build_pattern_from_elements(gb300_matrix *A, int ne, int nloc,
                                 int complex_mode, int rep = 1);
 int build_csr_from_coo(gb300_matrix *A, long long m, const int *d_r,
                        const int *d_c, const double *d_v);
+// A's CSR as row-ordered triplets (device arrays of nnz entries)
+int csr_triplets(const gb300_matrix *A, int *d_r, int *d_c, double *d_v);
+int fetch_pageable(gb300_ctx *ctx, void *dst, const void *src, size_t bytes);
 
 void spmv64(const gb300_matrix *A, const double *x, double *y, cudaStream_t st);
 void spmv_plain(const gb300_matrix *A, const double *val, const double *x,
