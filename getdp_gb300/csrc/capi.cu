@@ -652,20 +652,24 @@ int gb300_matrix_zero(gb300_matrix *A)
   GB_TRY(gb300_matrix_assemble(A));
   cudaStream_t st = A->ctx->stream;
   if(A->nnz > 0) GB_CUDA(cudaMemsetAsync(A->val.p, 0, sizeof(double) * A->nnz, st));
-  // every row gets its diagonal (LinAlg_SPARSKIT.cpp:168-169)
-  DevBuf<int> missing;
-  GB_TRY(missing.alloc(1));
-  GB_CUDA(cudaMemsetAsync(missing.p, 0, sizeof(int), st));
-  int hm = A->n > 0 ? 1 : 0;
-  if(A->csr_valid && A->n > 0) {
-    k_add_diag<<<grid_for(A->n, 256), 256, 0, st>>>(A->n, A->rowptr.p, A->col.p,
-                                                     missing.p);
-    GB_CUDA(cudaMemcpyAsync(&hm, missing.p, sizeof(int), cudaMemcpyDeviceToHost, st));
-    GB_CUDA(cudaStreamSynchronize(st));
-  }
-  if(hm) {
-    for(int i = 0; i < A->n; i++) GB_TRY(gb300_matrix_add_double(A, 0.0, i, i));
-    GB_TRY(gb300_matrix_assemble(A));
+  // every row gets its diagonal (LinAlg_SPARSKIT.cpp:168-169); looked for once
+  // per pattern
+  if(A->n > 0 && !(A->csr_valid && A->diag_version == A->pattern_version)) {
+    DevBuf<int> missing;
+    GB_TRY(missing.alloc(1));
+    GB_CUDA(cudaMemsetAsync(missing.p, 0, sizeof(int), st));
+    int hm = 1;
+    if(A->csr_valid) {
+      k_add_diag<<<grid_for(A->n, 256), 256, 0, st>>>(A->n, A->rowptr.p, A->col.p,
+                                                       missing.p);
+      GB_CUDA(cudaMemcpyAsync(&hm, missing.p, sizeof(int), cudaMemcpyDeviceToHost, st));
+      GB_CUDA(cudaStreamSynchronize(st));
+    }
+    if(hm) {
+      for(int i = 0; i < A->n; i++) GB_TRY(gb300_matrix_add_double(A, 0.0, i, i));
+      GB_TRY(gb300_matrix_assemble(A));
+    }
+    A->diag_version = A->pattern_version;
   }
   A->val32_valid = false;
   gb::coarse_values_changed(A);

@@ -432,6 +432,7 @@ struct gb300_matrix {
   // bumped whenever the pattern is rebuilt; the multicolour ordering of the
   // ILU solves (created on demand) remembers the version it was made for
   unsigned pattern_version = 0;
+  unsigned diag_version = ~0u;  // the pattern known to hold every diagonal entry
   gb::Colouring *mc = nullptr;
   // on a permuted copy: the ordering it is the copy of (owned by the source)
   const gb::Colouring *order = nullptr;
