@@ -639,9 +639,18 @@ k_colour_sweep(int r0, int w, int slice0, const int *__restrict__ width,
 #pragma unroll
   for(int u = 0; u < kSweepU; u++)
     if(c[u] >= 0) acc = acc - (X)v[u] * xv[u];
-  for(int j = kSweepU; j < W; j++) {
-    const int cc = ecol[e + 32LL * j];
-    if(cc >= 0) acc = acc - (X)ev[e + 32LL * j] * gather(cc);
+  for(int j = kSweepU; j < W; j += kSweepU) {  // longer rows, as many at a time
+    e += 32 * kSweepU;
+#pragma unroll
+    for(int u = 0; u < kSweepU; u++) {
+      c[u] = j + u < W ? ecol[e + 32 * u] : -1;
+      v[u] = j + u < W ? ev[e + 32 * u] : (T)0;
+    }
+#pragma unroll
+    for(int u = 0; u < kSweepU; u++) xv[u] = c[u] >= 0 ? gather(c[u]) : (X)0;
+#pragma unroll
+    for(int u = 0; u < kSweepU; u++)
+      if(c[u] >= 0) acc = acc - (X)v[u] * xv[u];
   }
   if(PART != 0) acc = (X)iv * acc;
   x[i] = acc;
@@ -709,14 +718,22 @@ k_ell_chain(int n, const int *__restrict__ width, const long long *__restrict__ 
 #pragma unroll
   for(int u = 0; u < U; u++)
     if(c[u] >= 0) sum += v[u] * xv[u];
-#pragma unroll 4
-  for(int j = U; j < W; j++) {
-    const int cc = ecol[e + 32LL * j];
-    if(cc >= 0) {
-      double x = a.x[cc];
-      if(MODE == kChainProlong) x += a.ec[a.agg[cc]];
-      sum += ev[e + 32LL * j] * x;
+  for(int j = U; j < W; j += U) {
+    e += 32 * U;
+#pragma unroll
+    for(int u = 0; u < U; u++) {
+      c[u] = j + u < W ? ecol[e + 32 * u] : -1;
+      v[u] = j + u < W ? ev[e + 32 * u] : 0.;
+      if(MODE == kChainProlong) g[u] = c[u] >= 0 ? a.agg[c[u]] : 0;
     }
+#pragma unroll
+    for(int u = 0; u < U; u++) {
+      xv[u] = c[u] >= 0 ? a.x[c[u]] : 0.;
+      if(MODE == kChainProlong && c[u] >= 0) xv[u] += a.ec[g[u]];
+    }
+#pragma unroll
+    for(int u = 0; u < U; u++)
+      if(c[u] >= 0) sum += v[u] * xv[u];
   }
   chain_store<MODE>(a, i, grow, sum);
 }
@@ -1470,12 +1487,15 @@ int gmres_solve(gb300_matrix *A, const double *val, const double *rhs,
   int gs = grid_for(n, 256, kReduceBlocks * 4);
   // row shares of the Gram-Schmidt kernels, fixed for a given n and step, so
   // deterministic.  Dots: the groups' CTAs fill the SMs once (see k_gm_dots),
-  // twice from 200,000 rows on, where the loads need more warps.  Update:
-  // whole waves of 152, as many as leave a thread some 6 rows (512 CTAs on
-  // 152 SMs, 4 on some and 3 on others, took 85 us at 1,046,529 rows, k = 25)
+  // twice from 200,000 rows on, where the loads need more warps (304 against
+  // 152 CTAs: 26 / 25 us at 261,121 rows, 39 / 50 at 434,281, k = 33).  Update:
+  // every CTA that is resident at once, as far as there are rows: it reads k
+  // vectors a row, and one CTA per SM leaves too few loads in flight (k = 33,
+  // 152 / 456 / 760 CTAs: 35 / 32 / 31 us at 261,121 rows, 106 / 51 / 44 at
+  // 434,281, 259 / 105 / 84 at 1,046,529; a second wave costs 15 % again)
   const int rows256 = (n + 255) / 256;
   const int nbd = std::min(152 * (n > 200000 ? 2 : 1), rows256 * (m / kDotCols + 1));
-  const int nbu = std::min(rows256, 152 * std::min(8, std::max(1, n / (152 * 256 * 6))));
+  const int nbu = std::min(rows256, resident_grid(k_gm_update, 256, 0));
   const double *no_z = nullptr;
 
   // One graph holds a few Arnoldi steps (they find their place in the cycle
