@@ -615,6 +615,19 @@ k_coarse_gemv(int nc, const double *__restrict__ inv, const double *rc, double *
   if(lane == 0) ec[i] = s;
 }
 
+// out = z + P0 ec
+__global__ void __launch_bounds__(256)
+k_prolong_to(int n, const int *__restrict__ agg, const double *ec, const double *z, double *out,
+             const int *flag)
+{
+  const int i = blockIdx.x * 256 + threadIdx.x;
+  const int g = i < n ? agg[i] : 0;
+  chain_wait();
+  const int go = flag ? *flag : 1;
+  if(i >= n || !go) return;
+  out[i] = z[i] + ec[g];
+}
+
 static void coarse_solve(const Coarse *c, const double *t, int n, const int *flag,
                          cudaStream_t st)
 {
@@ -631,7 +644,16 @@ void coarse_correct(const gb300_matrix *A, const double *val, const double *v,
   const Coarse *c = A->coarse;
   product_chain(kChainRes, A, val, {z, v, t, nullptr, nullptr, nullptr, flag}, st);
   coarse_solve(c, t, A->n, flag, st);
-  product_chain(kChainProlong, A, val, {z, v, t, c->agg.p, c->ec.p, out, flag}, st);
+  // the prolongation inside the residual saves a launch and a pass, but adds
+  // an FP64 addition per matrix entry: 6.0 against 7.2 us at 65,025 rows, 45
+  // against 31 at 1,046,529
+  if(chain_early(A->n)) {
+    product_chain(kChainProlong, A, val, {z, v, t, c->agg.p, c->ec.p, out, flag}, st);
+    return;
+  }
+  launch_chain(false, k_prolong_to, grid_for(A->n, 256), 256, st, A->n, c->agg.p, c->ec.p, z,
+               out, flag);
+  product_chain(kChainRes, A, val, {out, v, t, nullptr, nullptr, nullptr, flag}, st);
 }
 
 // one block: out = rc . ec over the nc coarse entries, in a fixed order

@@ -47,6 +47,11 @@ struct Segment {
 // not yet written would be NaN when that memory happens to hold one)
 struct EllPart {
   std::vector<int> slice0;  // per segment: its first slice (wide segments)
+  // per segment: the common width of its slices and the place of its first
+  // entry, so that a kernel finds a row's entries without reading its slice's
+  // width and offset (0: the widths differ)
+  std::vector<int> common;
+  std::vector<long long> first;
   int nslices = 0;
   long long entries = 0;
   DevBuf<int> width, col, src;
@@ -256,6 +261,8 @@ static int build_ell(gb300_matrix *A, const std::vector<Segment> &seg, const int
       E.nslices += (seg[q].width + 31) / 32;
     }
   E.entries = 0;
+  E.common.assign(seg.size(), 0);
+  E.first.assign(seg.size(), 0);
   if(E.nslices == 0) return GB300_OK;
   GB_TRY(E.width.alloc(E.nslices));
   GB_TRY(E.wscan.alloc(E.nslices));
@@ -265,9 +272,38 @@ static int build_ell(gb300_matrix *A, const std::vector<Segment> &seg, const int
       k_ell_width<UPPER><<<grid_for((long long)nsl * 32, 256), 256, 0, st>>>(
         seg[q].r0, seg[q].width, nsl, E.slice0[q], rows, A->rowptr.p, diag, E.width.p);
     }
+  // slices of a segment padded to its widest where that adds at most a quarter
+  std::vector<int> w(E.nslices);
+  GB_CUDA(cudaMemcpyAsync(w.data(), E.width.p, sizeof(int) * E.nslices, cudaMemcpyDeviceToHost,
+                          st));
+  GB_CUDA(cudaStreamSynchronize(st));
+  long long at = 0;
+  bool padded = false;
+  for(size_t q = 0; q < seg.size(); q++) {
+    if(seg[q].narrow) continue;
+    const int s0 = E.slice0[q], nsl = (seg[q].width + 31) / 32;
+    long long sum = 0;
+    int most = 0;
+    for(int t = s0; t < s0 + nsl; t++) {
+      sum += w[t];
+      most = std::max(most, w[t]);
+    }
+    E.first[q] = 32 * at;
+    if(most > 0 && 4LL * most * nsl <= 5 * sum) {
+      E.common[q] = most;
+      std::fill(w.begin() + s0, w.begin() + s0 + nsl, most);
+      sum = (long long)most * nsl;
+      padded = true;
+    }
+    at += sum;
+  }
+  if(padded)
+    GB_CUDA(cudaMemcpyAsync(E.width.p, w.data(), sizeof(int) * E.nslices,
+                            cudaMemcpyHostToDevice, st));
   DevBuf<long long> tmp;
   long long total = 0;
   GB_TRY(exclusive_scan(E.width.p, E.nslices, E.wscan.p, &total, tmp, st));
+  GB_CUDA(cudaStreamSynchronize(st));  // (total; w goes out of scope)
   E.entries = 32 * total;
   GB_TRY(E.col.alloc(E.entries > 0 ? E.entries : 1));
   GB_TRY(E.src.alloc(E.entries > 0 ? E.entries : 1));
@@ -591,18 +627,19 @@ int ilu_factor(gb300_matrix *A, const double *val, bool fp32, int *zero_row_out,
 // instead of 2 C, and no pass that converts the vector.  A row's first
 // kSweepU entries and its pivot are loaded before the wait for the preceding
 // colour, and the guard is tested once the gathers are on their way: one
-// memory latency and a store remain of each colour.  Both sweeps at 65,025
+// memory latency and a store remain of each colour.  kSweepU is 4 or 6 where all
+// slices of the colour are that narrow (fewer registers, so more of a large
+// colour's rows are in flight at once: 9.0 -> 5.8 us at 262,000 rows), else 8.  Both sweeps at 65,025
 // rows, 4 colours: 15.4 us, 27 with a launch per level and sweep (rows of a
 // level in the order the schedule's atomics left them).  The accumulation
 // order is that of lusol.
 //   PART 0: forward, x = value          PART 1: last colour, both sweeps
 //   PART 2: backward, from x            PART 3: backward, from src (colour 0)
 // OUT 1: final values also to z as doubles; 2: added into z
-constexpr int kSweepU = 8;
-
-template <int PART, int OUT, typename T, typename X>
+template <int PART, int OUT, typename T, typename X, int kSweepU>
 __global__ void __launch_bounds__(256)
-k_colour_sweep(int r0, int w, int slice0, const int *__restrict__ width,
+k_colour_sweep(int r0, int w, int slice0, int common, long long first,
+               const int *__restrict__ width,
                const long long *__restrict__ wscan, const int *__restrict__ ecol,
                const T *__restrict__ ev, const T *__restrict__ inv, int n0, const double *src,
                X *x, double *z, const int *flag)
@@ -614,9 +651,10 @@ k_colour_sweep(int r0, int w, int slice0, const int *__restrict__ width,
   T iv = (T)0, v[kSweepU];
   int c[kSweepU];
   if(t < w) {
-    const int s = slice0 + (t >> 5);
-    W = width[s];
-    e = 32 * wscan[s] + (t & 31);
+    const int s = t >> 5;
+    W = common > 0 ? common : width[slice0 + s];
+    e = common > 0 ? first + 32LL * common * s : 32 * wscan[slice0 + s];
+    e += t & 31;
     if(PART != 0) iv = inv[i];
   }
 #pragma unroll
@@ -663,39 +701,46 @@ static void colour_sweeps(const ilu_data *L, const T *inv, const double *src, X 
                           const int *flag, cudaStream_t st)
 {
   const int C = (int)L->lseg.size();
-  auto go = [&](auto kernel, const EllPart &E, const Segment &g, int slice0) {
-    launch_chain(chain_early(L->n), kernel, grid_for(g.width, 256), 256, st, g.r0, g.width,
-                 slice0, E.width.p, E.wscan.p, E.col.p, ell_vals<T>(E), inv, L->n0, src, x, z,
-                 flag);
+  auto go = [&](auto u4, auto u6, auto u8, const EllPart &E, const std::vector<Segment> &seg,
+                int q) {
+    const Segment &g = seg[q];
+    const int cw = E.common[q];
+    launch_chain(chain_early(L->n), cw > 0 && cw <= 4 ? u4 : cw > 0 && cw <= 6 ? u6 : u8,
+                 grid_for(g.width, 256), 256, st, g.r0, g.width, E.slice0[q], E.common[q],
+                 E.first[q], E.width.p, E.wscan.p, E.col.p, ell_vals<T>(E), inv, L->n0, src, x,
+                 z, flag);
   };
-  for(int c = 1; c < C - 1; c++)
-    go(k_colour_sweep<0, OUT, T, X>, L->lell, L->lseg[c], L->lell.slice0[c]);
-  go(k_colour_sweep<1, OUT, T, X>, L->lell, L->lseg[C - 1], L->lell.slice0[C - 1]);
+#define GB_SWEEP(PART, E, seg, q) \
+  go(k_colour_sweep<PART, OUT, T, X, 4>, k_colour_sweep<PART, OUT, T, X, 6>,      \
+     k_colour_sweep<PART, OUT, T, X, 8>, E, seg, q)
+  for(int c = 1; c < C - 1; c++) GB_SWEEP(0, L->lell, L->lseg, c);
+  GB_SWEEP(1, L->lell, L->lseg, C - 1);
   for(int q = 1; q < C; q++) {  // useg[q] is colour C - 1 - q
     if(q < C - 1)
-      go(k_colour_sweep<2, OUT, T, X>, L->uell, L->useg[q], L->uell.slice0[q]);
+      GB_SWEEP(2, L->uell, L->useg, q);
     else
-      go(k_colour_sweep<3, OUT, T, X>, L->uell, L->useg[q], L->uell.slice0[q]);
+      GB_SWEEP(3, L->uell, L->useg, q);
   }
+#undef GB_SWEEP
 }
 
 // A multicolour copy's products, one thread per row of a sliced-ELL copy of
 // A: GB300's FP64 pipe, not memory, bounds them from ~500,000 rows on (14 us
 // for the 7.3 M FMAs at 1,046,529 rows), and a row shared by two lanes issues
 // 10 FP64 instructions per 32 rows of 7 entries where a thread per row issues 7
-template <int MODE>
+template <int MODE, int U>
 __global__ void __launch_bounds__(256)
-k_ell_chain(int n, const int *__restrict__ width, const long long *__restrict__ wscan,
+k_ell_chain(int n, int common, const int *__restrict__ width,
+            const long long *__restrict__ wscan,
             const int *__restrict__ ecol, const double *__restrict__ ev, ChainArgs a)
 {
-  constexpr int U = 8;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   int W = 0, c[U], g[U], grow = 0;
   long long e = 0;
   double v[U];
   if(i < n) {
-    W = width[i >> 5];
-    e = 32 * wscan[i >> 5] + (i & 31);
+    W = common > 0 ? common : width[i >> 5];
+    e = (common > 0 ? 32LL * common * (i >> 5) : 32 * wscan[i >> 5]) + (i & 31);
     if(MODE == kChainProlong) grow = a.agg[i];
   }
 #pragma unroll
@@ -757,16 +802,17 @@ void product_chain(ChainMode mode, const gb300_matrix *A, const double *val,
     return;
   }
   const EllPart &E = L->aell;
-  auto go = [&](auto kernel) {
-    launch_chain(chain_early(A->n), kernel, grid_for(A->n, 256), 256, st, A->n, E.width.p,
-                 E.wscan.p, E.col.p, E.v64.p, a);
+  auto go = [&](auto u7, auto u8) {  // (7: 2D meshes, fewer registers)
+    launch_chain(chain_early(A->n), E.common[0] == 7 ? u7 : u8, grid_for(A->n, 256), 256, st,
+                 A->n, E.common[0],
+                 E.width.p, E.wscan.p, E.col.p, E.v64.p, a);
   };
   switch(mode) {
-  case kChainMul: go(k_ell_chain<kChainMul>); break;
-  case kChainAdd: go(k_ell_chain<kChainAdd>); break;
-  case kChainRes: go(k_ell_chain<kChainRes>); break;
-  case kChainProlong: go(k_ell_chain<kChainProlong>); break;
-  case kChainAddBoth: go(k_ell_chain<kChainAddBoth>); break;
+  case kChainMul: go(k_ell_chain<kChainMul, 7>, k_ell_chain<kChainMul, 8>); break;
+  case kChainAdd: go(k_ell_chain<kChainAdd, 7>, k_ell_chain<kChainAdd, 8>); break;
+  case kChainRes: go(k_ell_chain<kChainRes, 7>, k_ell_chain<kChainRes, 8>); break;
+  case kChainProlong: go(k_ell_chain<kChainProlong, 7>, k_ell_chain<kChainProlong, 8>); break;
+  case kChainAddBoth: go(k_ell_chain<kChainAddBoth, 7>, k_ell_chain<kChainAddBoth, 8>); break;
   }
 }
 
