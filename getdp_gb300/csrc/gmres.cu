@@ -629,10 +629,9 @@ int ilu_factor(gb300_matrix *A, const double *val, bool fp32, int *zero_row_out,
 // colour, and the guard is tested once the gathers are on their way: one
 // memory latency and a store remain of each colour.  kSweepU is 4 or 6 where all
 // slices of the colour are that narrow (fewer registers, so more of a large
-// colour's rows are in flight at once: 9.0 -> 5.8 us at 262,000 rows), else 8.  Both sweeps at 65,025
-// rows, 4 colours: 15.4 us, 27 with a launch per level and sweep (rows of a
-// level in the order the schedule's atomics left them).  The accumulation
-// order is that of lusol.
+// colour's rows are in flight at once: 9.0 -> 5.8 us at 262,000 rows), else 8.
+// Both sweeps at 1,046,529 rows, 4 colours: 94 us.  The accumulation order is
+// that of lusol.
 //   PART 0: forward, x = value          PART 1: last colour, both sweeps
 //   PART 2: backward, from x            PART 3: backward, from src (colour 0)
 // OUT 1: final values also to z as doubles; 2: added into z
@@ -781,6 +780,132 @@ k_ell_chain(int n, int common, const int *__restrict__ width,
       if(c[u] >= 0) sum += v[u] * xv[u];
   }
   chain_store<MODE>(a, i, grow, sum);
+}
+
+// Small systems: both sweeps and the product in one CTA, a row per thread and
+// x in shared memory.  A launch per colour costs some 2 us whatever its rows
+// (launch, guard, gather, store); a colour here costs a shared gather, a short
+// FMA chain and a barrier, its entries loaded during the colour before: 5.4 us
+// at 529 rows against 9 for the chain.  One SM's FP64 pipe sets the limit.
+// Solve per GMRES step, set-up included, chain / this kernel: 65 / 48 us at 81
+// rows, 38 / 34 at 529, 40 / 36 at 961; with two rows a thread 35.6 / 36.7 at
+// 1,225 and 33 / 36 at 1,521, so the line lies at one.
+constexpr int kSmallRows = 1024, kSmallColours = 12;
+struct SmallStep {
+  int n, C;
+  int r0[kSmallColours + 1];                    // rows of colour c
+  int lslice[kSmallColours], uslice[kSmallColours];
+};
+
+template <typename T, typename X>
+__global__ void __launch_bounds__(kSmallRows)
+k_small_step(SmallStep P, const int *__restrict__ lw, const long long *__restrict__ ls,
+             const int *__restrict__ lc, const T *__restrict__ lv, const int *__restrict__ uw,
+             const long long *__restrict__ us, const int *__restrict__ uc,
+             const T *__restrict__ uv, const T *__restrict__ inv, const int *__restrict__ aw,
+             const long long *__restrict__ as, const int *__restrict__ ac,
+             const double *__restrict__ av, const double *src, double *z, double *y,
+             const int *flag)
+{
+  constexpr int U = 6;
+  __shared__ X x[kSmallRows];
+  int c[U], W = 0;
+  T v[U];
+  long long e = 0;
+  auto load = [&](int slice0, int t, bool in, const int *width, const long long *scan,
+                  const int *col, const T *val) {
+    W = in ? width[slice0 + (t >> 5)] : 0;
+    e = in ? 32 * scan[slice0 + (t >> 5)] + (t & 31) : 0;
+#pragma unroll
+    for(int u = 0; u < U; u++) {
+      c[u] = u < W ? col[e + 32 * u] : -1;
+      v[u] = u < W ? val[e + 32 * u] : (T)0;
+    }
+  };
+  auto apply = [&](X acc, const int *col, const T *val) {
+#pragma unroll
+    for(int u = 0; u < U; u++)
+      if(c[u] >= 0) acc = acc - (X)v[u] * x[c[u]];
+    for(int j = U; j < W; j++) {
+      const int cc = col[e + 32LL * j];
+      if(cc >= 0) acc = acc - (X)val[e + 32LL * j] * x[cc];
+    }
+    return acc;
+  };
+  const int t = threadIdx.x, C = P.C;
+  auto rows = [&](int cc) { return P.r0[cc + 1] - P.r0[cc]; };
+  if(C > 1) load(P.lslice[1], t, t < rows(1), lw, ls, lc, lv);
+  chain_wait();
+  if(flag && !*flag) return;  // the same in every thread
+  if(t < P.n) x[t] = (X)src[t];
+  __syncthreads();
+  for(int cc = 1; cc < C; cc++) {
+    const int i = P.r0[cc] + t;
+    const bool in = t < rows(cc);
+    X s = in ? apply(x[i], lc, lv) : (X)0;
+    if(cc + 1 < C)
+      load(P.lslice[cc + 1], t, t < rows(cc + 1), lw, ls, lc, lv);
+    else {  // no upper entries
+      load(P.uslice[C - 2], t, t < rows(C - 2), uw, us, uc, uv);
+      if(in) s = (X)inv[i] * s;
+    }
+    if(in) x[i] = s;
+    __syncthreads();
+  }
+  if(C == 1) {  // no sweeps: the copy is diagonal
+    if(t < P.n) x[t] = (X)inv[t] * x[t];
+    __syncthreads();
+  }
+  for(int cc = C - 2; cc >= 0; cc--) {
+    const int i = P.r0[cc] + t;
+    if(t < rows(cc)) x[i] = (X)inv[i] * apply(x[i], uc, uv);
+    if(cc > 0) load(P.uslice[cc - 1], t, t < rows(cc - 1), uw, us, uc, uv);
+    __syncthreads();
+  }
+  if(t >= P.n) return;
+  z[t] = (double)x[t];
+  if(!y) return;
+  const int w = aw[t >> 5];
+  const long long b = 32 * as[t >> 5] + (t & 31);
+  double s = 0.;
+#pragma unroll 8
+  for(int j = 0; j < w; j++) {
+    const int cc = ac[b + 32LL * j];
+    if(cc >= 0) s += av[b + 32LL * j] * (double)x[cc];
+  }
+  y[t] = s;
+}
+
+// z = M^-1 v and, with y, y = A z for the plain ILU(0) of a small multicolour
+// copy; false (nothing launched) where that form does not apply
+static bool small_step(const gb300_matrix *A, const double *val, int mode, const double *v,
+                       double *z, double *y, const int *flag, cudaStream_t st)
+{
+  const ilu_data *L = A->ilu;
+  if(!L || !L->by_colour || L->aell_of != val || A->n > kSmallRows ||
+     (int)L->lseg.size() > kSmallColours)
+    return false;
+  SmallStep P = {};
+  P.n = A->n;
+  P.C = (int)L->lseg.size();
+  for(int c = 0; c < P.C; c++) {
+    P.r0[c] = L->lseg[c].r0;
+    P.lslice[c] = L->lell.slice0[c];
+    P.uslice[c] = L->uell.slice0[P.C - 1 - c];  // useg[q] is colour C - 1 - q
+  }
+  P.r0[P.C] = P.n;
+  auto go = [&](auto kernel, const auto *lv, const auto *uv, const auto *inv) {
+    launch_chain(true, kernel, 1, (A->n + 31) / 32 * 32, st, P, L->lell.width.p, L->lell.wscan.p,
+                 L->lell.col.p, lv, L->uell.width.p, L->uell.wscan.p, L->uell.col.p, uv, inv,
+                 L->aell.width.p, L->aell.wscan.p, L->aell.col.p, L->aell.v64.p, v, z, y, flag);
+  };
+  if(mode == 0)
+    go(k_small_step<double, double>, L->lell.v64.p, L->uell.v64.p, L->inv64.p);
+  else if(mode == 2)
+    go(k_small_step<float, double>, L->lell.v32.p, L->uell.v32.p, L->inv32.p);
+  else
+    go(k_small_step<float, float>, L->lell.v32.p, L->uell.v32.p, L->inv32.p);
+  return true;
 }
 
 int ilu_products(gb300_matrix *A, const double *val)
@@ -1555,8 +1680,11 @@ int gmres_solve(gb300_matrix *A, const double *val, const double *rhs,
     k_gm_scale<<<gs, 256, 0, st>>>(n, &S->scale, V, V, cur, &S->cycle);
   };
   auto step = [&]() {
-    precond_run(A, val, p, cur, zt, ps, &S->cycle, st);
-    product_chain(kChainMul, A, val, {zt, nullptr, w, nullptr, nullptr, nullptr, &S->cycle}, st);
+    if(p->preconditioner != 6 || !small_step(A, val, ilu_mode(p), cur, zt, w, &S->cycle, st)) {
+      precond_run(A, val, p, cur, zt, ps, &S->cycle, st);
+      product_chain(kChainMul, A, val, {zt, nullptr, w, nullptr, nullptr, nullptr, &S->cycle},
+                    st);
+    }
     // classical Gram-Schmidt, a second pass only when the test after the
     // first asks for it; the reductions, the test and the end of the step
     // run in the last CTA of each kernel
@@ -1572,7 +1700,8 @@ int gmres_solve(gb300_matrix *A, const double *val, const double *rhs,
     else {
       k_gm_combine<0><<<gs, 256, 0, st>>>(n, V, ldv, u, S);
       k_gm_apply_ok<<<1, 32, 0, st>>>(S, okflag);
-      precond_run(A, val, p, u, zt, ps, okflag, st);
+      if(p->preconditioner != 6 || !small_step(A, val, ilu_mode(p), u, zt, nullptr, okflag, st))
+        precond_run(A, val, p, u, zt, ps, okflag, st);
       k_gm_addto<<<gs, 256, 0, st>>>(n, zt, x, S);
     }
     k_gm_after<<<1, 32, 0, st>>>(S);

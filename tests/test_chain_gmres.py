@@ -115,3 +115,20 @@ def test_both_sides_of_the_early_start(side):
     # 2-norm: ||A^-1||_2 <= 2 sqrt(n) would be far from sharp; the residual
     # bound and the condition number of a dominant matrix (<= 3) give
     assert np.linalg.norm(x.numpy() - x0) <= 10 * 3 * 1e-10 * np.linalg.norm(x0)
+
+
+@pytest.mark.parametrize("precision", [0, 1, 2])
+@pytest.mark.parametrize("name", ["path32", "path33", "path1024", "path1025", "grid1024",
+                                  "clique11", "clique12", "clique13"])
+def test_small_step(name, precision):
+    """Both sides of the one-CTA step's limits: 1,024 rows, twelve colours."""
+    size = int(name.lstrip("pathgridclque"))
+    if name.startswith("path"):
+        A = sp.diags([np.ones(size - 1)], [1])
+    elif name.startswith("grid"):
+        A = _grid(32, True)
+    else:
+        A = sp.kron(sp.identity(40), np.ones((size, size))) + \
+            sp.kron(sp.diags([np.ones(39)], [1]), np.eye(size))
+    # (an FP32 result of M^-1 is 1e-7 off when x is formed: FGMRES only)
+    _solve(_dominant(A, size), {"Precision": precision, "Algorithm": 9 if precision == 1 else 8})
