@@ -109,7 +109,7 @@ int coarse_set(gb300_matrix *A, const int *agg, int nc)
   GB_TRY(c->aperm.alloc(n));
   GB_TRY(c->aptr.alloc(nc + 1));
   GB_TRY(c->inv.alloc((size_t)nc * nc));
-  GB_TRY(c->panel.alloc((2 * (size_t)nc + kSwB) * kSwB));
+  GB_TRY(c->panel.alloc(2 * ((size_t)nc + kSwB) * kSwB));
   GB_TRY(c->rc.alloc(nc));
   GB_TRY(c->ec.alloc(nc));
   GB_TRY(c->err.alloc(1));
@@ -245,7 +245,7 @@ int coarse_follow(const gb300_matrix *A, gb300_matrix *B, const Colouring *C,
   GB_TRY(c->aperm.alloc(n));
   GB_TRY(c->aptr.alloc(nc + 1));
   GB_TRY(c->inv.alloc((size_t)nc * nc));
-  GB_TRY(c->panel.alloc((2 * (size_t)nc + kSwB) * kSwB));
+  GB_TRY(c->panel.alloc(2 * ((size_t)nc + kSwB) * kSwB));
   GB_TRY(c->rc.alloc(nc));
   GB_TRY(c->ec.alloc(nc));
   GB_TRY(c->err.alloc(1));
@@ -338,32 +338,81 @@ __global__ void k_coarse_to_double(long long m, int headroom,
 // per launch read and wrote all nc^2 entries 1,024 times (8 GB each way
 // through L2 and 1,024 launches, 14.6 ms).  32 columns: narrower blocks
 // re-read the triangle more often, wider ones lengthen the serial inversion
-// of D.  No pivoting: the pivots met inside the blocks are those of the
-// unblocked elimination, and one that is not positive is reported.
-constexpr int kSwRows = 16;  // panel rows per CTA
+// of D (32 pivots, each a division and an FMA deep: 27 us).  That inversion
+// runs beside the update of the block before, in a CTA that computes its tile
+// first: 45 us a block (panel 5, update 40) and 1.5 ms in all at nc = 1024,
+// against 80 us and 2.4 ms with D inverted by every CTA of the panel.  No
+// pivoting: the pivots met inside the blocks are those of the unblocked
+// elimination, and one that is not positive is reported.
+constexpr int kSwRows = 8;  // panel rows per CTA
 
-// W(i) = P(i) D^-1 for this CTA's kSwRows rows; P, W: nc x kSwB; the first
-// CTA also writes D^-1.  Every CTA inverts D itself (in shared memory, one
-// barrier per pivot): cheaper than a launch of its own.
+// D^-1 by Gauss-Jordan steps, one barrier per pivot, for a block of 256
+// threads with D in buf[0] (complete in every thread's sight, padded with the
+// identity); thread t has entries (t / 8, t % 8 * 4 + 0..3).  False (in every
+// thread) where a pivot is not positive and finite.
+__device__ bool sweep_invert(double (*buf)[kSwB][kSwB + 1], double *rp, int k0, double *dinv,
+                             int *err)
+{
+  const int t = threadIdx.x, i = t >> 3, j0 = (t & 7) * 4;
+  if(t == 0) rp[0] = 1. / buf[0][0][0];
+  __syncthreads();
+  for(int k = 0; k < kSwB; k++) {
+    const int cur = k & 1, nxt = cur ^ 1;
+    const double piv = buf[cur][k][k];
+    if(!(piv > 0.) || !(piv <= 1.7976931348623157e308)) {  // the same in every thread
+      if(t == 0) atomicCAS(err, 0, k0 + k + 1);
+      return false;
+    }
+    // one FMA per entry (FP64 instructions, not memory, pace the pivots):
+    // row k is 0 + p R, column k is 0 + m 1, the rest D + m R
+    const double p = rp[cur], m = i == k ? p : -buf[cur][i][k] * p;
+#pragma unroll
+    for(int u = 0; u < 4; u++) {
+      const int j = j0 + u;
+      const double r = j == k ? 1. : buf[cur][k][j];
+      const double v = fma(m, r, (i == k || j == k) ? 0. : buf[cur][i][j]);
+      buf[nxt][i][j] = v;
+      if(i == k + 1 && j == k + 1) rp[nxt] = 1. / v;
+    }
+    __syncthreads();
+  }
+  static_assert(kSwB % 2 == 0, "the result is in buf[0]");
+#pragma unroll
+  for(int u = 0; u < 4; u++) dinv[i * kSwB + j0 + u] = buf[0][i][j0 + u];
+  return true;
+}
+
+// D^-1 of the first block
 __global__ void __launch_bounds__(256)
-k_sweep_panel(int nc, int k0, const double *__restrict__ a, double *__restrict__ P,
-              double *__restrict__ W, double *__restrict__ dinv, int *err)
+k_sweep_first(int nc, const double *__restrict__ a, double *__restrict__ dinv, int *err)
 {
   if(*err) return;
-  __shared__ double D[2][kSwB][kSwB + 1];
-  __shared__ double sp[kSwRows][kSwB + 1];
-  __shared__ double rp[2];
-  const int t = threadIdx.x;
-  const int bw = nc - k0 < kSwB ? nc - k0 : kSwB;
-  const int i = t >> 3, j0 = (t & 7) * 4;
+  __shared__ double D[2][kSwB][kSwB + 1], rp[2];
+  const int t = threadIdx.x, i = t >> 3, j0 = (t & 7) * 4;
 #pragma unroll
   for(int u = 0; u < 4; u++) {
     const int j = j0 + u;
     const int hi = i > j ? i : j, lo = i > j ? j : i;
-    D[0][i][j] = hi < bw ? a[(size_t)(k0 + hi) * nc + k0 + lo] : (i == j ? 1. : 0.);
+    D[0][i][j] = hi < nc ? a[(size_t)hi * nc + lo] : (i == j ? 1. : 0.);
   }
+  __syncthreads();
+  sweep_invert(D, rp, 0, dinv, err);
+}
+
+// W(i) = P(i) D^-1 for this CTA's kSwRows rows; P, W: nc x kSwB
+__global__ void __launch_bounds__(128)
+k_sweep_panel(int nc, int k0, const double *__restrict__ a, double *__restrict__ P,
+              double *__restrict__ W, const double *__restrict__ dinv, const int *err)
+{
+  if(*err) return;
+  __shared__ double D[kSwB][kSwB], sp[kSwRows][kSwB + 1];
+  const int t = threadIdx.x;
+  const int bw = nc - k0 < kSwB ? nc - k0 : kSwB;
   const int r0 = blockIdx.x * kSwRows;
-  for(int q = t; q < kSwRows * kSwB; q += 256) {
+#pragma unroll
+  for(int q = t; q < kSwB * kSwB; q += 128) D[q / kSwB][q % kSwB] = dinv[q];
+#pragma unroll
+  for(int q = t; q < kSwRows * kSwB; q += 128) {
     // the panel's rows below K by row, those above K (stored transposed) by
     // column, so that both read runs of the lower triangle
     int r, c;
@@ -382,63 +431,85 @@ k_sweep_panel(int nc, int k0, const double *__restrict__ a, double *__restrict__
     sp[r][c] = v;
   }
   __syncthreads();
-  if(t == 0) rp[0] = 1. / D[0][0][0];
-  __syncthreads();
+  const int r = t >> 4, c = (t & 15) * 2;
+  double w0 = 0., w1 = 0.;
+#pragma unroll 8
   for(int k = 0; k < kSwB; k++) {
-    const int cur = k & 1, nxt = cur ^ 1;
-    const double piv = D[cur][k][k];
-    if(!(piv > 0.) || !(piv <= 1.7976931348623157e308)) {  // the same in every thread
-      if(blockIdx.x == 0 && t == 0) atomicCAS(err, 0, k0 + k + 1);
-      return;
+    w0 = fma(sp[r][k], D[k][c], w0);
+    w1 = fma(sp[r][k], D[k][c + 1], w1);
+  }
+  if(r0 + r < nc) {
+    const size_t o = (size_t)(r0 + r) * kSwB + c;
+    P[o] = sp[r][c];
+    P[o + 1] = sp[r][c + 1];
+    W[o] = w0;
+    W[o + 1] = w1;
+  }
+}
+
+// The lower triangle's 32 x 32 tiles after the sweep of block kb, four to a
+// CTA (64 threads each); CTA 0 has tile (kb + 1, kb + 1) alone and inverts it
+// for the next block.  Four tiles a CTA, not one: at nc = 1024 the 133 CTAs
+// then lie on an SM each, and the inversion shares its FP64 pipe with none.
+constexpr int kSwTiles = 4;
+constexpr size_t kSwShared = sizeof(double) * kSwTiles * 2 * kSwB * (kSwB + 1);
+
+__global__ void __launch_bounds__(64 * kSwTiles)
+k_sweep_update(int nc, int nb, int kb, double *__restrict__ a, const double *__restrict__ P,
+               const double *__restrict__ W, const double *__restrict__ dinv,
+               double *__restrict__ dnext, int *err)
+{
+  if(*err) return;
+  extern __shared__ double shared[];
+  double (*buf)[kSwB][kSwB + 1] = reinterpret_cast<double (*)[kSwB][kSwB + 1]>(shared);
+  __shared__ double rp[2];
+  const int g = threadIdx.x >> 6, t = threadIdx.x & 63;
+  const int nk = kb + 1;
+  if(blockIdx.x == 0) {
+    if(nk >= nb) return;
+    const int k0 = nk * kSwB;
+    for(int q = threadIdx.x; q < kSwB * kSwB; q += 256) {
+      const int r = q / kSwB, c = q % kSwB;
+      buf[0][c][r] = k0 + r < nc ? W[(size_t)(k0 + r) * kSwB + c] : 0.;
+      buf[1][c][r] = k0 + r < nc ? P[(size_t)(k0 + r) * kSwB + c] : 0.;
     }
-    // one FMA per entry (FP64 instructions, not memory, pace the pivots):
-    // row k is 0 + p R, column k is 0 + m 1, the rest D + m R
-    const double p = rp[cur], m = i == k ? p : -D[cur][i][k] * p;
+    __syncthreads();
+    const int i = threadIdx.x >> 3, j0 = (threadIdx.x & 7) * 4;
+    double acc[4];
+#pragma unroll
+    for(int u = 0; u < 4; u++)
+      acc[u] = k0 + i < nc && k0 + j0 + u < nc ? a[(size_t)(k0 + i) * nc + k0 + j0 + u] : 0.;
+#pragma unroll 8
+    for(int k = 0; k < kSwB; k++)
+#pragma unroll
+      for(int u = 0; u < 4; u++)
+        acc[u] = fma(-buf[0][k][i], buf[1][k][j0 + u], acc[u]);
 #pragma unroll
     for(int u = 0; u < 4; u++) {
       const int j = j0 + u;
-      const double r = j == k ? 1. : D[cur][k][j];
-      const double v = fma(m, r, (i == k || j == k) ? 0. : D[cur][i][j]);
-      D[nxt][i][j] = v;
-      if(i == k + 1 && j == k + 1) rp[nxt] = 1. / v;
+      const bool in = k0 + i < nc && k0 + j < nc;
+      if(in) a[(size_t)(k0 + i) * nc + k0 + j] = acc[u];
+      if(j <= i) {  // (the inversion takes the lower triangle for both)
+        const double v = in ? acc[u] : (i == j ? 1. : 0.);
+        buf[2][i][j] = v;
+        buf[2][j][i] = v;
+      }
     }
     __syncthreads();
+    sweep_invert(buf + 2, rp, k0, dnext, err);
+    return;
   }
-  static_assert(kSwB % 2 == 0, "the result is in D[0]");
-  {
-    const int r = t >> 4, c = (t & 15) * 2;
-    double w0 = 0., w1 = 0.;
-#pragma unroll 8
-    for(int k = 0; k < kSwB; k++) {
-      w0 = fma(sp[r][k], D[0][k][c], w0);
-      w1 = fma(sp[r][k], D[0][k][c + 1], w1);
-    }
-    if(r0 + r < nc) {
-      const size_t o = (size_t)(r0 + r) * kSwB + c;
-      P[o] = sp[r][c];
-      P[o + 1] = sp[r][c + 1];
-      W[o] = w0;
-      W[o + 1] = w1;
-    }
-  }
-  if(blockIdx.x == 0)
-#pragma unroll
-    for(int u = 0; u < 4; u++) dinv[i * kSwB + j0 + u] = D[0][i][j0 + u];
-}
-
-// the lower triangle's 32 x 32 tile (ti, tj) after the sweep of block K
-__global__ void __launch_bounds__(64)
-k_sweep_update(int nc, int kb, double *__restrict__ a, const double *__restrict__ P,
-               const double *__restrict__ W, const double *__restrict__ dinv, const int *err)
-{
-  if(*err) return;
   // tile number -> (ti, tj), tj <= ti
-  int ti = (int)((sqrtf(8.f * (float)blockIdx.x + 1.f) - 1.f) * 0.5f);
-  while((long long)(ti + 1) * (ti + 2) / 2 <= (long long)blockIdx.x) ti++;
-  while((long long)ti * (ti + 1) / 2 > (long long)blockIdx.x) ti--;
-  const int tj = (int)((long long)blockIdx.x - (long long)ti * (ti + 1) / 2);
-  const int t = threadIdx.x, i0 = ti * kSwB, j0 = tj * kSwB;
-  if(ti == kb || tj == kb) {
+  const long long tile = (long long)(blockIdx.x - 1) * kSwTiles + g;
+  int ti = (int)((sqrtf(8.f * (float)tile + 1.f) - 1.f) * 0.5f);
+  while((long long)(ti + 1) * (ti + 2) / 2 <= tile) ti++;
+  while((long long)ti * (ti + 1) / 2 > tile) ti--;
+  const int tj = (int)(tile - (long long)ti * (ti + 1) / 2);
+  const int i0 = ti * kSwB, j0 = tj * kSwB;
+  const bool there = ti < nb && !(ti == nk && tj == nk);
+  const bool inside = there && ti != kb && tj != kb;
+  double (*sw)[kSwB + 1] = buf[2 * g], (*spt)[kSwB + 1] = buf[2 * g + 1];  // [k][row]
+  if(there && !inside)
     for(int q = t; q < kSwB * kSwB; q += 64) {
       const int r = q / kSwB, c = q % kSwB;
       if(i0 + r >= nc || j0 + c >= nc) continue;
@@ -451,26 +522,26 @@ k_sweep_update(int nc, int kb, double *__restrict__ a, const double *__restrict_
         v = W[(size_t)(j0 + c) * kSwB + r];
       a[(size_t)(i0 + r) * nc + j0 + c] = v;
     }
-    return;
-  }
-  __shared__ double sw[kSwB][kSwB + 1], spt[kSwB][kSwB + 1];  // [k][row]
-  for(int q = t; q < kSwB * kSwB; q += 64) {
-    const int r = q / kSwB, c = q % kSwB;
-    sw[c][r] = i0 + r < nc ? W[(size_t)(i0 + r) * kSwB + c] : 0.;
-    spt[c][r] = j0 + r < nc ? P[(size_t)(j0 + r) * kSwB + c] : 0.;
-  }
   // 4 x 4 entries per thread, rows and columns 8 apart (no bank conflicts,
   // coalesced columns)
   const int ty = t >> 3, tx = t & 7;
   double acc[4][4];
-#pragma unroll
-  for(int u = 0; u < 4; u++)
-#pragma unroll
-    for(int v = 0; v < 4; v++) {
-      const int r = i0 + ty + 8 * u, c = j0 + tx + 8 * v;
-      acc[u][v] = (r < nc && c < nc) ? a[(size_t)r * nc + c] : 0.;
+  if(inside) {
+    for(int q = t; q < kSwB * kSwB; q += 64) {
+      const int r = q / kSwB, c = q % kSwB;
+      sw[c][r] = i0 + r < nc ? W[(size_t)(i0 + r) * kSwB + c] : 0.;
+      spt[c][r] = j0 + r < nc ? P[(size_t)(j0 + r) * kSwB + c] : 0.;
     }
+#pragma unroll
+    for(int u = 0; u < 4; u++)
+#pragma unroll
+      for(int v = 0; v < 4; v++) {
+        const int r = i0 + ty + 8 * u, c = j0 + tx + 8 * v;
+        acc[u][v] = (r < nc && c < nc) ? a[(size_t)r * nc + c] : 0.;
+      }
+  }
   __syncthreads();
+  if(!inside) return;
 #pragma unroll 4
   for(int k = 0; k < kSwB; k++) {
     double wr[4], pc[4];
@@ -537,11 +608,18 @@ int coarse_setup(gb300_matrix *A, const double *val, bool reuse)
                                                                       c->inv.p);
   GB_CUDA(cudaGetLastError());
   const int nb = (nc + kSwB - 1) / kSwB;
+  const int tiles = nb * (nb + 1) / 2;
   double *P = c->panel.p, *Wp = P + (size_t)nc * kSwB, *dinv = Wp + (size_t)nc * kSwB;
+  GB_CUDA(cudaFuncSetAttribute(k_sweep_update, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)kSwShared));
+  k_sweep_first<<<1, 256, 0, st>>>(nc, c->inv.p, dinv, c->err.p);
   for(int k = 0; k < nb; k++) {
-    k_sweep_panel<<<grid_for(nc, kSwRows), 256, 0, st>>>(nc, k * kSwB, c->inv.p, P, Wp, dinv,
+    double *dnext = dinv + (k & 1 ? -1 : 1) * kSwB * kSwB;  // two, in turn
+    k_sweep_panel<<<grid_for(nc, kSwRows), 128, 0, st>>>(nc, k * kSwB, c->inv.p, P, Wp, dinv,
                                                          c->err.p);
-    k_sweep_update<<<nb * (nb + 1) / 2, 64, 0, st>>>(nc, k, c->inv.p, P, Wp, dinv, c->err.p);
+    k_sweep_update<<<1 + (tiles + kSwTiles - 1) / kSwTiles, 64 * kSwTiles, kSwShared, st>>>(
+        nc, nb, k, c->inv.p, P, Wp, dinv, dnext, c->err.p);
+    dinv = dnext;
   }
   k_sweep_finish<<<dim3(nb, nb), 256, 0, st>>>(nc, c->inv.p, c->err.p);
   GB_CUDA(cudaGetLastError());
