@@ -144,9 +144,10 @@ void from_nodes64(int nn, const double *in, double *out, cudaStream_t st)
   k_from_nodes<double, double><<<grid_for(nn, 256), 256, 0, st>>>(nn, in, out);
 }
 
+// (p is written within the chain of a CG step: plain loads)
 template <typename T> struct Vec4;
 template <> struct Vec4<float> {
-  __device__ static float4 load(const float *p) { return __ldg((const float4 *)p); }
+  __device__ static float4 load(const float *p) { return *(const float4 *)p; }
 };
 struct D4 {
   double x, y, z, w;
@@ -154,10 +155,70 @@ struct D4 {
 template <> struct Vec4<double> {
   __device__ static D4 load(const double *p)
   {
-    double2 a = __ldg((const double2 *)p), b = __ldg((const double2 *)(p + 2));
+    double2 a = *(const double2 *)p, b = *(const double2 *)(p + 2);
     return D4{a.x, a.y, b.x, b.y};
   }
 };
+
+// A block row's three sums over its LPR lanes: the first step leaves a lane
+// two of the six half sums to add instead of three, every later one a single
+// value (LPR 16: 5 additions and shuffles per lane instead of 12, which on
+// GB300's FP64 pipe took as long as a third of the product's FMAs at 26
+// blocks a row).  The pairs added are those of the plain tree, so the sums
+// are the same to the last bit.  FP64 CG per iteration 49.1 -> 46.1 us at
+// 124,950 unknowns, 605 -> 562 at 2,709,792.  The result: component c in the lane for
+// which bsr_component gives c (LPR 2: y0 and y1 both in lane 0, y1 in b).
+template <int LPR> __device__ __forceinline__ int bsr_component(int lane)
+{
+  return lane == 0 ? 0 : lane == LPR / 2 ? 2 : (LPR > 2 && lane == LPR / 4) ? 1 :
+         (LPR > 2 && lane == LPR / 2 + LPR / 4) ? 3 : -1;
+}
+
+template <typename T, int LPR>
+__device__ __forceinline__ T bsr_row_sum(int lane, T y0, T y1, T y2, T &b)
+{
+  constexpr unsigned all = 0xffffffffu;
+  const bool high = lane & (LPR / 2);
+  T a = (high ? y2 : y0) + __shfl_xor_sync(all, high ? y0 : y2, LPR / 2);
+  b = y1 + __shfl_xor_sync(all, y1, LPR / 2);
+  if constexpr(LPR > 2) {
+    const bool second = !high && (lane & (LPR / 4));  // takes y1
+    const T give = high || second ? a : b;
+    a = (second ? b : a) + __shfl_xor_sync(all, give, LPR / 4);
+#pragma unroll
+    for(int o = LPR / 8; o > 0; o >>= 1) a += __shfl_xor_sync(all, a, o);
+  }
+  return a;
+}
+
+// the row's result into y (MODE 1: bvec less the product), and what it adds
+// to the dot product (MODE 2: <p, y>, MODE 1: <y, y>)
+template <int MODE, typename T, int LPR, typename R>
+__device__ __forceinline__ void bsr_finish(int lane, bool in, size_t a, T y0, T y1, T y2,
+                                           const T *p, const T *bvec, T *y, R &red)
+{
+  T second;
+  const T mine = bsr_row_sum<T, LPR>(lane, y0, y1, y2, second);
+  const int c = bsr_component<LPR>(lane);
+  if(!in || c < 0) return;
+  auto put = [&](int q, T v) {
+    const size_t o = 4 * a + q;
+    if(MODE == 1) v = bvec[o] - v;
+    y[o] = v;
+    if(MODE == 1) red += (R)v * v;
+    if(MODE == 2) red += (R)p[o] * v;
+  };
+  if(c < 3)
+    put(c, mine);
+  else
+    y[4 * a + 3] = 0;
+  if(LPR == 2) {
+    if(c == 0)
+      put(1, second);
+    else
+      y[4 * a + 3] = 0;
+  }
+}
 
 // y = A p over block rows, LPR lanes per block row (LPR consecutive blocks
 // of a row are one 32-byte sector per value plane); MODE 2: partial
@@ -213,21 +274,30 @@ __device__ __forceinline__ void bsr_block(const int *__restrict__ col,
 template <int MODE, typename T, int LPR, int UNR, int CS, int MINB = 0>
 __global__ void __launch_bounds__(256, MINB)
 k_bsr_spmv(int nn, const int *__restrict__ ptr, const int *__restrict__ col,
-           const T *__restrict__ val, long long nblk, const T *__restrict__ p,
+           const T *__restrict__ val, long long nblk, const T *p,
            const T *__restrict__ bvec, T *__restrict__ y,
            double *__restrict__ part, const int *flag, double *dot_out,
            unsigned *counter)
 {
-  if(flag && !*flag) return;
   const int rows_per_block = 256 / LPR;
   int lane = threadIdx.x % LPR, sub = threadIdx.x / LPR;
   typename Acc<T>::type red = 0;
-  for(long long a0 = (long long)blockIdx.x * rows_per_block; a0 < nn;
-      a0 += (long long)gridDim.x * rows_per_block) {
+  const long long first = (long long)blockIdx.x * rows_per_block;
+  int s = 0, e = 0;
+  if(first + sub < nn) {
+    s = ptr[first + sub];
+    e = ptr[first + sub + 1];
+  }
+  chain_wait();
+  if(flag && !*flag) return;
+  for(long long a0 = first; a0 < nn; a0 += (long long)gridDim.x * rows_per_block) {
     long long a = a0 + sub;
     T y0 = 0, y1 = 0, y2 = 0;
     if(a < nn) {
-      int s = ptr[a], e = ptr[a + 1];
+      if(a0 != first) {
+        s = ptr[a];
+        e = ptr[a + 1];
+      }
       int k = s + lane;
       for(; k + (UNR - 1) * LPR < e; k += UNR * LPR) {  // UNR blocks in flight
 #pragma unroll
@@ -236,31 +306,7 @@ k_bsr_spmv(int nn, const int *__restrict__ ptr, const int *__restrict__ col,
       }
       for(; k < e; k += LPR) bsr_block<T, CS>(col, val, nblk, p, k, y0, y1, y2);
     }
-#pragma unroll
-    for(int o = LPR / 2; o > 0; o >>= 1) {
-      y0 += __shfl_down_sync(0xffffffffu, y0, o, LPR);
-      y1 += __shfl_down_sync(0xffffffffu, y1, o, LPR);
-      y2 += __shfl_down_sync(0xffffffffu, y2, o, LPR);
-    }
-    if(lane == 0 && a < nn) {
-      size_t o = 4 * (size_t)a;
-      if(MODE == 1) {
-        T r0 = bvec[o] - y0, r1 = bvec[o + 1] - y1, r2 = bvec[o + 2] - y2;
-        y[o] = r0;
-        y[o + 1] = r1;
-        y[o + 2] = r2;
-        y[o + 3] = 0;
-        red += r0 * r0 + r1 * r1 + r2 * r2;
-      }
-      else {
-        y[o] = y0;
-        y[o + 1] = y1;
-        y[o + 2] = y2;
-        y[o + 3] = 0;
-        if(MODE == 2)
-          red += p[o] * y0 + p[o + 1] * y1 + p[o + 2] * y2;
-      }
-    }
+    bsr_finish<MODE, T, LPR>(lane, a < nn, a, y0, y1, y2, p, bvec, y, red);
   }
   if(MODE != 0) {
     double s = block_sum<double, 256>((double)red);
@@ -287,12 +333,11 @@ k_bsr_spmv(int nn, const int *__restrict__ ptr, const int *__restrict__ col,
 template <int MODE, typename T, int LPR, int UNR, int MINB = 0>
 __global__ void __launch_bounds__(256, MINB)
 k_bsr_spmv_pf(int nn, const int *__restrict__ ptr, const int *__restrict__ col,
-              const T *__restrict__ val, long long nblk, const T *__restrict__ p,
+              const T *__restrict__ val, long long nblk, const T *p,
               const T *__restrict__ bvec, T *__restrict__ y,
               double *__restrict__ part, const int *flag, double *dot_out,
               unsigned *counter)
 {
-  if(flag && !*flag) return;
   const int rows_per_block = 256 / LPR;
   const long long stride = (long long)gridDim.x * rows_per_block;
   int lane = threadIdx.x % LPR, sub = threadIdx.x / LPR;
@@ -303,6 +348,8 @@ k_bsr_spmv_pf(int nn, const int *__restrict__ ptr, const int *__restrict__ col,
     s = __ldg(ptr + a0 + sub);
     e = __ldg(ptr + a0 + sub + 1);
   }
+  chain_wait();
+  if(flag && !*flag) return;
   for(; a0 < nn; a0 += stride) {
     long long a = a0 + sub;
     // the next row's bounds
@@ -359,30 +406,7 @@ k_bsr_spmv_pf(int nn, const int *__restrict__ ptr, const int *__restrict__ col,
     }
     s = sn;
     e = en;
-#pragma unroll
-    for(int o = LPR / 2; o > 0; o >>= 1) {
-      y0 += __shfl_down_sync(0xffffffffu, y0, o, LPR);
-      y1 += __shfl_down_sync(0xffffffffu, y1, o, LPR);
-      y2 += __shfl_down_sync(0xffffffffu, y2, o, LPR);
-    }
-    if(lane == 0 && a < nn) {
-      size_t o = 4 * (size_t)a;
-      if(MODE == 1) {
-        T r0 = bvec[o] - y0, r1 = bvec[o + 1] - y1, r2 = bvec[o + 2] - y2;
-        y[o] = r0;
-        y[o + 1] = r1;
-        y[o + 2] = r2;
-        y[o + 3] = 0;
-        red += r0 * r0 + r1 * r1 + r2 * r2;
-      }
-      else {
-        y[o] = y0;
-        y[o + 1] = y1;
-        y[o + 2] = y2;
-        y[o + 3] = 0;
-        if(MODE == 2) red += p[o] * y0 + p[o + 1] * y1 + p[o + 2] * y2;
-      }
-    }
+    bsr_finish<MODE, T, LPR>(lane, a < nn, a, y0, y1, y2, p, bvec, y, red);
   }
   if(MODE != 0) {
     double sm = block_sum<double, 256>((double)red);
@@ -475,10 +499,11 @@ template <int MODE, typename T, int LPR>
 __global__ void __launch_bounds__(kTmaThreads)
 k_bsr_spmv_tma(int nn, const int *__restrict__ ptr, const int *__restrict__ col,
                const T *__restrict__ val, long long pstride,
-               const T *__restrict__ p, const T *__restrict__ bvec,
+               const T *p, const T *__restrict__ bvec,
                T *__restrict__ y, double *__restrict__ part, const int *flag,
                int *__restrict__ err, double *dot_out, unsigned *counter)
 {
+  chain_wait();
   if(flag && !*flag) return;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   TmaTile<T> *stage = (TmaTile<T> *)smem_raw;
@@ -576,31 +601,7 @@ k_bsr_spmv_tma(int nn, const int *__restrict__ ptr, const int *__restrict__ col,
           y2 = fma(v[8], xb.z, y2);
         }
       }
-#pragma unroll
-      for(int o = LPR / 2; o > 0; o >>= 1) {
-        y0 += __shfl_down_sync(0xffffffffu, y0, o, LPR);
-        y1 += __shfl_down_sync(0xffffffffu, y1, o, LPR);
-        y2 += __shfl_down_sync(0xffffffffu, y2, o, LPR);
-      }
-      if(lane == 0 && a < r1) {
-        size_t o = 4 * (size_t)a;
-        if(MODE == 1) {
-          T q0 = bvec[o] - y0, q1 = bvec[o + 1] - y1, q2 = bvec[o + 2] - y2;
-          y[o] = q0;
-          y[o + 1] = q1;
-          y[o + 2] = q2;
-          y[o + 3] = 0;
-          red += (double)q0 * q0 + (double)q1 * q1 + (double)q2 * q2;
-        }
-        else {
-          y[o] = y0;
-          y[o + 1] = y1;
-          y[o + 2] = y2;
-          y[o + 3] = 0;
-          if(MODE == 2)
-            red += (double)p[o] * y0 + (double)p[o + 1] * y1 + (double)p[o + 2] * y2;
-        }
-      }
+      bsr_finish<MODE, T, LPR>(lane, a < r1, a, y0, y1, y2, p, bvec, y, red);
     }
     __syncthreads();  // every thread is done with stage s
     if(tid == 0 && t + 2 * (int)gridDim.x < ntiles) issue(t + 2 * gridDim.x, s);
@@ -662,36 +663,38 @@ static void launch_tma(const Bsr3 &B, const T *val, const T *p, const T *b,
 template <int MODE, typename T, int L, int U, int C, int M>
 static void launch_plain(const Bsr3 &B, const T *val, const T *p, const T *b,
                          T *y, double *part, const int *flag, double *dot_out,
-                         unsigned *counter, cudaStream_t st)
+                         unsigned *counter, cudaStream_t st, bool early)
 {
   static int grid = 0;  // per instantiation
   if(!grid) grid = resident_grid(k_bsr_spmv<MODE, T, L, U, C, M>, 256, 0);
   // (no CTA without rows: each would still arrive at the sum's counter)
   const int g = grid_for(B.nn, 256 / L, grid);
-  k_bsr_spmv<MODE, T, L, U, C, M><<<g, 256, 0, st>>>(
-    B.nn, B.ptr.p, B.col.p, val, B.pstride, p, b, y, part, flag, dot_out, counter);
+  launch_chain(early, k_bsr_spmv<MODE, T, L, U, C, M>, g, 256, st, B.nn, B.ptr.p, B.col.p, val,
+               B.pstride, p, b, y, part, flag, dot_out, counter);
 }
 
 template <int MODE, typename T, int L, int U, int M>
 static void launch_pf(const Bsr3 &B, const T *val, const T *p, const T *b, T *y,
                       double *part, const int *flag, double *dot_out, unsigned *counter,
-                      cudaStream_t st)
+                      cudaStream_t st, bool early)
 {
   static int grid = 0;  // per instantiation
   if(!grid) grid = resident_grid(k_bsr_spmv_pf<MODE, T, L, U, M>, 256, 0);
   const int g = grid_for(B.nn, 256 / L, grid);
-  k_bsr_spmv_pf<MODE, T, L, U, M><<<g, 256, 0, st>>>(
-    B.nn, B.ptr.p, B.col.p, val, B.pstride, p, b, y, part, flag, dot_out, counter);
+  launch_chain(early, k_bsr_spmv_pf<MODE, T, L, U, M>, g, 256, st, B.nn, B.ptr.p, B.col.p, val,
+               B.pstride, p, b, y, part, flag, dot_out, counter);
 }
 
 template <int MODE, typename T>
 static void launch_bsr(int variant, const Bsr3 &B, const T *val, const T *p,
                        const T *b, T *y, double *part, const int *flag,
                        cudaStream_t st, double *dot_out = nullptr,
-                       unsigned *counter = nullptr)
+                       unsigned *counter = nullptr, bool early = false)
 {
 #define GB_BSR(L, U, C, M) \
-  launch_plain<MODE, T, L, U, C, M>(B, val, p, b, y, part, flag, dot_out, counter, st)
+  launch_plain<MODE, T, L, U, C, M>(B, val, p, b, y, part, flag, dot_out, counter, st, early)
+#define GB_PF(L, U, M) \
+  launch_pf<MODE, T, L, U, M>(B, val, p, b, y, part, flag, dot_out, counter, st, early)
   switch(variant) {
   case 6: launch_tma<MODE, T, 16>(B, val, p, b, y, part, flag, dot_out, counter, st); break;
   case 7: launch_tma<MODE, T, 8>(B, val, p, b, y, part, flag, dot_out, counter, st); break;
@@ -706,29 +709,30 @@ static void launch_bsr(int variant, const Bsr3 &B, const T *val, const T *p,
   case 11: GB_BSR(4, 2, 0, 0); break;
   case 12: GB_BSR(4, 4, 0, 0); break;
   case 13: GB_BSR(2, 4, 0, 0); break;
-  case 14: launch_pf<MODE, T, 8, 2, 0>(B, val, p, b, y, part, flag, dot_out, counter, st); break;
-  case 15: launch_pf<MODE, T, 8, 4, 0>(B, val, p, b, y, part, flag, dot_out, counter, st); break;
-  case 16: launch_pf<MODE, T, 4, 4, 0>(B, val, p, b, y, part, flag, dot_out, counter, st); break;
-  case 17: launch_pf<MODE, T, 4, 2, 0>(B, val, p, b, y, part, flag, dot_out, counter, st); break;
-  case 18: launch_pf<MODE, T, 8, 2, 8>(B, val, p, b, y, part, flag, dot_out, counter, st); break;
+  case 14: GB_PF(8, 2, 0); break;
+  case 15: GB_PF(8, 4, 0); break;
+  case 16: GB_PF(4, 4, 0); break;
+  case 17: GB_PF(4, 2, 0); break;
+  case 18: GB_PF(8, 2, 8); break;
   default: GB_BSR(8, 2, 1, 0); break;
   }
 #undef GB_BSR
+#undef GB_PF
 }
 
 void bsr_spmv_dot32(const Bsr3 &B, const float *p, float *q, double *part,
                     const int *flag, double *dot_out, unsigned *counter,
-                    cudaStream_t st)
+                    cudaStream_t st, bool early)
 {
   launch_bsr<2, float>(B.var32, B, B.val32.p, p, nullptr, q, part, flag, st,
-                       dot_out, counter);
+                       dot_out, counter, early);
 }
 void bsr_spmv_dot64(const Bsr3 &B, const double *p, double *q, double *part,
                     const int *flag, double *dot_out, unsigned *counter,
-                    cudaStream_t st)
+                    cudaStream_t st, bool early)
 {
   launch_bsr<2, double>(B.var64, B, B.val64.p, p, nullptr, q, part, flag, st,
-                        dot_out, counter);
+                        dot_out, counter, early);
 }
 void bsr_residual64(const Bsr3 &B, const double *x, const double *b, double *r,
                     double *part, const int *flag, cudaStream_t st)

@@ -77,7 +77,6 @@ __global__ void k_convert(long long n, const TI *__restrict__ in,
 // ---------------------------------------------------------------------------
 struct CgState {
   double rho;    // <r, r> of the previous step (fpar(7))
-  double alpha;  // step length
   double beta;
   double tol;    // fpar(4) = rtol * ||r0|| + atol
   double res;    // fpar(5) = fpar(6) = ||r||
@@ -115,7 +114,7 @@ __global__ void k_cg_start(CgState *S, const double *__restrict__ part_rr,
     S->maxit = maxit;
     S->status = 1;
     S->active = 1;
-    S->alpha = S->beta = 0.;
+    S->beta = 0.;
     S->update = S->convert = S->final_ = S->updates = 0;
     S->tick_dot = S->tick_step = 0u;
     // no test before the first step, as in iters.f's cg: a zero or
@@ -155,45 +154,53 @@ __device__ __forceinline__ int cg_breakdown(double pq)
   return fabs(pq) <= 1.7976931348623157e308 ? 0 : -9;
 }
 
+// what the tests below need of the state, loaded while the step's vectors are
+// on their way (each would be a round trip to L2 at the end of the chain)
+struct CgTest {
+  double rho, tol, maxrr, delta2;
+  int its, maxit;
+};
+
 // the stopping test of the FP64 CG (stopbis: the iteration cap first, then
 // the residual test)
-__device__ void cg_check_tail(CgState *S, double rr)
+__device__ void cg_check_tail(CgState *S, const CgTest &c, double rr)
 {
-  if(S->maxit > 0 && S->its >= S->maxit) {
+  const double beta = rr / c.rho;  // (beside the root, not after it)
+  const double res = sqrt(rr);
+  S->res = res;
+  if(c.maxit > 0 && c.its >= c.maxit) {
     S->status = -1;
-    S->active = 0;
-    S->res = sqrt(rr);
+    S->go = S->active = 0;
     return;
   }
-  S->res = sqrt(rr);
-  if(!(S->res > S->tol)) {
-    S->status = (S->res == S->res) ? 0 : -10;
-    S->active = 0;
+  if(!(res > c.tol)) {
+    S->status = (res == res) ? 0 : -10;
+    S->go = S->active = 0;
     return;
   }
-  S->beta = rr / S->rho;  // (beside the root, not after it)
+  S->beta = beta;
   S->rho = rr;
 }
 
 // the reliable-update test of the mixed CG: replace the residual when the
 // FP32 one has dropped by delta since the last update, claims convergence,
 // or the iteration cap is reached
-__device__ void rcg_check_tail(CgState *S, double rr)
+__device__ void rcg_check_tail(CgState *S, const CgTest &c, double rr)
 {
+  const double beta = rr / c.rho;
+  const double tol2 = c.tol * c.tol;
+  const bool cap = (c.maxit > 0 && c.its >= c.maxit);
   S->convert = 0;
-  double tol2 = S->tol * S->tol;
-  bool cap = (S->maxit > 0 && S->its >= S->maxit);
-  if(cap || !(rr > tol2) || rr < S->delta2 * S->maxrr) {
+  if(cap || !(rr > tol2) || rr < c.delta2 * c.maxrr) {
     S->update = 1;
+    S->go = 0;
     S->final_ = cap ? 1 : 0;
     S->res = sqrt(rr);
     return;
   }
-  S->update = 0;
-  if(rr > S->maxrr) S->maxrr = rr;
-  S->beta = rr / S->rho;
+  if(rr > c.maxrr) S->maxrr = rr;
+  S->beta = beta;
   S->rho = rr;
-  S->res = sqrt(rr);
 }
 
 // One CG step after the SpMV: alpha = rho / <p, Ap> (from S->pq), x += alpha
@@ -201,10 +208,8 @@ __device__ void rcg_check_tail(CgState *S, double rr)
 // the iteration, applies brkdn and the stopping (or update) test.
 template <typename T, bool MIXED>
 __global__ void __launch_bounds__(256)
-k_cg_step(int n, CgState *__restrict__ S, T *__restrict__ x, T *__restrict__ r,
-          const T *__restrict__ p, const T *__restrict__ q, double *__restrict__ part)
+k_cg_step(int n, CgState *S, T *x, T *r, const T *p, const T *q, double *__restrict__ part)
 {
-  if(!S->go) return;
   // alpha and the breakdown test once per CTA: FP64 divisions in every
   // thread would keep the FP64 pipe busier than the vector traffic.  The
   // first entries are on their way meanwhile.  Vectors are cudaMalloc'ed
@@ -219,12 +224,15 @@ k_cg_step(int n, CgState *__restrict__ S, T *__restrict__ x, T *__restrict__ r,
     ld4(x, i4, xv);
     ld4(r, i4, rv);
     ld4(p, i4, pv);
-    ld4(q, i4, qv);
   }
-  const double pq = S->pq, rho = S->rho;
+  const CgTest test = {S->rho, S->tol, S->maxrr, S->delta2, S->its + 1, S->maxit};
+  chain_wait();  // q and pq are the product's, all above is older
+  if(!S->go) return;  // the same in every CTA (as the product read it)
+  if(i4 < n4) ld4(q, i4, qv);
   if(threadIdx.x == 0) {
+    const double pq = S->pq;
     s_bad = cg_breakdown(pq);
-    s_alpha = s_bad ? (T)0 : (T)(rho / pq);
+    s_alpha = s_bad ? (T)0 : (T)(test.rho / pq);
   }
   __syncthreads();
   const int bad = s_bad;
@@ -262,43 +270,37 @@ k_cg_step(int n, CgState *__restrict__ S, T *__restrict__ x, T *__restrict__ r,
   if(!arrive_last(&S->tick_step)) return;
   double rr = sum_partials_l2<256>(part, gridDim.x);
   if(threadIdx.x == 0) {
-    S->its += 1;
+    S->its = test.its;
     if(bad) {
       S->status = bad;
-      S->active = 0;
-      S->alpha = 0.;
+      S->go = S->active = 0;
     }
-    else {
-      S->alpha = rho / pq;
-      if(MIXED)
-        rcg_check_tail(S, rr);
-      else
-        cg_check_tail(S, rr);
-    }
-    S->go = S->active && !S->update;
+    else if(MIXED)
+      rcg_check_tail(S, test, rr);
+    else
+      cg_check_tail(S, test, rr);
   }
 }
 
+// p = r + beta p
 template <typename T>
-__global__ void k_cg_p(int n, const CgState *__restrict__ S, T *__restrict__ p,
-                       const T *__restrict__ r)
+__global__ void __launch_bounds__(256) k_cg_p(int n, const CgState *S, T *p, const T *r)
 {
-  if(!S->go) return;
-  T b = (T)S->beta;
   const long long stride = (long long)gridDim.x * blockDim.x;
-  const long long n4 = n / 4;
-  for(long long i4 = (long long)blockIdx.x * blockDim.x + threadIdx.x; i4 < n4;
-      i4 += stride) {
-    T rv[4], pv[4];
+  const long long n4 = n / 4, first = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  T rv[4], pv[4];
+  if(first < n4) ld4(p, first, pv);
+  chain_wait();  // r, beta and go are the step's, p is older
+  if(!S->go) return;
+  const T b = (T)S->beta;
+  for(long long i4 = first; i4 < n4; i4 += stride) {
     ld4(r, i4, rv);
-    ld4(p, i4, pv);
+    if(i4 != first) ld4(p, i4, pv);
 #pragma unroll
     for(int c = 0; c < 4; c++) pv[c] = rv[c] + b * pv[c];
     st4(p, i4, pv);
   }
-  for(long long i = 4 * n4 + (long long)blockIdx.x * blockDim.x + threadIdx.x;
-      i < n; i += stride)
-    p[i] = r[i] + b * p[i];
+  for(long long i = 4 * n4 + first; i < n; i += stride) p[i] = r[i] + b * p[i];
 }
 
 template <typename T>
@@ -312,9 +314,10 @@ __global__ void k_copy(long long n, const T *__restrict__ a, T *__restrict__ b)
 template <int TPR, typename V, typename XT>
 __global__ void __launch_bounds__(256)
 k_cg_spmv(int n, const int *__restrict__ rowptr, const int *__restrict__ col,
-          const V *__restrict__ val, const XT *__restrict__ p,
+          const V *__restrict__ val, const XT *p,
           XT *__restrict__ q, double *__restrict__ part, CgState *S)
 {
+  chain_wait();
   if(!S->go) return;
   const int rows_per_block = 256 / TPR;
   int lane = threadIdx.x % TPR;
@@ -346,20 +349,31 @@ k_cg_spmv(int n, const int *__restrict__ rowptr, const int *__restrict__ col,
 
 template <typename V, typename XT>
 static void cg_spmv(const gb300_matrix *A, const V *val, const XT *p, XT *q,
-                    double *part, CgState *S, cudaStream_t st)
+                    double *part, CgState *S, cudaStream_t st, bool early = false)
 {
   int n = A->n;
   const int g = grid_for(n, 256 / A->tpr, kReduceBlocks);
+  auto go = [&](auto kernel) {
+    launch_chain(early, kernel, g, 256, st, n, A->rowptr.p, A->col.p, val, p, q, part, S);
+  };
   switch(A->tpr) {
-  case 2: k_cg_spmv<2><<<g, 256, 0, st>>>(n, A->rowptr.p, A->col.p, val, p, q, part, S); break;
-  case 4: k_cg_spmv<4><<<g, 256, 0, st>>>(n, A->rowptr.p, A->col.p, val, p, q, part, S); break;
-  case 8: k_cg_spmv<8><<<g, 256, 0, st>>>(n, A->rowptr.p, A->col.p, val, p, q, part, S); break;
-  case 16: k_cg_spmv<16><<<g, 256, 0, st>>>(n, A->rowptr.p, A->col.p, val, p, q, part, S); break;
-  default: k_cg_spmv<32><<<g, 256, 0, st>>>(n, A->rowptr.p, A->col.p, val, p, q, part, S); break;
+  case 2: go(k_cg_spmv<2, V, XT>); break;
+  case 4: go(k_cg_spmv<4, V, XT>); break;
+  case 8: go(k_cg_spmv<8, V, XT>); break;
+  case 16: go(k_cg_spmv<16, V, XT>); break;
+  default: go(k_cg_spmv<32, V, XT>); break;
   }
 }
 
-// Runs CG on the operator applied by spmv_dot(p, q, part, S, stream)
+// Up to which vector length a CG step's kernels start while the one before
+// drains (launch_chain): their CTAs then load what is older than it (block row
+// bounds, x, r, p) and wait.  Where the product fills the chip, the waiting
+// CTAs take slots from it.  Time per iteration without / with, FP64 and mixed:
+// 18.2 / 17.9 and 20.7 / 19.1 us at 3,630 unknowns, 26.7 / 26.3 and 20.6 / 18.8
+// at 34,914 (46,552 entries), 46.1 / 49.9 and 25.6 / 26.7 at 124,950 (166,600).
+static bool cg_early(int n) { return n <= 65536; }
+
+// Runs CG on the operator applied by spmv_dot(p, q, part, S, stream, early)
 // (q = A p with the partials of <p, q>), y = rhs from y = 0, to
 // ||r|| <= rtol ||rhs||.  T is the vector type, n the vector length.
 // Returns the final state in *hs.
@@ -388,6 +402,7 @@ static int cg_core(cudaStream_t st, int n, SPMV spmv_dot, const T *rhs, T *y,
 
   // capture a batch of iterations once
   const int batch = n > 200000 ? 16 : 32;
+  const bool early = cg_early(n);
   // no CTA without rows: each would still arrive at the counter the step's
   // sums wait for (1,216 CTAs for 46 CTAs' rows at 34,914 unknowns)
   const int step_grid =
@@ -396,9 +411,10 @@ static int cg_core(cudaStream_t st, int n, SPMV spmv_dot, const T *rhs, T *y,
   cudaGraphExec_t exec;
   GB_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
   for(int it = 0; it < batch; it++) {
-    spmv_dot(p, q, part, S, st);
-    k_cg_step<T, false><<<step_grid, 256, 0, st>>>(n, S, y, r, p, q, part);
-    k_cg_p<T><<<grid_for((n + 3) / 4, 256, kReduceBlocks * 4), 256, 0, st>>>(n, S, p, r);
+    spmv_dot(p, q, part, S, st, early);
+    launch_chain(early, k_cg_step<T, false>, step_grid, 256, st, n, S, y, r, p, q, part);
+    launch_chain(early, k_cg_p<T>, grid_for((n + 3) / 4, 256, kReduceBlocks * 4), 256, st, n, S,
+                 p, r);
   }
   GB_CUDA(cudaStreamEndCapture(st, &graph));
   GB_CUDA(cudaGraphInstantiate(&exec, graph, 0));
@@ -594,7 +610,7 @@ static double reliable_delta(const gb300_solver_params *p)
   return (d > 0. && d < 1.) ? d : 0.3;
 }
 
-// spmv32(p, q, part, S, st): FP32 q = A p with partial <p, q>;
+// spmv32(p, q, part, S, st, early): FP32 q = A p with partial <p, q>;
 // res64(x, b, r, part, flag, st): FP64 r = b - A x with partial ||r||^2
 template <typename SPMV32, typename RES64>
 static int cg_mixed_core(cudaStream_t st, int n, SPMV32 spmv32, RES64 res64,
@@ -626,15 +642,17 @@ static int cg_mixed_core(cudaStream_t st, int n, SPMV32 spmv32, RES64 res64,
   // resumes.  The iterations and their arithmetic are those of the one-graph
   // sequence; only the place where the update kernels run moves.
   const int batch = n > 200000 ? 16 : 32;
+  const bool early = cg_early(n);
   const int step_grid =
     std::min(resident_grid(k_cg_step<float, true>, 256, 0), grid_for((n + 3) / 4, 256));
   cudaGraph_t graph, ugraph;
   cudaGraphExec_t exec, uexec;
   GB_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
   for(int it = 0; it < batch; it++) {
-    spmv32(p32, q32, part, S, st);
-    k_cg_step<float, true><<<step_grid, 256, 0, st>>>(n, S, x32, r32, p32, q32, part);
-    k_cg_p<float><<<gs, 256, 0, st>>>(n, S, p32, r32);
+    spmv32(p32, q32, part, S, st, early);
+    launch_chain(early, k_cg_step<float, true>, step_grid, 256, st, n, S, x32, r32, p32, q32,
+                 part);
+    launch_chain(early, k_cg_p<float>, gs, 256, st, n, S, p32, r32);
   }
   GB_CUDA(cudaStreamEndCapture(st, &graph));
   GB_CUDA(cudaGraphInstantiate(&exec, graph, 0));
@@ -863,16 +881,16 @@ int solve(gb300_matrix *A, const gb300_vector *bvec,
       to_nodes64(nn, rhs, rhs4, st);
       if(!mixed) {
         auto spmv = [&](const double *pp, double *qq, double *part,
-                        CgState *S, cudaStream_t s) {
-          bsr_spmv_dot64(B, pp, qq, part, &S->go, &S->pq, &S->tick_dot, s);
+                        CgState *S, cudaStream_t s, bool early) {
+          bsr_spmv_dot64(B, pp, qq, part, &S->go, &S->pq, &S->tick_dot, s, early);
         };
         GB_TRY(cg_core<double>(st, n4, spmv, rhs4, x4, p->stopping_test,
                                p->nb_iter_max, &hs, W));
       }
       else {
         auto spmv = [&](const float *pp, float *qq, double *part,
-                        CgState *S, cudaStream_t s) {
-          bsr_spmv_dot32(B, pp, qq, part, &S->go, &S->pq, &S->tick_dot, s);
+                        CgState *S, cudaStream_t s, bool early) {
+          bsr_spmv_dot32(B, pp, qq, part, &S->go, &S->pq, &S->tick_dot, s, early);
         };
         auto res = [&](const double *xx, const double *bb, double *rr,
                        double *part, const int *flag, cudaStream_t s) {
@@ -886,8 +904,8 @@ int solve(gb300_matrix *A, const gb300_vector *bvec,
     }
     else if(!mixed) {
       auto spmv = [&](const double *pp, double *qq, double *part,
-                      CgState *S, cudaStream_t s) {
-        cg_spmv<double, double>(A, val, pp, qq, part, S, s);
+                      CgState *S, cudaStream_t s, bool early) {
+        cg_spmv<double, double>(A, val, pp, qq, part, S, s, early);
       };
       GB_TRY(cg_core<double>(st, n, spmv, rhs, x, p->stopping_test,
                              p->nb_iter_max, &hs, W));
@@ -898,8 +916,8 @@ int solve(gb300_matrix *A, const gb300_vector *bvec,
       k_convert<float, double><<<grid_for(A->nnz, 256), 256, 0, st>>>(A->nnz, val, v32.p);
       const float *v32p = v32.p;
       auto spmv = [&](const float *pp, float *qq, double *part,
-                      CgState *S, cudaStream_t s) {
-        cg_spmv<float, float>(A, v32p, pp, qq, part, S, s);
+                      CgState *S, cudaStream_t s, bool early) {
+        cg_spmv<float, float>(A, v32p, pp, qq, part, S, s, early);
       };
       auto res = [&](const double *xx, const double *bb, double *rr,
                      double *part, const int *flag, cudaStream_t s) {

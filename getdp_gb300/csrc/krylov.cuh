@@ -52,10 +52,10 @@ void from_nodes64(int nn, const double *in, double *out, cudaStream_t st);
 // writes the sum <p, q> there (counter: a zeroed word owned by the caller)
 void bsr_spmv_dot32(const Bsr3 &B, const float *p, float *q, double *part,
                     const int *flag, double *dot_out, unsigned *counter,
-                    cudaStream_t st);
+                    cudaStream_t st, bool early = false);
 void bsr_spmv_dot64(const Bsr3 &B, const double *p, double *q, double *part,
                     const int *flag, double *dot_out, unsigned *counter,
-                    cudaStream_t st);
+                    cudaStream_t st, bool early = false);
 void bsr_residual64(const Bsr3 &B, const double *x, const double *b, double *r,
                     double *part, const int *flag, cudaStream_t st);
 // GB300_ERR_CUDA if a staged SpMV variant timed out during the solve
