@@ -10,8 +10,11 @@
 // its own grid launch.  For the solves, each wide level also keeps its rows'
 // L (resp. U) entries in a sliced-ELL copy (32 rows per slice, entry j of
 // the slice's rows side by side), so that a warp reads them coalesced and
-// without the row-pointer indirection.  The triangular solves follow lusol
-// (ilut.F:2297-2347) row by row in the same accumulation order.
+// without the row-pointer indirection; on a multicolour copy the sweeps are a
+// chain of launches colour by colour over consecutive rows (k_colour_sweep),
+// and a small system's whole step of sweeps and product is one CTA
+// (k_small_step).  The triangular solves follow lusol (ilut.F:2297-2347) row
+// by row in the same accumulation order.
 //
 // GMRES(m) and FGMRES(m) follow iters.f:1912-2219 / :2522-2806 with right
 // preconditioning (Preconditioner_Position 2): restart residual, Arnoldi

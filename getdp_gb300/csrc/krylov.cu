@@ -766,20 +766,6 @@ int norm2_dev(int n, const double *v, double *out, Work &W, cudaStream_t st)
   return GB300_OK;
 }
 
-__global__ void k_axpy_scaled(int n, double a, const float *__restrict__ d,
-                              double *__restrict__ x)
-{
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if(i < n) x[i] += a * (double)d[i];
-}
-
-__global__ void k_to32_scaled(int n, double s, const double *__restrict__ r,
-                              float *__restrict__ o)
-{
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if(i < n) o[i] = (float)(r[i] * s);
-}
-
 // the first empty row, if any (Sparskit.cpp:220-223); found on the device (the
 // row pointers had been copied to pageable host memory, 0.7 ms at 1 M rows)
 __global__ void k_zero_row(int n, const int *__restrict__ rowptr, int *__restrict__ first)
