@@ -249,13 +249,14 @@ template <typename T> __device__ __forceinline__ T ld_stream(const T *p)
 
 // Partial dot product of one CSR row with x for the TPR lanes that share
 // the row: each lane first issues U independent (column, value) loads, then
-// the U gathers of x through the read-only path, then the multiply-adds, so
-// a warp keeps U memory requests in flight instead of one dependent chain.
-template <int TPR, int U, typename ACC, typename V, typename XT>
+// the U gathers of x, then the multiply-adds, so a warp keeps U memory
+// requests in flight instead of one dependent chain.  READ_ONLY: x through the
+// read-only path, for kernels in whose lifetime nothing writes it; a kernel
+// that may start while x's writer runs (launch_chain) takes plain loads.
+template <int TPR, int U, typename ACC, bool READ_ONLY = true, typename V, typename XT>
 __device__ __forceinline__ ACC csr_row_dot(int s, int e, int lane,
                                            const int *__restrict__ col,
-                                           const V *__restrict__ val,
-                                           const XT *__restrict__ x)
+                                           const V *__restrict__ val, const XT *x)
 {
   ACC sum = 0;
   for(int k0 = s + lane; k0 < e; k0 += TPR * U) {
@@ -270,7 +271,7 @@ __device__ __forceinline__ ACC csr_row_dot(int s, int e, int lane,
     }
     XT xv[U];
 #pragma unroll
-    for(int u = 0; u < U; u++) xv[u] = __ldg(x + c[u]);
+    for(int u = 0; u < U; u++) xv[u] = READ_ONLY ? __ldg(x + c[u]) : x[c[u]];
 #pragma unroll
     for(int u = 0; u < U; u++) sum += (ACC)v[u] * (ACC)xv[u];
   }

@@ -310,7 +310,8 @@ __global__ void k_copy(long long n, const T *__restrict__ a, T *__restrict__ b)
   if(i < n) b[i] = a[i];
 }
 
-// SpMV with the CG dot fused, guarded by the active flag
+// SpMV with the CG dot fused, guarded by the active flag.  p is written by the
+// kernel before, which may still run when this one starts: plain loads
 template <int TPR, typename V, typename XT>
 __global__ void __launch_bounds__(256)
 k_cg_spmv(int n, const int *__restrict__ rowptr, const int *__restrict__ col,
@@ -329,7 +330,7 @@ k_cg_spmv(int n, const int *__restrict__ rowptr, const int *__restrict__ col,
     XT sum = 0;
     if(row < n) {
       int s = rowptr[row], e = rowptr[row + 1];
-      sum = csr_row_dot<TPR, (TPR >= 16 ? 4 : 2), XT>(s, e, lane, col, val, p);
+      sum = csr_row_dot<TPR, (TPR >= 16 ? 4 : 2), XT, false>(s, e, lane, col, val, p);
     }
 #pragma unroll
     for(int o = TPR / 2; o > 0; o >>= 1)
