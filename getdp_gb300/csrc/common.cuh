@@ -253,6 +253,8 @@ template <typename T> __device__ __forceinline__ T ld_stream(const T *p)
 // requests in flight instead of one dependent chain.  READ_ONLY: x through the
 // read-only path, for kernels in whose lifetime nothing writes it; a kernel
 // that may start while x's writer runs (launch_chain) takes plain loads.
+// Lanes past the row's end add nothing: the product of a zero with an entry of
+// x that the row does not hold is NaN where that entry is not finite.
 template <int TPR, int U, typename ACC, bool READ_ONLY = true, typename V, typename XT>
 __device__ __forceinline__ ACC csr_row_dot(int s, int e, int lane,
                                            const int *__restrict__ col,
@@ -266,14 +268,16 @@ __device__ __forceinline__ ACC csr_row_dot(int s, int e, int lane,
     for(int u = 0; u < U; u++) {
       int k = k0 + u * TPR;
       bool in = k < e;
-      c[u] = in ? __ldcs(col + k) : 0;
+      c[u] = in ? __ldcs(col + k) : -1;
       v[u] = in ? __ldcs(val + k) : (V)0;
     }
     XT xv[U];
 #pragma unroll
-    for(int u = 0; u < U; u++) xv[u] = READ_ONLY ? __ldg(x + c[u]) : x[c[u]];
+    for(int u = 0; u < U; u++)
+      xv[u] = c[u] < 0 ? (XT)0 : READ_ONLY ? __ldg(x + c[u]) : x[c[u]];
 #pragma unroll
-    for(int u = 0; u < U; u++) sum += (ACC)v[u] * (ACC)xv[u];
+    for(int u = 0; u < U; u++)
+      if(c[u] >= 0) sum += (ACC)v[u] * (ACC)xv[u];
   }
   return sum;
 }

@@ -9,8 +9,9 @@
 // MODE 1) whose scratch memory -- one partial sum per block plus the final
 // sum -- lives in a file-scope device array instead of a per-call buffer.
 //
-// Limit: one partial sum per block of kRowsPerBlock rows, at most
-// kMaxBlocks blocks, so n <= kMaxBlocks * kRowsPerBlock = 33,554,432 rows;
+// Limit: one partial sum per block, at most kMaxBlocks blocks, each of as many
+// rows as that takes (kRowsPerBlock at most), so
+// n <= kMaxBlocks * kRowsPerBlock = 33,554,432 rows;
 // the array takes (kMaxBlocks + 1) * 8 bytes = 128 KiB + 8 bytes on every GPU
 // that loads the library, until the process exits.
 //
