@@ -27,7 +27,9 @@
 //     number of entries one coarse entry receives (2^-51 for 1,000);
 //   * the dense inverse is a blocked symmetric elimination without pivoting,
 //     two launches per 32 pivots (Ac is symmetric positive definite when A is
-//     and no aggregate is empty; a pivot <= 0 is reported as an error);
+//     and no aggregate is empty; a pivot <= 0 is reported as an error).  An Ac
+//     that is not symmetric is found on the device and inverted by Gauss-Jordan
+//     steps, one launch per pivot;
 //   * restriction and the coarse product are warp sums in a fixed order.
 #include <math.h>
 #include <string.h>
@@ -589,6 +591,96 @@ k_sweep_finish(int nc, double *__restrict__ a, const int *err)
   }
 }
 
+// *err = kAsymmetric where two mirrored entries differ by more than rounding:
+// than the fixed-point sums' own (2^(headroom - 1) terms, half a quantum each,
+// in both) and 2^-44 of their rows' diagonals, for an A assembled in another
+// order above and below its diagonal (the elimination's backward error, some
+// nc 2^-53, is no smaller).  The symmetric sweep's kernels then do nothing.
+constexpr int kAsymmetric = -2;
+
+__global__ void __launch_bounds__(256)
+k_coarse_symmetric(int nc, int headroom, const unsigned long long *amax_bits,
+                   const double *__restrict__ a, int *err)
+{
+  __shared__ double s[32][33];
+  const int ti = blockIdx.y, tj = blockIdx.x;
+  if(tj > ti) return;
+  const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
+  for(int r = y; r < 32; r += 8) {
+    const int i = tj * 32 + r, j = ti * 32 + x;  // the transposed tile
+    s[r][x] = i < nc && j < nc ? a[(size_t)i * nc + j] : 0.;
+  }
+  __syncthreads();
+  int e = 0;
+  frexp(__longlong_as_double((long long)*amax_bits), &e);
+  const double sums = ldexp(1., e + 2 * headroom - 63);
+  for(int r = y; r < 32; r += 8) {
+    const int i = ti * 32 + r, j = tj * 32 + x;
+    if(i >= nc || j >= i) continue;
+    const double d = fabs(a[(size_t)i * nc + j] - s[x][r]) - sums;
+    if(d <= 0.) continue;
+    const double di = a[(size_t)i * nc + i], dj = a[(size_t)j * nc + j];
+    if(d > 0x1p-44 * sqrt(fabs(di)) * sqrt(fabs(dj))) atomicCAS(err, 0, kAsymmetric);
+  }
+}
+
+// The inverse of any other Ac, by Gauss-Jordan steps without pivoting (14.6 ms
+// at nc = 1024 against the sweep's 1.5: nc launches that read and write all
+// nc^2 entries).
+__global__ void k_gj_init(int nc, const double *__restrict__ a, double *rbuf, double *cbuf)
+{
+  for(int j = blockIdx.x * blockDim.x + threadIdx.x; j < nc; j += gridDim.x * blockDim.x) {
+    rbuf[j] = a[j];                 // row 0
+    cbuf[j] = a[(size_t)j * nc];    // column 0
+  }
+}
+
+// pivot step k of the in-place Gauss-Jordan inversion; row k and column k of
+// the matrix before the step come from the buffers of parity k, and the step
+// writes row and column k + 1 of its result to the other parity
+__global__ void k_gj_step(int nc, int k, double *a, double *rbuf, double *cbuf, int *err)
+{
+  if(*err) return;
+  const double *R = rbuf + (size_t)(k & 1) * nc;
+  const double *Cc = cbuf + (size_t)(k & 1) * nc;
+  double *Rn = rbuf + (size_t)((k + 1) & 1) * nc;
+  double *Cn = cbuf + (size_t)((k + 1) & 1) * nc;
+  const double piv = R[k];
+  if(!(piv > 0.) || !(piv <= 1.7976931348623157e308)) {
+    if(blockIdx.x == 0 && threadIdx.x == 0) atomicCAS(err, 0, k + 1);
+    return;
+  }
+  const double p = 1.0 / piv;
+  const long long m = (long long)nc * nc;
+  for(long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < m;
+      idx += (long long)gridDim.x * blockDim.x) {
+    const int i = (int)(idx / nc), j = (int)(idx - (long long)i * nc);
+    double v;
+    if(i == k)
+      v = (j == k) ? p : R[j] * p;
+    else if(j == k)
+      v = -Cc[i] * p;
+    else
+      v = fma(-Cc[i] * p, R[j], a[idx]);
+    a[idx] = v;
+    if(i == k + 1) Rn[j] = v;
+    if(j == k + 1) Cn[i] = v;
+  }
+}
+
+static int coarse_invert_general(Coarse *c, cudaStream_t st)
+{
+  const int nc = c->nc;
+  double *rbuf = c->panel.p, *cbuf = rbuf + 2 * (size_t)nc;  // (4 nc of 64 (nc + 32))
+  GB_CUDA(cudaMemsetAsync(c->err.p, 0, sizeof(int), st));
+  k_gj_init<<<grid_for(nc, 256), 256, 0, st>>>(nc, c->inv.p, rbuf, cbuf);
+  const int g = grid_for((long long)nc * nc, 256, kReduceBlocks * 2);
+  for(int k = 0; k < nc; k++)
+    k_gj_step<<<g, 256, 0, st>>>(nc, k, c->inv.p, rbuf, cbuf, c->err.p);
+  GB_CUDA(cudaGetLastError());
+  return GB300_OK;
+}
+
 int coarse_setup(gb300_matrix *A, const double *val, bool reuse)
 {
   Coarse *c = A->coarse;
@@ -606,8 +698,9 @@ int coarse_setup(gb300_matrix *A, const double *val, bool reuse)
       reinterpret_cast<unsigned long long *>(c->inv.p), c->err.p);
   k_coarse_to_double<<<grid_for(m, 256, kReduceBlocks), 256, 0, st>>>(m, c->headroom, amax,
                                                                       c->inv.p);
-  GB_CUDA(cudaGetLastError());
   const int nb = (nc + kSwB - 1) / kSwB;
+  k_coarse_symmetric<<<dim3(nb, nb), 256, 0, st>>>(nc, c->headroom, amax, c->inv.p, c->err.p);
+  GB_CUDA(cudaGetLastError());
   const int tiles = nb * (nb + 1) / 2;
   double *P = c->panel.p, *Wp = P + (size_t)nc * kSwB, *dinv = Wp + (size_t)nc * kSwB;
   GB_CUDA(cudaFuncSetAttribute(k_sweep_update, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -626,6 +719,11 @@ int coarse_setup(gb300_matrix *A, const double *val, bool reuse)
   int err = 0;
   GB_CUDA(cudaMemcpyAsync(&err, c->err.p, sizeof(int), cudaMemcpyDeviceToHost, st));
   GB_CUDA(cudaStreamSynchronize(st));
+  if(err == kAsymmetric) {  // Ac is as it was
+    GB_TRY(coarse_invert_general(c, st));
+    GB_CUDA(cudaMemcpyAsync(&err, c->err.p, sizeof(int), cudaMemcpyDeviceToHost, st));
+    GB_CUDA(cudaStreamSynchronize(st));
+  }
   if(err < 0) {
     set_error("coarse matrix: the matrix values are zero or not finite");
     return GB300_ERR_ARG;
