@@ -461,7 +461,9 @@ k_sweep_update(int nc, int nb, int kb, double *__restrict__ a, const double *__r
                const double *__restrict__ W, const double *__restrict__ dinv,
                double *__restrict__ dnext, int *err)
 {
-  if(*err) return;
+  // CTA 0 may set *err while this launch runs: one answer for the whole CTA
+  // (its threads meet at barriers below)
+  if(__syncthreads_or(*(volatile int *)err)) return;
   extern __shared__ double shared[];
   double (*buf)[kSwB][kSwB + 1] = reinterpret_cast<double (*)[kSwB][kSwB + 1]>(shared);
   __shared__ double rp[2];

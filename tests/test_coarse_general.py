@@ -92,3 +92,24 @@ def test_cycle_on_a_transport_problem(renumbering):
     # Ac is summed in fixed point (2^-51 of max|a| a term) and inverted: cond(Ac)
     # is some 100 here, and its error reaches z through contractions
     assert np.linalg.norm(got - z) <= 1e-11 * np.linalg.norm(z)
+
+
+@pytest.mark.parametrize("bad", [33, 515, 991])
+def test_bad_pivot_while_other_tiles_run(bad):
+    """The pivot is found by one CTA of an update whose other CTAs are at any
+    point of theirs; the next inversion on the same handle starts clean."""
+    nc = 1000
+    d = np.linspace(1.0, 2.0, nc)
+    uh = np.random.default_rng(bad).standard_normal(nc)
+    A = LA.gMatrix(nc)
+    for value in (-1.0, 1.5):
+        d[bad] = value
+        S = sp.diags(d).tocsr()
+        A.set_csr(S.indptr, S.indices, S.data)
+        A.set_aggregates(np.arange(nc), nc)
+        if value < 0:
+            with pytest.raises(LA.GetDPError, match=f"pivot {bad + 1} of {nc}"):
+                _energy(A, uh)
+        else:  # (one rounding of the entry's sum, one of its inverse)
+            ref = uh @ (uh / d)
+            assert abs(_energy(A, uh) - ref) <= nc * 2.3e-16 * ref
