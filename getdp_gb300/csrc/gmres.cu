@@ -1252,12 +1252,12 @@ k_gm_dots(int n, const double *V, size_t ldv, const double *w, double *part, GmS
   else {
     // mgsro's checks on ||w||^2 before it orthogonalises (iters.f:3475-3600):
     // zero (ierr -1) or abnormal (-2) leaves the column unwritten and ends
-    // the cycle; gmres then reports a break-down
+    // the cycle; gmres then reports a break-down.  (k_gm_update clears
+    // S->cycle: CTAs of the other groups may only now be reading it)
     S->nrm0 = v;
     if(!(v > 0. && 1. / v > 0.)) {
       S->its += 1;  // the Arnoldi step's product was formed
       S->breakdown = (v <= 0.) ? -1 : -2;
-      S->cycle = 0;
     }
   }
 }
@@ -1284,8 +1284,11 @@ k_gm_update(int n, int m, double *V, size_t ldv, const double *w, double *cur,
             const double *zt, double *Z, double *pn, GmState *S, int pass)
 {
   chain_wait();
-  const int go = S->cycle, again = S->reorth, k = S->k + 1;
-  if(!go || (pass == 1 && !again)) return;  // the same in every CTA
+  const int go = S->cycle, again = S->reorth, bad = S->breakdown, k = S->k + 1;
+  if(!go || bad || (pass == 1 && !again)) {  // the same in every CTA
+    if(bad && blockIdx.x == 0 && threadIdx.x == 0) S->cycle = 0;
+    return;
+  }
   const int nb = gridDim.x - 1;
   __shared__ double h[kMaxKrylov + 1];
   __shared__ double rc[kMaxKrylov], rs[kMaxKrylov], ra[kMaxKrylov];
