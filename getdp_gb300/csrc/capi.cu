@@ -21,23 +21,6 @@ void set_error(const char *fmt, ...)
   g_error = buf;
 }
 
-thread_local gb300_ctx *t_pool_ctx = nullptr;
-
-cudaError_t pool_alloc(void **p, size_t bytes, cudaStream_t *stream)
-{
-  gb300_ctx *c = t_pool_ctx;
-  if(!c->pool) return cudaMalloc(p, bytes);
-  cudaError_t e = cudaMallocFromPoolAsync(p, bytes, c->pool, c->stream);
-  if(e == cudaErrorMemoryAllocation) {  // what the pool holds in other sizes
-    cudaGetLastError();
-    cudaStreamSynchronize(c->stream);
-    cudaMemPoolTrimTo(c->pool, 0);
-    e = cudaMallocFromPoolAsync(p, bytes, c->pool, c->stream);
-  }
-  if(e == cudaSuccess) *stream = c->stream;
-  return e;
-}
-
 template <typename T> static int check(T *p, const char *what)
 {
   if(!p) {
@@ -166,17 +149,7 @@ int gb300_ctx_create(int device, gb300_ctx **out)
     set_error("cudaStreamCreate failed: %s", cudaGetErrorString(e));
     return GB300_ERR_CUDA;
   }
-  cudaMemPoolProps props = {};
-  props.allocType = cudaMemAllocationTypePinned;
-  props.location.type = cudaMemLocationTypeDevice;
-  props.location.id = device;
-  unsigned long long keep = gb::kPoolKeep;
-  if(cudaMemPoolCreate(&c->pool, &props) != cudaSuccess ||
-     cudaMemPoolSetAttribute(c->pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
-    cudaGetLastError();  // no pool: cudaMalloc instead
-    if(c->pool) cudaMemPoolDestroy(c->pool);
-    c->pool = nullptr;
-  }
+  gb::pool_open(&c->mem, device, c->stream);
   *out = c;
   return GB300_OK;
 }
@@ -188,7 +161,7 @@ int gb300_ctx_destroy(gb300_ctx *ctx)
   gb::gen_cache_free(ctx->gen);
   ctx->gen = nullptr;
   cudaStreamSynchronize(ctx->stream);  // (the frees above are in its order)
-  if(ctx->pool) cudaMemPoolDestroy(ctx->pool);
+  gb::pool_close(&ctx->mem);
   cudaStreamDestroy(ctx->stream);
   delete ctx;
   return GB300_OK;
@@ -218,14 +191,7 @@ int gb300_device_alloc(gb300_ctx *ctx, size_t bytes, void **out)
 {
   GB_TRY(check(ctx, "ctx"));
   GB_TRY(check(out, "out"));
-  cudaError_t e = cudaMalloc(out, bytes ? bytes : 1);
-  if(e == cudaErrorMemoryAllocation && ctx->pool) {
-    cudaGetLastError();
-    cudaStreamSynchronize(ctx->stream);
-    cudaMemPoolTrimTo(ctx->pool, 0);
-    e = cudaMalloc(out, bytes ? bytes : 1);
-  }
-  GB_CUDA(e);
+  GB_CUDA(gb::device_malloc(out, bytes ? bytes : 1));
   return GB300_OK;
 }
 

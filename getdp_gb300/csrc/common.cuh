@@ -12,6 +12,7 @@
 #include <vector>
 
 #include "../../include/getdp_gb300.h"
+#include "pool.h"
 
 namespace gb {
 
@@ -56,33 +57,6 @@ void set_error(const char *fmt, ...);
 constexpr int kReduceBlocks = 1216;  // 152 SMs x 8
 constexpr int kReduceThreads = 256;
 
-}  // namespace gb
-struct gb300_ctx;
-namespace gb {
-
-// The context whose memory pool DevBuf allocates from on this thread (null:
-// cudaMalloc).  Entry points that make scratch buffers on each call set it
-// for their duration: cudaMalloc and cudaFree cost some 10 to 200 us each and
-// the latter waits for the device (a Generate at 513^2 spent 0.2 of its
-// 0.3 ms in them).  A pool belongs to one context, so to one stream: a block
-// is handed out again in that stream's order only.
-extern thread_local gb300_ctx *t_pool_ctx;
-struct PoolScope {
-  gb300_ctx *before;
-  explicit PoolScope(gb300_ctx *c) : before(t_pool_ctx) { t_pool_ctx = c; }
-  ~PoolScope() { t_pool_ctx = before; }
-  PoolScope(const PoolScope &) = delete;
-  PoolScope &operator=(const PoolScope &) = delete;
-};
-// memory a pool holds on to (in use or free): several systems of 2.7 M unknowns
-// and 229 M entries (2.8 GB each, 4.8 GB of scratch in a solve), a ninth of the
-// device; at 8 GB a solve beside two other such systems mapped its scratch anew,
-// 14 ms each time
-constexpr unsigned long long kPoolKeep = 32ull << 30;
-// bytes from the pool of t_pool_ctx; *stream: where they are to be freed
-cudaError_t pool_alloc(void **p, size_t bytes, cudaStream_t *stream);
-inline bool pool_active() { return t_pool_ctx != nullptr; }
-
 template <typename T> struct DevBuf {
   T *p = nullptr;
   size_t n = 0;
@@ -108,8 +82,7 @@ template <typename T> struct DevBuf {
     if(count <= n && p) return GB300_OK;
     release();
     if(count == 0) return GB300_OK;
-    cudaError_t e = pool_active() ? pool_alloc((void **)&p, count * sizeof(T), &from)
-                                  : cudaMalloc((void **)&p, count * sizeof(T));
+    const cudaError_t e = device_alloc((void **)&p, count * sizeof(T), &from);
     if(e != cudaSuccess) {
       set_error("device allocation (%zu bytes) failed: %s", count * sizeof(T),
                 cudaGetErrorString(e));
@@ -375,15 +348,29 @@ struct gb300_ctx {
   int device = 0;
   cudaStream_t stream = nullptr;
   int num_sms = 152;
-  // scratch memory of the calls on this context (null: cudaMalloc); what is
-  // free in it beyond kPoolKeep goes back to the device at the next
-  // synchronisation, all of it with the context
-  cudaMemPool_t pool = nullptr;
+  // scratch memory of the calls on this context; what is free in it beyond
+  // kPoolKeep goes back to the device at the next synchronisation, all of it
+  // with the context or when the device has no other memory left
+  gb::MemPool mem;
   // CSR pattern, scatter positions and element colouring of the element
   // table last generated on this context: a Generate of the same table
   // (GetDP's ZeroMatrix recreates A before every Generate) reuses them
   gb::GenCache *gen = nullptr;
 };
+
+namespace gb {
+// DevBuf allocates from this context's pool on this thread.  Entry points that
+// make scratch buffers on each call set it for their duration: cudaMalloc and
+// cudaFree cost some 10 to 200 us each and the latter waits for the device (a
+// Generate at 513^2 spent 0.2 of its 0.3 ms in them).
+struct PoolScope {
+  MemPool *before;
+  explicit PoolScope(gb300_ctx *c) : before(t_pool) { t_pool = &c->mem; }
+  ~PoolScope() { t_pool = before; }
+  PoolScope(const PoolScope &) = delete;
+  PoolScope &operator=(const PoolScope &) = delete;
+};
+}  // namespace gb
 
 struct gb300_vector {
   gb300_ctx *ctx = nullptr;

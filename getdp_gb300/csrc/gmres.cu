@@ -1755,9 +1755,11 @@ int gmres_solve(gb300_matrix *A, const double *val, const double *rhs,
     }
   } steps, turns;
   auto capture = [&](Graph &G, auto body) -> int {
+    auto capturing = hold_capture();
     GB_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
     body();
     GB_CUDA(cudaStreamEndCapture(st, &G.g));
+    capturing.unlock();
     GB_CUDA(cudaGraphInstantiate(&G.e, G.g, 0));
     return GB300_OK;
   };

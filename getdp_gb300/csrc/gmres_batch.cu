@@ -588,6 +588,7 @@ int gmres_solve_batch(gb300_matrix *A, const double *val, const double *rhs,
 
   cudaGraph_t graph;
   cudaGraphExec_t exec;
+  auto capturing = hold_capture();
   GB_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
   k_b_residual<2, 0><<<gchunks, kBThreads, 0, st>>>(C, A->rowptr.p, A->col.p, val, x,
                                                     rhs, r, part, nullptr, V);
@@ -625,6 +626,7 @@ int gmres_solve_batch(gb300_matrix *A, const double *val, const double *rhs,
   k_b_after<<<gsys, 128, 0, st>>>(nsys, V);
   k_b_flags<<<1, 256, 0, st>>>(nsys, V, flags.p);
   GB_CUDA(cudaStreamEndCapture(st, &graph));
+  capturing.unlock();
   GB_CUDA(cudaGraphInstantiate(&exec, graph, 0));
 
   int hf[4] = {0, 1, 0, 0};

@@ -410,6 +410,7 @@ static int cg_core(cudaStream_t st, int n, SPMV spmv_dot, const T *rhs, T *y,
     std::min(resident_grid(k_cg_step<T, false>, 256, 0), grid_for((n + 3) / 4, 256));
   cudaGraph_t graph;
   cudaGraphExec_t exec;
+  auto capturing = hold_capture();
   GB_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
   for(int it = 0; it < batch; it++) {
     spmv_dot(p, q, part, S, st, early);
@@ -418,6 +419,7 @@ static int cg_core(cudaStream_t st, int n, SPMV spmv_dot, const T *rhs, T *y,
                  p, r);
   }
   GB_CUDA(cudaStreamEndCapture(st, &graph));
+  capturing.unlock();
   GB_CUDA(cudaGraphInstantiate(&exec, graph, 0));
   int active = 1;
   int launches = 0;
@@ -648,6 +650,7 @@ static int cg_mixed_core(cudaStream_t st, int n, SPMV32 spmv32, RES64 res64,
     std::min(resident_grid(k_cg_step<float, true>, 256, 0), grid_for((n + 3) / 4, 256));
   cudaGraph_t graph, ugraph;
   cudaGraphExec_t exec, uexec;
+  auto capturing = hold_capture();
   GB_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
   for(int it = 0; it < batch; it++) {
     spmv32(p32, q32, part, S, st, early);
@@ -656,7 +659,9 @@ static int cg_mixed_core(cudaStream_t st, int n, SPMV32 spmv32, RES64 res64,
     launch_chain(early, k_cg_p<float>, gs, 256, st, n, S, p32, r32);
   }
   GB_CUDA(cudaStreamEndCapture(st, &graph));
+  capturing.unlock();
   GB_CUDA(cudaGraphInstantiate(&exec, graph, 0));
+  capturing = hold_capture();
   GB_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
   k_rcg_fold<<<kReduceBlocks, 256, 0, st>>>(n, S, x, x32);
   res64(x, rhs, r64, part, &S->update, st);
@@ -664,6 +669,7 @@ static int cg_mixed_core(cudaStream_t st, int n, SPMV32 spmv32, RES64 res64,
   k_rcg_convert<<<kReduceBlocks, 256, 0, st>>>(n, S, r64, r32);
   k_cg_p<float><<<gs, 256, 0, st>>>(n, S, p32, r32);
   GB_CUDA(cudaStreamEndCapture(st, &ugraph));
+  capturing.unlock();
   GB_CUDA(cudaGraphInstantiate(&uexec, ugraph, 0));
   struct Flags {
     int active, update;
