@@ -362,10 +362,11 @@ namespace gb {
 // DevBuf allocates from this context's pool on this thread.  Entry points that
 // make scratch buffers on each call set it for their duration: cudaMalloc and
 // cudaFree cost some 10 to 200 us each and the latter waits for the device (a
-// Generate at 513^2 spent 0.2 of its 0.3 ms in them).
+// Generate at 513^2 spent 0.2 of its 0.3 ms in them).  Null: no pool, for
+// buffers that may outlive the context.
 struct PoolScope {
   MemPool *before;
-  explicit PoolScope(gb300_ctx *c) : before(t_pool) { t_pool = &c->mem; }
+  explicit PoolScope(gb300_ctx *c) : before(t_pool) { t_pool = c ? &c->mem : nullptr; }
   ~PoolScope() { t_pool = before; }
   PoolScope(const PoolScope &) = delete;
   PoolScope &operator=(const PoolScope &) = delete;

@@ -582,17 +582,22 @@ static int mp_prepare(gb300_mpnn *net, const gb300_matrix *A)
     set_error("network: matrix not assembled");
     return GB300_ERR_ARG;
   }
-  GB_TRY(g.ehat.alloc(A->nnz));
-  GB_TRY(g.feat.alloc((size_t)n * 4));
-  GB_TRY(g.dscale.alloc(n));
-  GB_TRY(g.dinv.alloc(n));
-  GB_TRY(g.diag.alloc(n));
-  GB_TRY(g.tpos.alloc(A->nnz));
-  GB_TRY(g.h.alloc((size_t)(kLayers + 1) * n * kH));
-  GB_TRY(g.m.alloc((size_t)kLayers * n * kH));
-  GB_TRY(g.dh.alloc((size_t)2 * n * kH));
-  GB_TRY(g.dm.alloc((size_t)n * kH));
-  GB_TRY(g.G.alloc(A->nnz));
+  {
+    // kept with the network, which may be used on another context's matrix next
+    // and outlive this one's: not from its pool
+    PoolScope kept(nullptr);
+    GB_TRY(g.ehat.alloc(A->nnz));
+    GB_TRY(g.feat.alloc((size_t)n * 4));
+    GB_TRY(g.dscale.alloc(n));
+    GB_TRY(g.dinv.alloc(n));
+    GB_TRY(g.diag.alloc(n));
+    GB_TRY(g.tpos.alloc(A->nnz));
+    GB_TRY(g.h.alloc((size_t)(kLayers + 1) * n * kH));
+    GB_TRY(g.m.alloc((size_t)kLayers * n * kH));
+    GB_TRY(g.dh.alloc((size_t)2 * n * kH));
+    GB_TRY(g.dm.alloc((size_t)n * kH));
+    GB_TRY(g.G.alloc(A->nnz));
+  }
   DevBuf<int> bad;
   GB_TRY(bad.alloc(1));
   GB_CUDA(cudaMemsetAsync(bad.p, 0, sizeof(int), st));
