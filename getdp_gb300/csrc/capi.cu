@@ -81,6 +81,9 @@ static int stage_bulk(gb300_matrix *A, long long count, const int *i, const int 
   GB_TRY(grow(A->sr, A->staged, host + count, st));
   GB_TRY(grow(A->sc, A->staged, host + count, st));
   GB_TRY(grow(A->sv, A->staged, host + count, st));
+  DevBuf<unsigned long long> first;
+  GB_TRY(first.alloc(1));
+  FetchEnd fetches(A->ctx);
   if(host > 0) {  // entries staged on the host were added before
     GB_TRY(fetch_pageable(A->ctx, A->sr.p + A->staged, A->hr.data(), sizeof(int) * host));
     GB_TRY(fetch_pageable(A->ctx, A->sc.p + A->staged, A->hc.data(), sizeof(int) * host));
@@ -89,14 +92,13 @@ static int stage_bulk(gb300_matrix *A, long long count, const int *i, const int 
   GB_TRY(fetch_pageable(A->ctx, A->sr.p + at, i, sizeof(int) * count));
   GB_TRY(fetch_pageable(A->ctx, A->sc.p + at, j, sizeof(int) * count));
   GB_TRY(fetch_pageable(A->ctx, A->sv.p + at, v, sizeof(double) * count));
-  DevBuf<unsigned long long> first;
-  GB_TRY(first.alloc(1));
   GB_CUDA(cudaMemsetAsync(first.p, 0xff, sizeof(unsigned long long), st));
   k_bad_entry<<<grid_for(count, 256), 256, 0, st>>>(count, A->n, A->sr.p + at, A->sc.p + at,
                                                     first.p);
   unsigned long long h = 0;
   GB_CUDA(cudaMemcpyAsync(&h, first.p, sizeof(h), cudaMemcpyDeviceToHost, st));
   GB_CUDA(cudaStreamSynchronize(st));  // the caller's arrays have been read
+  fetches.done = true;
   if(h != ~0ull) {  // nothing of this call is added
     set_error("entry %lld (%d, %d) out of range [0, %d)", (long long)h, i[h], j[h], A->n);
     return GB300_ERR_ARG;
@@ -597,6 +599,7 @@ int gb300_matrix_assemble(gb300_matrix *A)
     GB_CUDA(cudaMemcpyAsync(dv.p + old, A->sv.p, sizeof(double) * A->staged,
                             cudaMemcpyDeviceToDevice, st));
   }
+  FetchEnd fetches(A->ctx);
   if(added > 0) {
     GB_TRY(fetch_pageable(A->ctx, dr.p + have, A->hr.data(), sizeof(int) * added));
     GB_TRY(fetch_pageable(A->ctx, dc.p + have, A->hc.data(), sizeof(int) * added));
@@ -607,6 +610,7 @@ int gb300_matrix_assemble(gb300_matrix *A)
     A->ilu = nullptr;
   }
   GB_TRY(build_csr_from_coo(A, m, dr.p, dc.p, dv.p));
+  fetches.done = true;
   A->drop_staged();
   return GB300_OK;
 }

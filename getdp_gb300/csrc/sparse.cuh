@@ -17,7 +17,21 @@ int build_csr_from_coo(gb300_matrix *A, long long m, const int *d_r,
                        const int *d_c, const double *d_v);
 // A's CSR as row-ordered triplets (device arrays of nnz entries)
 int csr_triplets(const gb300_matrix *A, int *d_r, int *d_c, double *d_v);
+// host memory to the device, read until the context's stream has come past:
+// src stays as it is until then, also where the caller returns an error (FetchEnd)
 int fetch_pageable(gb300_ctx *ctx, void *dst, const void *src, size_t bytes);
+// waits for the fetches of its scope unless `done` (the stream was synchronised)
+struct FetchEnd {
+  cudaStream_t st;
+  bool done = false;
+  explicit FetchEnd(const gb300_ctx *ctx) : st(ctx->stream) {}
+  ~FetchEnd()
+  {
+    if(!done) cudaStreamSynchronize(st);
+  }
+  FetchEnd(const FetchEnd &) = delete;
+  FetchEnd &operator=(const FetchEnd &) = delete;
+};
 
 void spmv64(const gb300_matrix *A, const double *x, double *y, cudaStream_t st);
 void spmv_plain(const gb300_matrix *A, const double *val, const double *x,
