@@ -1085,6 +1085,7 @@ int generate_pattern(gb300_matrix *A, const gb300_term_batch *t)
     GB_CUDA(cudaStreamSynchronize(st));
     if(!hd) {
       if(!linked(A, G)) {
+        A->csr_valid = false;  // until the arrays hold the new pattern
         GB_TRY(A->rowptr.alloc(A->n + 1));
         GB_TRY(A->col.alloc(G->nnz > 0 ? G->nnz : 1));
         GB_TRY(A->val.alloc(G->nnz > 0 ? G->nnz : 1));

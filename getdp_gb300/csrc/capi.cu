@@ -694,6 +694,7 @@ int gb300_matrix_set_csr(gb300_matrix *A, long long nnz, const int *rowptr,
     return GB300_ERR_ARG;
   }
   cudaStream_t st = A->ctx->stream;
+  A->csr_valid = false;  // until the arrays hold the new pattern
   GB_TRY(A->rowptr.alloc(A->n + 1));
   GB_TRY(A->col.alloc(nnz > 0 ? nnz : 1));
   GB_TRY(A->val.alloc(nnz > 0 ? nnz : 1));

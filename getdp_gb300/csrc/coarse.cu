@@ -103,7 +103,7 @@ int coarse_set(gb300_matrix *A, const int *agg, int nc)
   if(!A->coarse) A->coarse = new Coarse();
   Coarse *c = A->coarse;
   c->n = n;
-  c->nc = nc;
+  c->nc = 0;  // not valid until all buffers are there
   c->headroom = head;
   c->stamp++;
   c->ready = false;
@@ -122,6 +122,7 @@ int coarse_set(gb300_matrix *A, const int *agg, int nc)
   GB_CUDA(cudaMemcpyAsync(c->aptr.p, cnt.data(), sizeof(int) * (nc + 1),
                           cudaMemcpyHostToDevice, st));
   GB_CUDA(cudaStreamSynchronize(st));
+  c->nc = nc;
   c->version = A->pattern_version;
   return GB300_OK;
 }
@@ -240,7 +241,7 @@ int coarse_follow(const gb300_matrix *A, gb300_matrix *B, const Colouring *C,
     return GB300_OK;
   const int n = A->n, nc = a->nc;
   c->n = n;
-  c->nc = nc;
+  c->nc = 0;  // not valid until all buffers are there
   c->headroom = a->headroom;
   c->ready = false;
   GB_TRY(c->agg.alloc(n));
@@ -257,6 +258,7 @@ int coarse_follow(const gb300_matrix *A, gb300_matrix *B, const Colouring *C,
   GB_CUDA(cudaMemcpyAsync(c->aptr.p, a->aptr.p, sizeof(int) * (nc + 1),
                           cudaMemcpyDeviceToDevice, st));
   GB_CUDA(cudaGetLastError());
+  c->nc = nc;
   c->followed = a->stamp;
   c->version = B->pattern_version;
   return GB300_OK;

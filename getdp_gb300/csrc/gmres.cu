@@ -333,15 +333,9 @@ static int ell_values(EllPart &E, const T *lu, DevBuf<T> &v, cudaStream_t st)
   return GB300_OK;
 }
 
-static int ilu_setup(gb300_matrix *A)
+// the level schedule, diagonal positions and sliced-ELL structure of A's pattern
+static int ilu_schedule(gb300_matrix *A, ilu_data *L)
 {
-  // the level schedule and diagonal positions belong to one pattern
-  if(A->ilu && A->ilu->n == A->n && A->ilu->version == A->pattern_version) return GB300_OK;
-  if(A->ilu) ilu_free(A->ilu);
-  A->ilu = new ilu_data();
-  ilu_data *L = A->ilu;
-  L->n = A->n;
-  L->version = A->pattern_version;
   cudaStream_t st = A->ctx->stream;
   int n = A->n;
   DevBuf<int> indl, indu, err;
@@ -357,17 +351,12 @@ static int ilu_setup(gb300_matrix *A)
   GB_CUDA(cudaStreamSynchronize(st));
   if(herr & 1) {
     set_error("ILU(0): a row has no diagonal entry");
-    ilu_free(A->ilu);
-    A->ilu = nullptr;
     return GB300_ERR_ZERO_PIVOT;
   }
   if(herr & 2) {
     set_error("ILU(0): the level schedule needs a structurally symmetric pattern");
-    ilu_free(A->ilu);
-    A->ilu = nullptr;
     return GB300_ERR_UNSUPPORTED;
   }
-  int rc = GB300_OK;
   const Colouring *C = A->order;
   if(C && C->kind == 0 && C->bs == 1 && C->seg.size() == 2) {
     // first-fit colours: a row of colour c has neighbours of every smaller
@@ -380,19 +369,30 @@ static int ilu_setup(gb300_matrix *A)
     L->useg.assign(L->lseg.rbegin(), L->lseg.rend());
   }
   else {
-    rc = make_levels<0>(A, L, indl.p, L->lrows, L->lptr, L->hlptr, L->lseg);
-    if(rc == GB300_OK)
-      rc = make_levels<1>(A, L, indu.p, L->urows, L->uptr, L->huptr, L->useg);
+    GB_TRY(make_levels<0>(A, L, indl.p, L->lrows, L->lptr, L->hlptr, L->lseg));
+    GB_TRY(make_levels<1>(A, L, indu.p, L->urows, L->uptr, L->huptr, L->useg));
   }
-  if(rc == GB300_OK) rc = build_ell<0>(A, L->lseg, L->lrows.p, L->diag.p, L->lell, st);
-  if(rc == GB300_OK) rc = build_ell<1>(A, L->useg, L->urows.p, L->diag.p, L->uell, st);
-  if(rc == GB300_OK && L->by_colour)
-    rc = build_ell<2>(A, {{0, 0, false, n, 0}}, nullptr, L->diag.p, L->aell, st);
-  if(rc != GB300_OK) {
-    ilu_free(A->ilu);
-    A->ilu = nullptr;
-  }
-  return rc;
+  GB_TRY(build_ell<0>(A, L->lseg, L->lrows.p, L->diag.p, L->lell, st));
+  GB_TRY(build_ell<1>(A, L->useg, L->urows.p, L->diag.p, L->uell, st));
+  if(L->by_colour)
+    GB_TRY(build_ell<2>(A, {{0, 0, false, n, 0}}, nullptr, L->diag.p, L->aell, st));
+  return GB300_OK;
+}
+
+static int ilu_setup(gb300_matrix *A)
+{
+  // it belongs to one pattern
+  if(A->ilu && A->ilu->n == A->n && A->ilu->version == A->pattern_version) return GB300_OK;
+  if(A->ilu) ilu_free(A->ilu);
+  A->ilu = nullptr;
+  // (held by A once it is whole: a set-up that ran out of memory half way must
+  // not pass for one at the next call)
+  auto L = std::make_unique<ilu_data>();
+  L->n = A->n;
+  L->version = A->pattern_version;
+  GB_TRY(ilu_schedule(A, L.get()));
+  A->ilu = L.release();
+  return GB300_OK;
 }
 
 // ---------------------------------------------------------------------------

@@ -379,6 +379,7 @@ int build_pattern_from_elements(gb300_matrix *A, int ne, int nloc,
     set_error("pattern: %lld nonzeros exceed 32-bit CSR indexing", nnz);
     return GB300_ERR_CAPACITY;
   }
+  A->csr_valid = false;  // until the arrays hold the new pattern
   GB_TRY(A->rowptr.alloc(n + 1));
   GB_TRY(A->col.alloc(nnz > 0 ? nnz : 1));
   GB_TRY(A->val.alloc(nnz > 0 ? nnz : 1));
@@ -612,6 +613,7 @@ int build_csr_from_coo(gb300_matrix *A, long long m, const int *d_r,
               kCooCap);
     return GB300_ERR_CAPACITY;
   }
+  A->csr_valid = false;  // until the arrays hold the new pattern
   GB_TRY(A->rowptr.alloc(n + 1));
   GB_TRY(A->col.alloc(nnz > 0 ? nnz : 1));
   GB_TRY(A->val.alloc(nnz > 0 ? nnz : 1));
