@@ -39,6 +39,7 @@
 // every result computed with it, is deterministic.  For a
 // batch of independent systems (diagonal blocks) the rows are reordered
 // within each block only, so every block keeps its row range.
+#include <algorithm>
 #include <memory>
 
 #include "krylov.cuh"
@@ -87,33 +88,47 @@ __global__ void k_jp_round(int nv, int bs, const int *__restrict__ rowptr,
 // enters once, in any order: its colour depends on its later neighbours'
 // colours only).  A front costs some 3 us of dependent loads; a round over all
 // vertices took 8 to 14 us and there are about 2n of them on an n x n grid
-// (1024^2: 26 -> 12 ms).
+// (1024^2: 26 -> 12 ms).  It may start from what rounds have left: a vertex
+// without a colour has no coloured neighbour before it.
 constexpr int kFrontThreads = 1024;
+
+struct FrontState {
+  int unsym;  // the pattern is not structurally symmetric within the blocks
+  int first;  // vertices of the first fronts
+  int most;   // the largest colour
+  int done;   // vertices the fronts have coloured
+};
 
 __global__ void k_front_count(int nv, int bs, const int *__restrict__ rowptr,
                               const int *__restrict__ col, const int *__restrict__ blk,
-                              const int *__restrict__ off, int *__restrict__ cnt,
-                              int *__restrict__ queue, int *__restrict__ tail,
-                              int *__restrict__ unsym)
+                              const int *__restrict__ off, const int *__restrict__ color,
+                              int *__restrict__ cnt, int *__restrict__ queue,
+                              int *__restrict__ tail, FrontState *__restrict__ S)
 {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if(i >= nv) return;
+  const int coloured = i < nv ? color[i] : -1;
+  const int mx = __reduce_max_sync(0xffffffffu, coloured);
+  if((threadIdx.x & 31) == 0 && mx >= 0) atomicMax(&S->most, mx);
+  if(i >= nv || coloured >= 0) return;
   int later = 0;
   for(int r = i * bs; r < i * bs + bs; r++)
     for(int k = rowptr[r]; k < rowptr[r + 1]; k++) {
       const int c = col[k];
-      if(c / bs > i) later++;
+      if(c / bs > i && color[c / bs] < 0) later++;
       if(find_col(col, rowptr[c], rowptr[c + 1], r) < 0 || blk[c / bs] != blk[i])
-        atomicExch(unsym, 1);
+        atomicExch(&S->unsym, 1);
     }
   cnt[i] = later;
-  if(later == 0) queue[off[blk[i]] + atomicAdd(&tail[blk[i]], 1)] = i;
+  if(later == 0) {
+    queue[off[blk[i]] + atomicAdd(&tail[blk[i]], 1)] = i;
+    atomicAdd(&S->first, 1);
+  }
 }
 
 __global__ void __launch_bounds__(kFrontThreads)
 k_colour_fronts(int bs, const int *__restrict__ rowptr, const int *__restrict__ col,
                 const int *__restrict__ off, int *cnt, int *queue, const int *tail, int *color,
-                int *most, int *left)
+                FrontState *S)
 {
   constexpr int U = 8;
   __shared__ int s_tail;
@@ -167,8 +182,8 @@ k_colour_fronts(int bs, const int *__restrict__ rowptr, const int *__restrict__ 
     __syncthreads();
   }
   mx = __reduce_max_sync(0xffffffffu, mx);
-  if((threadIdx.x & 31) == 0) atomicMax(most, mx);
-  if(threadIdx.x == 0 && head != nv) atomicAdd(left, nv - head);
+  if((threadIdx.x & 31) == 0) atomicMax(&S->most, mx);
+  if(threadIdx.x == 0) atomicAdd(&S->done, head);
 }
 
 __global__ void k_colour_flag(int n, const int *__restrict__ color, int c,
@@ -378,60 +393,76 @@ int colour_build(gb300_matrix *A, int nseg, const int *off)
   if(cudaMemsetAsync(color.p, 0xff, sizeof(int) * nv, st) != cudaSuccess ||
      cudaMemsetAsync(err.p, 0, sizeof(int), st) != cudaSuccess)
     return fail(GB300_ERR_CUDA);
-  // the fronts of a structurally symmetric pattern, where a front's vertices
+  // The fronts of a structurally symmetric pattern, where a front's vertices
   // are few or their rows short: one CTA per block walks all entries twice
   // (edge elements 40^3, 16 entries a row: 12.6 ms against 8.7 ms of rounds;
-  // 1024^2, 7 a row: 12 against 26).  Any other pattern by rounds over all
-  // vertices.
-  bool fronts = false;
-  if(A->nnz <= 8LL * n || A->nnz <= 2000000LL * nseg) {
-    DevBuf<int> cnt, queue, tail, st3;  // st3: not symmetric, most, left
-    if(cnt.alloc(nv) || queue.alloc(nv) || tail.alloc(nseg) || st3.alloc(3))
-      return fail(GB300_ERR_CUDA);
-    const int init[3] = {0, -1, 0};
-    int h[3] = {0, 0, 0};
+  // 1024^2, 7 a row: 12 against 26; blocks of a batch side by side, so the
+  // largest counts).  Any other pattern by rounds over all vertices.
+  int largest = 1;
+  for(int q = 0; q < nseg; q++) largest = std::max(largest, vseg[q + 1] - vseg[q]);
+  bool fronts = A->nnz <= 8LL * n || A->nnz <= 2000000LL * (nv / largest);
+  DevBuf<int> cnt, queue, tail;
+  DevBuf<FrontState> state;
+  FrontState h = {0, 0, -1, 0};
+  auto count = [&]() -> bool {  // what the fronts start from
+    const FrontState init = {0, 0, -1, 0};
     if(cudaMemsetAsync(tail.p, 0, sizeof(int) * nseg, st) != cudaSuccess ||
-       cudaMemcpyAsync(st3.p, init, sizeof(init), cudaMemcpyHostToDevice, st) != cudaSuccess)
-      return fail(GB300_ERR_CUDA);
+       cudaMemcpyAsync(state.p, &init, sizeof(init), cudaMemcpyHostToDevice, st) != cudaSuccess)
+      return false;
     k_front_count<<<grid_for(nv, 256), 256, 0, st>>>(nv, bs, A->rowptr.p, A->col.p, blk.p,
-                                                     doff.p, cnt.p, queue.p, tail.p, st3.p);
-    if(cudaMemcpyAsync(h, st3.p, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+                                                     doff.p, color.p, cnt.p, queue.p, tail.p,
+                                                     state.p);
+    return cudaMemcpyAsync(&h, state.p, sizeof(h), cudaMemcpyDeviceToHost, st) == cudaSuccess &&
+           cudaStreamSynchronize(st) == cudaSuccess;
+  };
+  if(fronts) {
+    if(cnt.alloc(nv) || queue.alloc(nv) || tail.alloc(nseg) || state.alloc(1) || !count())
+      return fail(GB300_ERR_CUDA);
+    fronts = !h.unsym;
+  }
+  // A wide first front is the mark of an irregular numbering, in which a few
+  // rounds colour all there is: in a random order of a 2D mesh a seventh of the
+  // vertices is in the first front and some 17 rounds do; row by row, along a
+  // space-filling curve or shuffled in runs of 64, it is one in a thousand at
+  // most.  One group of rounds then (0.11 ms at 16,384 vertices), and the
+  // fronts for what it leaves.  First application of ILU(0) in a random order,
+  // fronts / rounds: 1.14 / 1.21 ms at 128^2, 1.55 / 1.33 at 256^2, 3.12 / 1.76
+  // at 512^2, 9.5 / 3.7 at 1024^2.
+  constexpr int kWideFront = 32, kRoundsFrom = 32768;
+  const bool wide = fronts && largest > kRoundsFrom && h.first >= nv / kWideFront;
+  // rounds in groups of 32; the last of a group counts what is left
+  constexpr int kGroup = 32;
+  int remaining = nv, rounds = 0;
+  while(remaining > 0 && rounds <= nv && (!fronts || (wide && rounds == 0))) {
+    if(cudaMemsetAsync(left.p, 0, sizeof(int), st) != cudaSuccess) return fail(GB300_ERR_CUDA);
+    for(int g = 0; g < kGroup; g++)
+      k_jp_round<<<grid_for(nv, 256), 256, 0, st>>>(nv, bs, A->rowptr.p, A->col.p, color.p,
+                                                     g == kGroup - 1 ? left.p : nullptr,
+                                                     err.p);
+    if(cudaMemcpyAsync(&remaining, left.p, sizeof(int), cudaMemcpyDeviceToHost, st) !=
+         cudaSuccess ||
        cudaStreamSynchronize(st) != cudaSuccess)
       return fail(GB300_ERR_CUDA);
-    if(!h[0]) {
-      k_colour_fronts<<<nseg, kFrontThreads, 0, st>>>(bs, A->rowptr.p, A->col.p, doff.p, cnt.p,
-                                                      queue.p, tail.p, color.p, st3.p + 1,
-                                                      st3.p + 2);
-      if(cudaMemcpyAsync(h, st3.p, sizeof(h), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-         cudaStreamSynchronize(st) != cudaSuccess)
-        return fail(GB300_ERR_CUDA);
-      if(h[2] != 0 || h[1] >= 1024) return fail(GB300_ERR_UNSUPPORTED);
-      fronts = true;
-      C->ncolors = h[1] + 1;
-    }
+    rounds += kGroup;
   }
-  if(!fronts) {
-    // rounds in groups of 32; the last of a group counts what is left
-    constexpr int kGroup = 32;
-    int remaining = nv, rounds = 0;
-    while(remaining > 0 && rounds <= nv) {
-      if(cudaMemsetAsync(left.p, 0, sizeof(int), st) != cudaSuccess)
-        return fail(GB300_ERR_CUDA);
-      for(int g = 0; g < kGroup; g++)
-        k_jp_round<<<grid_for(nv, 256), 256, 0, st>>>(nv, bs, A->rowptr.p, A->col.p, color.p,
-                                                       g == kGroup - 1 ? left.p : nullptr,
-                                                       err.p);
-      if(cudaMemcpyAsync(&remaining, left.p, sizeof(int), cudaMemcpyDeviceToHost, st) !=
-           cudaSuccess ||
-         cudaStreamSynchronize(st) != cudaSuccess)
-        return fail(GB300_ERR_CUDA);
-      rounds += kGroup;
-    }
+  if(rounds > 0) {
     int herr = 0;
     if(cudaMemcpyAsync(&herr, err.p, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
        cudaStreamSynchronize(st) != cudaSuccess)
       return fail(GB300_ERR_CUDA);
-    if(remaining > 0 || herr) return fail(GB300_ERR_UNSUPPORTED);
+    if(herr || (remaining > 0 && !fronts)) return fail(GB300_ERR_UNSUPPORTED);
+  }
+  if(remaining > 0) {
+    if(rounds > 0 && !count()) return fail(GB300_ERR_CUDA);
+    k_colour_fronts<<<nseg, kFrontThreads, 0, st>>>(bs, A->rowptr.p, A->col.p, doff.p, cnt.p,
+                                                    queue.p, tail.p, color.p, state.p);
+    if(cudaMemcpyAsync(&h, state.p, sizeof(h), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+       cudaStreamSynchronize(st) != cudaSuccess)
+      return fail(GB300_ERR_CUDA);
+    if(h.done != remaining || h.most >= 1024) return fail(GB300_ERR_UNSUPPORTED);
+    C->ncolors = h.most + 1;
+  }
+  else {
     std::vector<int> hc(nv);
     if(cudaMemcpyAsync(hc.data(), color.p, sizeof(int) * nv, cudaMemcpyDeviceToHost, st) !=
          cudaSuccess ||
