@@ -71,7 +71,7 @@ def parse():
     ap.add_argument("--skip-cpu", action="store_true")
     ap.add_argument("--no-plain", action="store_true",
                     help="skip the plain FP64 comparison solve (profiling runs)")
-    ap.add_argument("--batch-kernel", type=int, default=4,
+    ap.add_argument("--batch-kernel", type=int, default=-1,
                     help="--profile sweep: Batch_Kernel of the batched solve")
     ap.add_argument("--profile", choices=["spmv32", "spmv64", "generate", "step", "twolevel",
                                           "sweep",

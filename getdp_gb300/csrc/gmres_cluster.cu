@@ -49,7 +49,7 @@ namespace gb {
 // (ILU(0)-GMRES(40) in the multicolour order) four were the fastest: few CTAs
 // leave the largest systems' steps to one or two SMs, many CTAs leave fewer
 // systems running at once and make each cluster barrier dearer.  Fewer
-// systems want larger clusters (see where the default is chosen).  1024
+// systems want larger clusters: the default, GB300_BATCH_AUTO, sizes them.  1024
 // threads in one CTA per SM leave half as many clusters: 322 against 240 ms
 // on 64 systems.
 constexpr int kCMaxKrylov = 64;
@@ -875,7 +875,8 @@ int gmres_solve_batch_cluster(gb300_matrix *A, const double *val, const double *
                               bool *used, const Colouring *mc)
 {
   *used = false;
-  int cs = p->batch_kernel;
+  const bool sized = p->batch_kernel == GB300_BATCH_AUTO;  // here, by the batch
+  int cs = sized ? 4 : p->batch_kernel;
   if(cs != 1 && cs != 2 && cs != 4 && cs != 8 && cs != 16) return GB300_OK;
   if((p->algorithm != 8 && p->algorithm != 9) ||
      (p->preconditioner != 0 && p->preconditioner != 6))
@@ -886,8 +887,8 @@ int gmres_solve_batch_cluster(gb300_matrix *A, const double *val, const double *
   if(m > kCMaxKrylov || p->nb_iter_max <= 0 || p->nb_iter_max > 100000000 || nsys < 1 ||
      p->precision == 2)
     return GB300_OK;
-  if(cs == 4) {
-    // the default: larger clusters where a few systems would leave SMs idle,
+  if(sized) {
+    // larger clusters where a few systems would leave SMs idle,
     // while the largest system has a row per thread of its cluster.
     // Measured (ms, 4 / 8 / 16 CTAs): 64 systems of 1,922..50,562 rows 466 /
     // 231 / 230; 12 of 1,058..28,322 154 / 77 / 48; 32 of 450..6,962 20.4 /
@@ -1005,16 +1006,20 @@ int gmres_solve_batch_cluster(gb300_matrix *A, const double *val, const double *
   const bool f32 = precond && fp32;
 #define GB_LAUNCH_C(CSZ)                                                              \
   GB_TRY(f32 ? launch_c<float, CSZ>(a, st, &nc) : launch_c<double, CSZ>(a, st, &nc))
-  switch(cs) {
-  case 1: GB_LAUNCH_C(1); break;
-  case 2: GB_LAUNCH_C(2); break;
-  case 4: GB_LAUNCH_C(4); break;
-  case 8: GB_LAUNCH_C(8); break;
-  default: GB_LAUNCH_C(16); break;
+  for(;; cs /= 2) {
+    switch(cs) {
+    case 1: GB_LAUNCH_C(1); break;
+    case 2: GB_LAUNCH_C(2); break;
+    case 4: GB_LAUNCH_C(4); break;
+    case 8: GB_LAUNCH_C(8); break;
+    default: GB_LAUNCH_C(16); break;
+    }
+    // no cluster fits or the launch was refused: nothing ran, and of the sizes
+    // chosen here the next smaller one may do (16 is not portable)
+    if(nc > 0 || !sized || cs <= 4) break;
   }
 #undef GB_LAUNCH_C
-  // no cluster fits or the launch was refused: nothing ran (x was zeroed, as
-  // the per-kernel form does first), and that form solves instead
+  // none (x was zeroed, as the per-kernel form does first): that form solves
   if(nc < 1) return GB300_OK;
   std::vector<int> hst(nsys), hits(nsys);
   std::vector<double> hres(nsys), hrr(nsys), hbb(nsys);

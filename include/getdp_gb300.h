@@ -63,6 +63,7 @@ int gb300_copy_to_host(gb300_ctx *ctx, void *dst, const void *src, size_t bytes)
    9 FGMRES; Preconditioner 0 none, 6 ILU0, 8 DIAGONAL; Scaling 0 none,
    1 diagonal (D^-1/2 A D^-1/2).  The last four fields are extensions of
    this backend (keys Sparskit would reject as unknown). */
+#define GB300_BATCH_AUTO (-1)
 typedef struct gb300_solver_params {
   int matrix_format;
   int matrix_printing;
@@ -98,10 +99,10 @@ typedef struct gb300_solver_params {
                              (default 0.3) */
   int inner_iter_max;     /* Inner_Iter_Max */
   int batch_kernel;       /* Batch_Kernel: form of gb300_solve_batch: c = 1, 2,
-                             4 (default), 8 or 16: one launch for the whole
+                             4, 8 or 16: one launch for the whole
                              batch, a thread-block cluster of c CTAs per
-                             system (the default takes 8 or 16 for a batch of
-                             few, large systems) (GMRES/FGMRES, Nb_Iter_Max > 0,
+                             system; -1 (default): of 4, or of 8 or 16 for a
+                             batch of few, large systems (GMRES/FGMRES, Nb_Iter_Max > 0,
                              Krylov_Size <= 64, at most 64 ILU(0) levels per
                              system, e.g. Renumbering_Technique 1); 0, or
                              where that does not apply: one launch per Krylov

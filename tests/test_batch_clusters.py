@@ -45,3 +45,20 @@ def test_default_clusters_match_the_per_kernel_form(kind, sizes, algorithm, prec
         assert abs(i1[k]["iterations"] - i0[k]["iterations"]) <= 1, (i1[k], i0[k])
         r0, r1 = bt.offsets[k], bt.offsets[k + 1]
         assert np.linalg.norm(x1[r0:r1] - x0[r0:r1]) <= 1e-9 * np.linalg.norm(x0[r0:r1])
+
+
+def test_a_size_asked_for_is_the_size_used():
+    """The sums are split by the cluster's CTAs, so another size rounds otherwise
+    and the same one does not: the default takes 16 CTAs for these systems, and
+    a size given in Batch_Kernel is kept, the smallest of the default's too."""
+    bt = W.concat_problems([W.eddy_2d(n, seed=40 + n) for n in (92, 24)])
+    terms = G.DeviceTerms(bt.problem, bt.dofmap)
+    A, b = LA.gMatrix(bt.dofmap.n_dof), LA.gVector(bt.dofmap.n_dof)
+    G.generate(A, b, terms.batch)
+    x = {c: _solve(A, b, bt.offsets, c, 8, 0) for c in (4, 8, 16, -1, None)}
+    for infos, _ in x.values():
+        assert all(i["batch_form"] == 1 and i["status"] == 0 for i in infos)
+    assert np.array_equal(x[None][1], x[16][1]) and np.array_equal(x[-1][1], x[16][1])
+    assert not np.array_equal(x[4][1], x[16][1]) and not np.array_equal(x[4][1], x[8][1])
+    # asked for again: the same bits
+    assert np.array_equal(_solve(A, b, bt.offsets, 4, 8, 0)[1], x[4][1])
