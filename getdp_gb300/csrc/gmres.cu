@@ -1108,7 +1108,6 @@ struct GmState {
   double h1[kMaxKrylov + 1], h2[kMaxKrylov + 1];  // the column of each pass
   double nrm0;      // ||w||^2 before the Gram-Schmidt pass of this step
   int reorth;       // this step takes a second Gram-Schmidt pass
-  int reorths;      // second passes taken so far
   // arrival counters of the kernels whose last CTA finishes a reduction
   unsigned tick_dots[2][kMaxKrylov / kDotCols + 1], tick_upd[2];
 };
@@ -1386,10 +1385,7 @@ k_gm_update(int n, int m, double *V, size_t ldv, const double *w, double *cur,
   if(pass == 0) {
     const bool more = !(rr >= 0.02 * nrm0);
     S->reorth = more;
-    if(more) {
-      S->reorths += 1;
-      return;  // the step ends after the second pass
-    }
+    if(more) return;  // the step ends after the second pass
   }
   S->its = its + 1;
   S->k = k;
