@@ -309,9 +309,9 @@ inline void launch_chain(bool early, void (*kernel)(K...), dim3 grid, dim3 block
 // 2D meshes in the multicolour order, both sweeps / a product, early against
 // not: 14.2 / 2.8 against 15.4 / 3.4 us at 65,025 rows, but 25.3 / 7.0
 // against 19.3 / 7.6 at 261,121: the waiting CTAs of the next kernel take the
-// free slots of whichever SMs have them, and its load is uneven from then on
-// (the FP64-bound Gram-Schmidt kernels lose by that at every size and never
-// start early)
+// free slots of whichever SMs have them, and its load is uneven from then on.
+// (The FP64-bound Gram-Schmidt kernels lose by that at all but the smallest
+// sizes and have a line of their own, in gmres_solve.)
 inline bool chain_early(int n) { return n <= 131072; }
 
 inline int grid_for(long long work, int threads, int max_blocks = 1 << 30)

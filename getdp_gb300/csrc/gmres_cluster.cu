@@ -103,35 +103,30 @@ __device__ __forceinline__ void cluster_sum(cg::cluster_group &cl, double *buf, 
   __syncthreads();
 }
 
-// s - sum_k a[k] x[col[k]] over k = k0, k0 + step, ... < k1, in that order
-// (lusol's and amux's accumulation order), with the column indices and
-// values of up to eight entries loaded before their gathers, so that a
-// thread has eight loads in flight instead of a chain of dependent ones
-template <int STEP, bool SUB, typename T, typename X>
+// s - sum_k a[k] x[col[k]] over k0 <= k < k1, in that order (lusol's
+// accumulation order), with the column indices and values of four entries
+// loaded before their gathers, so that a thread has four loads in flight
+// instead of a chain of dependent ones
+template <typename T, typename X>
 __device__ __forceinline__ T row_acc(int k0, int k1, const int *__restrict__ col,
                                      const T *__restrict__ a, const X *x, T s)
 {
-  for(int kb = k0; kb < k1; kb += 4 * STEP) {
+  for(int kb = k0; kb < k1; kb += 4) {
     int c[4];
     T v[4];
     X xv[4];
 #pragma unroll
     for(int u = 0; u < 4; u++) {
-      int k = kb + u * STEP;
+      int k = kb + u;
       c[u] = k < k1 ? col[k] : 0;
       v[u] = k < k1 ? a[k] : (T)0;
     }
 #pragma unroll
     for(int u = 0; u < 4; u++)
-      if(kb + u * STEP < k1) xv[u] = __ldcg(x + c[u]);
+      if(kb + u < k1) xv[u] = __ldcg(x + c[u]);
 #pragma unroll
     for(int u = 0; u < 4; u++)
-      if(kb + u * STEP < k1) {
-        if(SUB)
-          s = s - v[u] * xv[u];
-        else
-          s += v[u] * xv[u];
-      }
+      if(kb + u < k1) s = s - v[u] * xv[u];
   }
   return s;
 }
@@ -353,7 +348,7 @@ template <typename T> struct RowAhead {
 #pragma unroll
     for(int u = 0; u < kAhead; u++)
       if(c[u] >= 0) s = s - v[u] * xv[u];
-    return k0 + kAhead < k1 ? row_acc<1, true>(k0 + kAhead, k1, col, lu, x, s) : s;
+    return k0 + kAhead < k1 ? row_acc(k0 + kAhead, k1, col, lu, x, s) : s;
   }
 };
 
@@ -521,10 +516,10 @@ __device__ __noinline__ void c_precond(const CArgs &P, cg::cluster_group &cl, in
       const int i = P.lrows[t];
       const int ke = P.diag[i];
       if constexpr(sizeof(T) == 8)
-        dst[i] = row_acc<1, true>(P.rowptr[i], ke, P.col, lu, (const double *)dst,
+        dst[i] = row_acc(P.rowptr[i], ke, P.col, lu, (const double *)dst,
                                   __ldcg(src + i));
       else
-        P.t32[i] = row_acc<1, true>(P.rowptr[i], ke, P.col, lu, (const float *)P.t32,
+        P.t32[i] = row_acc(P.rowptr[i], ke, P.col, lu, (const float *)P.t32,
                                     (float)__ldcg(src + i));
     }
     cl.sync();
@@ -537,12 +532,12 @@ __device__ __noinline__ void c_precond(const CArgs &P, cg::cluster_group &cl, in
       const int i = P.urows[t];
       const int ke = P.rowptr[i + 1];
       if constexpr(sizeof(T) == 8) {
-        double s = row_acc<1, true>(P.diag[i] + 1, ke, P.col, lu, (const double *)dst,
+        double s = row_acc(P.diag[i] + 1, ke, P.col, lu, (const double *)dst,
                                     __ldcg(dst + i));
         dst[i] = inv[i] * s;
       }
       else {
-        float s = row_acc<1, true>(P.diag[i] + 1, ke, P.col, lu, (const float *)P.t32,
+        float s = row_acc(P.diag[i] + 1, ke, P.col, lu, (const float *)P.t32,
                                    __ldcg(P.t32 + i));
         float v = inv[i] * s;
         P.t32[i] = v;

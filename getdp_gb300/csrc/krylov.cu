@@ -212,8 +212,9 @@ k_cg_step(int n, CgState *S, T *x, T *r, const T *p, const T *q, double *__restr
 {
   // alpha and the breakdown test once per CTA: FP64 divisions in every
   // thread would keep the FP64 pipe busier than the vector traffic.  The
-  // first entries are on their way meanwhile.  Vectors are cudaMalloc'ed
-  // (256-byte aligned): groups of four, then the n % 4 remainder
+  // first entries are on their way meanwhile.  Vectors are device buffers (256
+  // byte aligned, from cudaMalloc or a pool): groups of four, then the n % 4
+  // remainder
   __shared__ T s_alpha;
   __shared__ int s_bad;
   const long long stride = (long long)gridDim.x * blockDim.x;
