@@ -1075,8 +1075,6 @@ void ilu_factor_arrays(const gb300_matrix *A, bool fp32, const void **lu, const 
 constexpr int kMaxKrylov = 128;
 constexpr int kDotCols = 8;  // columns of one group of dot products
 
-constexpr int kNoShift = 16;
-
 struct GmState {
   int active;       // whole solve still running
   int cycle;        // current restart cycle still extending the basis
@@ -1096,13 +1094,8 @@ struct GmState {
   // vector j of the algorithm is sc[j] V_j: the basis vectors are left with
   // the norm h(j+1,j) they come out of the Gram-Schmidt step with, the
   // preconditioner and the product act on them as they are, and the scalars
-  // carry the normalisation (no pass over the vector scales it).  Where the
-  // norm of a step's product is not within 2^+-16, V_k is kept 2^-shift times
-  // as large (a power of two, in the coefficients of the update: nothing is
-  // rounded and no row costs more), so that the next product's square stays
-  // in range for every ||A M^-1|| within 2^+-490
+  // carry the normalisation (no pass over the vector scales it)
   double sc[kMaxKrylov + 1];
-  int shift;        // of the newest vector
   double H[(kMaxKrylov + 1) * kMaxKrylov];  // column-major, (m+1) x m
   double cs[kMaxKrylov], sn[kMaxKrylov], g[kMaxKrylov + 1], y[kMaxKrylov];
   double h1[kMaxKrylov + 1], h2[kMaxKrylov + 1];  // the column of each pass
@@ -1111,9 +1104,6 @@ struct GmState {
   // arrival counters of the kernels whose last CTA finishes a reduction
   unsigned tick_dots[2][kMaxKrylov / kDotCols + 1], tick_upd[2];
 };
-
-// 2^e, |e| <= 1022
-__device__ __forceinline__ double pow2(int e) { return __hiloint2double((1023 + e) << 20, 0); }
 
 // restart: r = rhs - A x was computed with its partial norms
 __global__ void k_gm_restart(GmState *S, const double *__restrict__ part, int m)
@@ -1264,8 +1254,6 @@ k_gm_dots(int n, const double *V, size_t ldv, const double *w, double *part, GmS
     // the cycle; gmres then reports a break-down.  (k_gm_update clears
     // S->cycle: CTAs of the other groups may only now be reading it)
     S->nrm0 = v;
-    const int e = (((__double2hiint(v) >> 20) & 0x7ff) - 1023) >> 1;  // of ||w||
-    S->shift = e > kNoShift || e < -kNoShift ? e : 0;
     if(!(v > 0. && 1. / v > 0.)) {
       S->its += 1;  // the Arnoldi step's product was formed
       S->breakdown = (v <= 0.) ? -1 : -2;
@@ -1300,7 +1288,7 @@ k_gm_update(int n, int m, double *V, size_t ldv, const double *w, double *cur,
     if(bad && blockIdx.x == 0 && threadIdx.x == 0) S->cycle = 0;
     return;
   }
-  const int nb = gridDim.x - 1, e = S->shift;
+  const int nb = gridDim.x - 1;
   __shared__ double h[kMaxKrylov + 1];
   __shared__ double rc[kMaxKrylov], rs[kMaxKrylov], ra[kMaxKrylov];
   double *Hc = S->H + (size_t)(k - 1) * (kMaxKrylov + 1);  // column k
@@ -1310,8 +1298,7 @@ k_gm_update(int n, int m, double *V, size_t ldv, const double *w, double *cur,
     const int j = threadIdx.x;
     double c = 0., s = 0., b = 0.;
     if(j < k) {
-      h[j] = S->h1[j];
-      if(pass == 1) h[j] += e ? S->h2[j] * pow2(e) : S->h2[j];
+      h[j] = S->h1[j] + (pass == 0 ? 0. : S->h2[j]);
       c = S->cs[j];
       s = S->sn[j];
     }
@@ -1335,14 +1322,9 @@ k_gm_update(int n, int m, double *V, size_t ldv, const double *w, double *cur,
     if(j < k) Hc[j] = j < k - 1 ? fma(c, ra[j], s * b) : ra[j];
   }
   else {
-    double sw = pass == 0 ? S->sc[k - 1] : 1.;
-    const double p2 = pow2(-e);
-    if(e && pass == 0) sw *= p2;
-    for(int j = threadIdx.x; j < k; j += blockDim.x) {
-      double hj = pass == 0 ? S->h1[j] : S->h2[j];
-      if(e && pass == 0) hj *= p2;
-      h[j] = -S->sc[j] * hj;
-    }
+    for(int j = threadIdx.x; j < k; j += blockDim.x)
+      h[j] = -S->sc[j] * (pass == 0 ? S->h1[j] : S->h2[j]);
+    const double sw = pass == 0 ? S->sc[k - 1] : 1.;
     __syncthreads();
     double v = 0.;
     for(int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += nb * blockDim.x) {
@@ -1368,15 +1350,10 @@ k_gm_update(int n, int m, double *V, size_t ldv, const double *w, double *cur,
     if(threadIdx.x == 0) pn[blockIdx.x] = s;
   }
   // what the end of the step reads, on its way while the ticket is drawn
-  const double tol = S->tol, g = S->g[k - 1];
-  double nrm0 = S->nrm0;
+  const double nrm0 = S->nrm0, tol = S->tol, g = S->g[k - 1];
   const int its = S->its, maxit = S->maxit;
   if(!arrive_last(&S->tick_upd[pass], gridDim.x)) return;
-  double hk = __ldcg(Hc + k - 1);
-  if(e) {  // in V_k's units, as rr is
-    hk *= pow2(-e);
-    nrm0 = nrm0 * pow2(-e) * pow2(-e);
-  }
+  const double hk = __ldcg(Hc + k - 1);
   double rr = 0.;
 #pragma unroll 4
   for(int i = threadIdx.x; i < nb; i += blockDim.x) rr += __ldcg(pn + i);
@@ -1393,8 +1370,8 @@ k_gm_update(int n, int m, double *V, size_t ldv, const double *w, double *cur,
   if(!(rr > 0.)) {
     // mgsro ierr -3: the new vector depends on the others; the reference
     // solves with the column as mgsro left it, no rotation applied
-    for(int j = 0; j < k; j++) Hc[j] = S->h1[j] + (pass == 0 ? 0. : S->h2[j] * pow2(e));
-    Hc[k] = sqrt(rr) * pow2(e);
+    for(int j = 0; j < k; j++) Hc[j] = S->h1[j] + (pass == 0 ? 0. : S->h2[j]);
+    Hc[k] = sqrt(rr);
     S->breakdown = -3;
     S->cycle = 0;
     return;
@@ -1403,21 +1380,20 @@ k_gm_update(int n, int m, double *V, size_t ldv, const double *w, double *cur,
   // independent reciprocal roots, a third of the serial chain of its root,
   // divisions and root (an FP64 division takes about 0.8 us here)
   const double r2 = fma(hk, hk, rr);
-  double c, s, rkk;
+  double c, s;
   if(rr > 1e-280 && r2 < 1e280) {
     const double ri = rsqrt(rr), q = rsqrt(r2);
     S->sc[k] = ri;
     c = hk * q;
     s = rr * ri * q;
-    rkk = r2 * q;
+    Hc[k - 1] = r2 * q;
   }
   else {
     double x = hk, y = sqrt(rr);
     S->sc[k] = 1. / y;
     givens_dev(&x, &y, &c, &s);
-    rkk = x;
+    Hc[k - 1] = x;
   }
-  Hc[k - 1] = e ? rkk * pow2(e) : rkk;
   S->cs[k - 1] = c;
   S->sn[k - 1] = s;
   S->g[k - 1] = c * g;
