@@ -363,7 +363,7 @@ namespace gb {
 // make scratch buffers on each call set it for their duration: cudaMalloc and
 // cudaFree cost some 10 to 200 us each and the latter waits for the device (a
 // Generate at 513^2 spent 0.2 of its 0.3 ms in them).  Null: no pool, for
-// buffers that may outlive the context.
+// buffers that may outlive the matrix's context.
 struct PoolScope {
   MemPool *before;
   explicit PoolScope(gb300_ctx *c) : before(t_pool) { t_pool = c ? &c->mem : nullptr; }

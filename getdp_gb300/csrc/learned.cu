@@ -584,8 +584,9 @@ static int mp_prepare(gb300_mpnn *net, const gb300_matrix *A)
   }
   {
     // kept with the network, which may be used on another context's matrix next
-    // and outlive this one's: not from its pool
-    PoolScope kept(nullptr);
+    // and outlive this one's: from its own context's pool, or from none (a new
+    // network's buffers cost 0.3 ms by cudaMalloc)
+    PoolScope kept(A->ctx == net->ctx ? net->ctx : nullptr);
     GB_TRY(g.ehat.alloc(A->nnz));
     GB_TRY(g.feat.alloc((size_t)n * 4));
     GB_TRY(g.dscale.alloc(n));
