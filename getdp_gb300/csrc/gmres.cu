@@ -26,6 +26,8 @@
 // re-orthogonalises selectively (a second pass when the first removed more
 // than 98 % of ||w||^2), and both return an orthonormal basis to working
 // precision.
+#include <math.h>
+
 #include <algorithm>
 #include <memory>
 
@@ -1577,9 +1579,8 @@ void precond_run(const gb300_matrix *A, const double *val, const gb300_solver_pa
   smooth(s.t3, z, s.t4, true, learned_post && !sai);
 }
 
-int gmres_solve(gb300_matrix *A, const double *val, const double *rhs,
-                double *x, const gb300_solver_params *p, gb300_solve_info *info,
-                Work &W)
+static int gmres_run(gb300_matrix *A, const double *val, const double *rhs, double *x,
+                     const gb300_solver_params *p, gb300_solve_info *info, Work &W)
 {
   cudaStream_t st = A->ctx->stream;
   int n = A->n;
@@ -1756,6 +1757,56 @@ int gmres_solve(gb300_matrix *A, const double *val, const double *rhs,
   info->status = active ? -1 : h0.status;
   info->iterations = h0.its;
   info->residual_estimate = h0.res6;
+  return GB300_OK;
+}
+
+// the largest |v_k| (non-negative doubles order like their bit patterns)
+__global__ void k_max_abs(long long m, const double *__restrict__ v, unsigned long long *out)
+{
+  unsigned long long t = 0;
+  for(long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x; k < m;
+      k += (long long)gridDim.x * blockDim.x)
+    t = max(t, (unsigned long long)__double_as_longlong(fabs(v[k])));
+  for(int o = 16; o > 0; o >>= 1) t = max(t, __shfl_down_sync(0xffffffffu, t, o));
+  if((threadIdx.x & 31) == 0) atomicMax(out, t);
+}
+
+__global__ void k_times(long long m, double f, const double *v, double *out)
+{
+  for(long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x; k < m;
+      k += (long long)gridDim.x * blockDim.x)
+    out[k] = f * v[k];
+}
+
+// The basis is left unnormalised, so the square of a product is of the order of
+// ||A M^-1||^4.  With a preconditioner that is some power of one; without, a
+// matrix whose largest entry is not within 2^+-64 is solved as
+// (2^-e A) (2^e x) = b, which rounds nothing.  (Powers of two inside the step
+// instead, where nothing has to be known in advance, cost every solve 1 %.)
+int gmres_solve(gb300_matrix *A, const double *val, const double *rhs,
+                double *x, const gb300_solver_params *p, gb300_solve_info *info,
+                Work &W)
+{
+  if(p->preconditioner != 0 && p->preconditioner != 8)
+    return gmres_run(A, val, rhs, x, p, info, W);
+  cudaStream_t st = A->ctx->stream;
+  DevBuf<unsigned long long> top;
+  GB_TRY(top.alloc(1));
+  GB_CUDA(cudaMemsetAsync(top.p, 0, sizeof(unsigned long long), st));
+  k_max_abs<<<grid_for(A->nnz, 256, kReduceBlocks), 256, 0, st>>>(A->nnz, val, top.p);
+  double most = 0.;
+  GB_CUDA(cudaMemcpyAsync(&most, top.p, sizeof(most), cudaMemcpyDeviceToHost, st));
+  GB_CUDA(cudaStreamSynchronize(st));
+  int e = 0;
+  if(most > 0. && most <= 1.7976931348623157e308) frexp(most, &e);
+  if(e >= -64 && e <= 64) return gmres_run(A, val, rhs, x, p, info, W);
+  const double f = ldexp(1., -std::max(e, -1000));
+  DevBuf<double> sval;
+  GB_TRY(sval.alloc(A->nnz));
+  k_times<<<grid_for(A->nnz, 256, kReduceBlocks), 256, 0, st>>>(A->nnz, f, val, sval.p);
+  GB_TRY(gmres_run(A, sval.p, rhs, x, p, info, W));
+  k_times<<<grid_for(A->n, 256, kReduceBlocks), 256, 0, st>>>(A->n, f, x, x);
+  GB_CUDA(cudaGetLastError());
   return GB300_OK;
 }
 
